@@ -235,6 +235,14 @@ int resolve_form(int requested, int N, int M, int dev) {
   return softassign_band_preferred(N, M, dev) ? kFormBanded : kFormMatrixFree;
 }
 
+// Whether a registration's leading pose updates go to the series kernel: only
+// under AUTO (a form asked for by name runs as it is), and not where a phase
+// timeline of the affinity kernels was asked for. The kernel itself decides on
+// the device how far the clouds and temperatures let it go.
+int series_for(int requested, int form, int N, int M, bool timeline) {
+  return requested == CESA_SINKHORN_AUTO && form != kFormMaterialised && !timeline && softassign_series_fits(N, M);
+}
+
 // Shared body of the two host-pointer entry points.
 int run_host(int kind, const float* X, int N, const float* Y, int M, float R[9], float t[3],
              const cesa_params* p, cesa_report* rep) {
@@ -338,6 +346,7 @@ int run_host(int kind, const float* X, int N, const float* Y, int M, float R[9],
       L.TFACTOR = p->TFACTOR;
       L.moutlier = p->moutlier;
       L.form = form;
+      L.series = series_for(p->sinkhorn_form, form, N, M, tl_cap > 0);
       L.dRt = dRt;
       L.trace = dtrace;
       L.trace_cap = cap;
@@ -422,6 +431,7 @@ int batch_records(const cesa_pair* pairs, int npairs, std::vector<BatchLaunchPai
       L.T_0 = q.params.T_0;
       L.TFACTOR = q.params.TFACTOR;
       L.moutlier = q.params.moutlier;
+      L.series = q.params.sinkhorn_form == CESA_SINKHORN_AUTO && softassign_series_fits(q.N, q.M);
     } else {
       return CESA_ERR_INVALID_ARGUMENT;
     }
@@ -585,6 +595,7 @@ int cesa_softassign_device(const float* dX, int N, const float* dY, int M, float
   L.TFACTOR = p->TFACTOR;
   L.moutlier = p->moutlier;
   L.form = form;
+  L.series = series_for(p->sinkhorn_form, form, N, M, false);
   L.dRt = dRt;
   L.d_status = d_status;
   L.timeout_ns = timeout_ns_of(p);

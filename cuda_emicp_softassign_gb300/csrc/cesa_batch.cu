@@ -73,6 +73,8 @@ struct BPair {
   float *a, *s, *rs;  // Softassign rows [N]
   float *b, *u, *cs;  // Softassign columns [M]
   float* state;
+  int series;
+  const SeriesHand* hand;  // Softassign: where the series kernel stopped (null: it did not run)
 };
 
 struct BatchArgs {
@@ -87,6 +89,7 @@ struct BatchArgs {
 
 struct Sched {
   int algo, rounds, I1, units0, units1;
+  int done;  // pose updates the series kernel ran
 };
 
 struct Ph {
@@ -105,7 +108,7 @@ __device__ __forceinline__ Ph phase_of(const Sched& s, int r) {
   }
   const int per = 2 * s.I1 + 2;
   const int upd = r / per, k = r - upd * per;
-  p.step = upd;
+  p.step = upd + s.done;
   if (k < 2 * s.I1) {
     p.k = k >> 1;
     if (k & 1) {
@@ -659,18 +662,25 @@ __global__ void __launch_bounds__(kThreads, 2) batch_kernel(const BatchArgs A) {
   __shared__ df s_red[kThreads];
   __shared__ df s_tot[kSaNV];
   __shared__ float s_S[9], s_v[12];
+  __shared__ int s_rounds;
 
   const int tid = threadIdx.x;
   const int G = (int)gridDim.x;
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
     mbar_init_fence();
-  }
-  for (int p = tid; p < A.npairs; p += kThreads) {
-    const BPair& P = A.pairs[p];
-    s_sched[p] = Sched{P.algo, P.rounds, P.I1, P.g0.units, P.g1.units};
+    s_rounds = 0;
   }
   __syncthreads();
+  for (int p = tid; p < A.npairs; p += kThreads) {
+    const BPair& P = A.pairs[p];
+    const int done = P.hand ? P.hand->titer * P.I0 + P.hand->iter0 : 0;
+    s_sched[p] = Sched{P.algo, P.algo == 0 ? P.rounds : P.rounds - done * (2 * P.I1 + 2), P.I1, P.g0.units, P.g1.units,
+                       done};
+    atomicMax(&s_rounds, s_sched[p].rounds);
+  }
+  __syncthreads();
+  const int rounds = s_rounds;  // of what is left, over the pairs
 
   Ring rg{{0u, 0u}, 0};
   unsigned epoch = 0;
@@ -684,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, 2) batch_kernel(const BatchArgs A) {
   __shared__ Task s_tn;
   unsigned pending = 0;  // thread 0: next unit of this round
   if (tid == 0) pending = (unsigned)G + atomicAdd(&A.rctr[0], 1u);
-  for (int r = 0; r < A.rounds && ok; ++r) {
+  for (int r = 0; r < rounds && ok; ++r) {
     // Weights copied by TMA this round were written by other blocks in earlier
     // rounds (generic proxy, ordered by the grid barrier); the proxy fence
     // makes them visible to the async proxy of the copies thread 0 issues.
@@ -744,7 +754,7 @@ __global__ void __launch_bounds__(kThreads, 2) batch_kernel(const BatchArgs A) {
         slot = ns;
       }
     }
-    if (tid == 0 && r + 1 < A.rounds) pending = (unsigned)G + atomicAdd(&A.rctr[r + 1], 1u);
+    if (tid == 0 && r + 1 < rounds) pending = (unsigned)G + atomicAdd(&A.rctr[r + 1], 1u);
     ok = ok && grid_sync(A.ctl, epoch, (unsigned)G, A.timeout_ns, 70);
   }
   if (blockIdx.x == 0 && tid == 0) {
@@ -838,7 +848,7 @@ int batch_slice(const BatchLaunchPair* in, int npairs, int G) {
 // The pair table is ordered by decreasing size, so the largest units of a
 // round are handed out first. With base == nullptr only sizes are computed.
 size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std::vector<BPair>* out, Ctl** ctl,
-                   size_t* zero_bytes, BPair** dpairs, int* rounds, unsigned** rctr) {
+                   size_t* zero_bytes, BPair** dpairs, int* rounds, unsigned** rctr, void** series_tab) {
   Carve c(base);
   *ctl = c.take<Ctl>(1);
   const int slice = batch_slice(in, npairs, G);
@@ -878,6 +888,7 @@ size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std
       P.moutlier = L.moutlier;
       P.I0 = L.I0;
       P.I1 = L.I1;
+      P.series = L.series;
     }
     ncnt += (size_t)P.g0.nblk + (size_t)P.g1.nblk;
     P.X = L.dX;
@@ -887,8 +898,10 @@ size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std
   }
   unsigned* cnt = c.take<unsigned>(ncnt > 0 ? ncnt : 1);
   *rctr = c.take<unsigned>((size_t)rmax + 1);
+  SeriesHand* hand = c.take<SeriesHand>((size_t)npairs);
   *zero_bytes = c.off;
   *dpairs = c.take<BPair>((size_t)npairs);
+  *series_tab = c.take<char>(softassign_series_table_bytes(npairs));
   size_t co = 0;
   for (int i = 0; i < npairs; ++i) {
     BPair& P = v[(size_t)i];
@@ -914,6 +927,7 @@ size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std
       P.b = c.take<float>(Mp);
       P.u = c.take<float>(Mp);
       P.cs = c.take<float>(Mp);
+      if (P.nsteps > 0 && P.series) P.hand = hand ? hand + i : nullptr;
     }
     P.state = c.take<float>(kStateFloats);
   }
@@ -934,8 +948,9 @@ size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device) {
   BPair* dp = nullptr;
   int rounds = 0;
   unsigned* rctr = nullptr;
+  void* stab = nullptr;
   const int G = persistent_grid_limit(device, (const void*)batch_kernel, batch_smem(npairs));
-  return carve_batch(nullptr, pairs, npairs, G, nullptr, &ctl, &zb, &dp, &rounds, &rctr);
+  return carve_batch(nullptr, pairs, npairs, G, nullptr, &ctl, &zb, &dp, &rounds, &rctr, &stab);
 }
 
 int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint64_t timeout_ns, void* ws,
@@ -950,9 +965,10 @@ int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint6
   BPair* dpairs = nullptr;
   int rounds = 0;
   unsigned* rctr = nullptr;
+  void* stab = nullptr;
   const size_t smem = batch_smem(npairs);
   const int limit = persistent_grid_limit(device, (const void*)batch_kernel, smem);
-  const size_t need = carve_batch(ws, pairs, npairs, limit, &host, &ctl, &zero_bytes, &dpairs, &rounds, &rctr);
+  const size_t need = carve_batch(ws, pairs, npairs, limit, &host, &ctl, &zero_bytes, &dpairs, &rounds, &rctr, &stab);
   if (need > ws_bytes) return (int)cudaErrorInvalidValue;
   if (rounds_out) *rounds_out = rounds;
   e = cudaMemsetAsync(ws, 0, zero_bytes, st);
@@ -965,6 +981,18 @@ int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint6
   if (e != cudaSuccess) return (int)e;
   if (grid_used) *grid_used = limit;
   if (rounds == 0) return 0;
+  // The leading updates of the Softassign pairs, as far as a short series
+  // represents their affinities: a cluster per pair, before the lock-step
+  // rounds (which then hold the EM-ICP pairs and what is left).
+  std::vector<SeriesJob> jobs;
+  for (const BPair& P : host)
+    if (P.hand)
+      jobs.push_back(SeriesJob{P.own0, P.own1, P.hdr, P.dRt, P.s, P.u, P.state, const_cast<SeriesHand*>(P.hand), P.N,
+                               P.M, P.nsteps / P.I0, P.I0, P.I1, P.alpha, P.init, P.TFACTOR, P.moutlier});
+  if (!jobs.empty()) {
+    const int r = enqueue_softassign_series_batch(jobs.data(), (int)jobs.size(), stab, ctl, st);
+    if (r) return r;
+  }
   BatchArgs A;
   A.pairs = dpairs;
   A.npairs = npairs;

@@ -101,6 +101,35 @@ __device__ __forceinline__ void df_add(df& a, const df& b) {
 __device__ __forceinline__ float df_val(const df& a) { return __fadd_rn(a.hi, a.lo); }
 __device__ __forceinline__ double df_dbl(const df& a) { return (double)a.hi + (double)a.lo; }
 
+// Pair arithmetic beyond sums (dd_*): results to ~45 bits.
+__device__ __forceinline__ df dd_fast(float a, float b) {  // a + b, |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return df{s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ df dd_sum(float a, float b) {
+  df r = df_make(a);
+  df_add(r, b);
+  return r;
+}
+__device__ __forceinline__ df dd_mul(df a, df b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, e));
+  return dd_fast(p, e);
+}
+// a / b; inv: 1 / b.hi to about FP32, or 0 where b.hi is outside [1e-30, 1e30] (then
+// a plain division of the leading parts, which keeps infinities and zeros).
+__device__ __forceinline__ df dd_div(df a, df b, float inv) {
+  if (inv == 0.f) return df_make(a.hi / b.hi);
+  const float q = __fmul_rn(a.hi, inv);
+  float r = __fmaf_rn(-q, b.hi, a.hi);
+  r = __fmaf_rn(-q, b.lo, __fadd_rn(r, a.lo));
+  return dd_fast(q, __fmul_rn(r, inv));
+}
+__device__ __forceinline__ float dd_inv(df b) {
+  return fabsf(b.hi) > 1e-30f && fabsf(b.hi) < 1e30f ? __fdividef(1.f, b.hi) : 0.f;
+}
+
 __device__ __forceinline__ df df_shfl_down(const df& a, int off) {
   return df{__shfl_down_sync(0xffffffffu, a.hi, off), __shfl_down_sync(0xffffffffu, a.lo, off)};
 }

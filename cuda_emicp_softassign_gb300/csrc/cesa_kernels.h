@@ -72,6 +72,7 @@ struct SoftassignLaunch {
   int JMAX, I0, I1;
   float alpha, T_0, TFACTOR, moutlier;
   int form;          // CESA_SINKHORN_MATRIX_FREE / _MATERIALISED (resolved)
+  int series;        // run the leading updates in the series kernel where it applies
   float* dRt;        // PoseIO in/out (device)
   float* s_io;       // optional slack column in/out [N] (else initialised to moutlier)
   float* u_io;       // optional slack row in/out [M]
@@ -102,6 +103,38 @@ struct SoftassignLaunch {
 //   20-22 Xc - oX  23-25 Yc - oY  26-34 S  35-38 q  39-54 Horn eigenbasis V[4][4]
 constexpr int kSaTape = 64;
 
+// Where the series kernel stopped: the affinity kernels run the schedule from
+// pose update iter0 of temperature step titer on, from this pose (centred
+// frame). All zeros: the start of the schedule, pose from the caller.
+struct SeriesHand {
+  int titer, iter0;
+  float pose[12];
+};
+// The leading pose updates of a schedule whose affinities a short series
+// represents (cesa_softassign_series.cu). Fits when both clouds' shares fit
+// the shared memory of one cluster.
+bool softassign_series_fits(int N, int M);
+// max_degree: the highest degree of the series that is worth it against the
+// affinity kernel that would run the update instead.
+int enqueue_softassign_series(const SoftassignLaunch& L, const float4* rows, const float4* cols, const CenterHdr* hdr,
+                              float* s_out, float* u_out, SeriesHand* hand, int max_degree, void* ctl,
+                              cudaStream_t st);
+// The same for the Softassign pairs of a batch, one cluster each. `state`
+// receives the pose (12, centred) and temperature reached; dRt the final pose
+// where the whole schedule ran here.
+struct SeriesJob {
+  const float4* rows;
+  const float4* cols;
+  const CenterHdr* hdr;
+  float* dRt;
+  float *s, *u, *state;
+  SeriesHand* hand;
+  int N, M, JMAX, I0, I1;
+  float alpha, T0, TFACTOR, moutlier;
+};
+size_t softassign_series_table_bytes(int njobs);
+int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_table, void* ctl, cudaStream_t st);
+
 // One pair of a batched launch (device pointers).
 constexpr int kMaxBatchPairs = 1024;
 struct BatchLaunchPair {
@@ -114,6 +147,7 @@ struct BatchLaunchPair {
   float sigma_p2, sigma_factor, d_02;
   int JMAX, I0, I1;  // Softassign
   float alpha, T_0, TFACTOR, moutlier;
+  int series;        // Softassign: run the leading updates in the series kernel where it applies
 };
 
 // Sinkhorn forms of SoftassignLaunch.form (the CESA_SINKHORN_* values).

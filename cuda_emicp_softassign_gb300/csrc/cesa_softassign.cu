@@ -56,6 +56,7 @@ struct SoftArgs {
   int JMAX, I0, I1;
   float alpha, T0, TFACTOR;
   const CenterHdr* hdr;
+  const SeriesHand* hand;  // optional: where the series kernel stopped
   float* dRt;
   float* pr;           // row-pass partials [S_r][Np]; ranged: [nblk_r][kmax_r][128]
   float* pc;           // column-pass partials [S_c][Mp]; ranged: [nblk_c][kmax_c][128]
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_kernel(const SoftArgs 
   __shared__ RangedShare rs_rows, rs_cols;  // this block's shares of the ranged Sinkhorn passes
   __shared__ float s_hdr[12];
   __shared__ SaPoseScratch ps;
+  __shared__ int s_start[2];  // first pose update: temperature step, update within it
 
   const int tid = threadIdx.x;
   const unsigned G = gridDim.x;
@@ -364,6 +366,12 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_kernel(const SoftArgs 
     pose_to_centred(R, t, &s_hdr[0], &s_hdr[3], tc);
     for (int k = 0; k < 9; ++k) s_pose[k] = R[k];
     for (int k = 0; k < 3; ++k) s_pose[9 + k] = tc[k];
+    s_start[0] = s_start[1] = 0;
+    if (A.hand && (A.hand->titer > 0 || A.hand->iter0 > 0)) {
+      s_start[0] = A.hand->titer;
+      s_start[1] = A.hand->iter0;
+      for (int k = 0; k < 12; ++k) s_pose[k] = A.hand->pose[k];
+    }
   }
   __shared__ HornState<float> horn;  // carried eigenbasis (thread 0)
   if (tid == 0) {
@@ -383,12 +391,13 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_kernel(const SoftArgs 
   const StreamSrc src_cols{A.cols, nullptr, false};
   const StreamSrc src_rows{A.rows, nullptr, false};
   float T = A.T0;
-  int step = 0;
+  for (int k = 0; k < s_start[0]; ++k) T = T * A.TFACTOR;  // FP32, as below
+  int step = s_start[0] * A.I0 + s_start[1];
   bool ok = true;
   Timeline tl{A.tl, A.tl_cap, 0};
   const int Np = A.Np, Mp = A.Mp;
 
-  for (int Titer = 0; Titer < A.JMAX && ok; ++Titer) {
+  for (int Titer = s_start[0]; Titer < A.JMAX && ok; ++Titer) {
     // K = exp((alpha - d^2)/T) / sqrt(T) = 2^(c0 + nk d^2) = 2^c0 2^-|x' - y'|^2
     // for clouds scaled by sc = sqrt(-nk): the sweeps see the scaled clouds,
     // and 2^c0 is folded into the streamed weights (a_r, b_c and the final
@@ -397,7 +406,7 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_kernel(const SoftArgs 
     const float c0 = fmaf(A.alpha, kk, -0.5f * log2f(T));
     const float sc = sqrtf(kk), wsc = exp2f(c0);
     const float Rdg[9] = {sc, 0.f, 0.f, 0.f, sc, 0.f, 0.f, 0.f, sc}, z3[3] = {0.f, 0.f, 0.f};  // owned X rows
-    for (int iter0 = 0; iter0 < A.I0 && ok; ++iter0, ++step) {
+    for (int iter0 = Titer == s_start[0] ? s_start[1] : 0; iter0 < A.I0 && ok; ++iter0, ++step) {
       tl.mark(1);
       float R[9], tc[3];  // the pose, times sc
 #pragma unroll
@@ -591,6 +600,7 @@ struct SaCarved {
   Ctl* ctl;
   unsigned* cnt_f;
   CenterHdr* hdr;
+  SeriesHand* hand;
   float4* rows;
   float4* cols;
   float *abuf, *bbuf, *sbuf, *ubuf, *rs, *cs;
@@ -614,6 +624,7 @@ SaCarved carve_sa(void* base, const SaPlan& P, int N, int M, size_t* total) {
   w.ctl = c.take<Ctl>(1);
   w.cnt_f = c.take<unsigned>((size_t)P.gf.nblk);
   w.hdr = c.take<CenterHdr>(1);
+  w.hand = c.take<SeriesHand>(1);
   w.rows = c.take<float4>((size_t)N);
   w.cols = c.take<float4>((size_t)M);
   w.abuf = c.take<float>((size_t)2 * w.Np);
@@ -681,8 +692,16 @@ int enqueue_softassign(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cud
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   if (L.JMAX <= 0 || L.I0 <= 0) return 0;
+  if (L.series) {
+    e = cudaMemsetAsync(w.hand, 0, sizeof(SeriesHand), st);
+    if (e != cudaSuccess) return (int)e;
+    constexpr int kSeriesDegree = 8;  // all it has: this kernel takes 45 us an update and more
+    const int r = enqueue_softassign_series(L, w.rows, w.cols, w.hdr, w.sbuf, w.ubuf, w.hand, kSeriesDegree, w.ctl, st);
+    if (r) return r;
+  }
 
   SoftArgs A;
+  A.hand = L.series ? w.hand : nullptr;
   A.rows = w.rows;
   A.cols = w.cols;
   A.abuf = w.abuf;

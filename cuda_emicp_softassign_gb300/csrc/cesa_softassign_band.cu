@@ -50,6 +50,7 @@ struct BandArgs {
   const float4* rows;  // X' centred (N)
   const float4* cols;  // Y' centred (M)
   const CenterHdr* hdr;
+  const SeriesHand* hand;  // optional: where the series kernel stopped
   float* dRt;
   int N, M, Mp;
   int nb, CS, W;       // bands, CTAs per cluster (column tiles), tile width
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_band_kernel(const Band
   __shared__ df s_tot[kSaNV];
   __shared__ SaPoseScratch ps;
   __shared__ HornState<float> horn;
+  __shared__ int s_start[2];  // first pose update: temperature step, update within it
 
   const int tid = threadIdx.x;
   const int CS = A.CS;
@@ -339,6 +341,12 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_band_kernel(const Band
     pose_to_centred(R, t, &s_hdr[0], &s_hdr[3], tc);
     for (int k = 0; k < 9; ++k) s_pose[k] = R[k];
     for (int k = 0; k < 3; ++k) s_pose[9 + k] = tc[k];
+    s_start[0] = s_start[1] = 0;
+    if (A.hand && (A.hand->titer > 0 || A.hand->iter0 > 0)) {
+      s_start[0] = A.hand->titer;
+      s_start[1] = A.hand->iter0;
+      for (int k = 0; k < 12; ++k) s_pose[k] = A.hand->pose[k];
+    }
     horn.reset();
   }
   __syncthreads();
@@ -346,18 +354,19 @@ __global__ void __launch_bounds__(kThreads, 2) softassign_band_kernel(const Band
   own_pairs(sm.xr, qx);
 
   unsigned epoch = 0, gepoch = 0, cpass = 0;
-  int xpar = 0, step = 0;
+  int xpar = 0, step = s_start[0] * A.I0 + s_start[1];
   bool ok = true;
   float T = A.T0;
+  for (int k = 0; k < s_start[0]; ++k) T = T * A.TFACTOR;  // FP32, as below
   Timeline tl{A.tl, A.tl_cap, 0};
   const size_t pc_stride = (size_t)A.nb * A.Mp;
 
-  for (int Titer = 0; Titer < A.JMAX; ++Titer) {
+  for (int Titer = s_start[0]; Titer < A.JMAX; ++Titer) {
     // K = exp((alpha - d^2)/T) / sqrt(T) = 2^(cK + nk d^2)
     const float kk2 = kLog2e / T;
     const float nk = -kk2;
     const float cK = fmaf(A.alpha, kk2, -0.5f * log2f(T));
-    for (int iter0 = 0; iter0 < A.I0; ++iter0, ++step) {
+    for (int iter0 = Titer == s_start[0] ? s_start[1] : 0; iter0 < A.I0; ++iter0, ++step) {
       tl.mark(1);
       float R[9], tc[3];
 #pragma unroll
@@ -622,8 +631,10 @@ BandPlan plan_band(int N, int M, int device) {
 struct BandCarved {
   Ctl* ctl;
   CenterHdr* hdr;
+  SeriesHand* hand;
   float4* rows;
   float4* cols;
+  float *s, *u;  // the slack that the series kernel hands over
   float* pc;
   df* mom;
   unsigned* gbar;
@@ -643,6 +654,9 @@ BandCarved carve_band(void* base, const BandPlan& P, int N, int M, size_t* total
   w.hdr = static_cast<CenterHdr*>(take(sizeof(CenterHdr)));
   w.rows = static_cast<float4*>(take(sizeof(float4) * (size_t)N));
   w.cols = static_cast<float4*>(take(sizeof(float4) * (size_t)M));
+  w.hand = static_cast<SeriesHand*>(take(sizeof(SeriesHand)));
+  w.s = static_cast<float*>(take(sizeof(float) * (size_t)N));
+  w.u = static_cast<float*>(take(sizeof(float) * (size_t)M));
   w.pc = static_cast<float*>(take(sizeof(float) * 2 * (size_t)P.nb * w.Mp));
   w.mom = static_cast<df*>(take(sizeof(df) * 2 * (size_t)P.nb * 32));
   w.gbar = static_cast<unsigned*>(take(sizeof(unsigned) * 32 * (size_t)P.CS));
@@ -691,7 +705,16 @@ int enqueue_softassign_band(const SoftassignLaunch& L, void* ws, size_t ws_bytes
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   if (L.JMAX <= 0 || L.I0 <= 0) return 0;
+  if (L.series) {
+    e = cudaMemsetAsync(w.hand, 0, sizeof(SeriesHand), st);
+    if (e != cudaSuccess) return (int)e;
+    // at ~26 us an update the banded kernel is overtaken by the series' higher degrees (P = 120 terms and more)
+    constexpr int kSeriesDegree = 6;
+    const int r = enqueue_softassign_series(L, w.rows, w.cols, w.hdr, w.s, w.u, w.hand, kSeriesDegree, w.ctl, st);
+    if (r) return r;
+  }
   BandArgs A;
+  A.hand = L.series ? w.hand : nullptr;
   A.rows = w.rows;
   A.cols = w.cols;
   A.hdr = w.hdr;
@@ -709,8 +732,8 @@ int enqueue_softassign_band(const SoftassignLaunch& L, void* ws, size_t ws_bytes
   A.T0 = L.T_0;
   A.TFACTOR = L.TFACTOR;
   A.moutlier = L.moutlier;
-  A.s_in = L.s_io;
-  A.u_in = L.u_io;
+  A.s_in = L.series ? w.s : L.s_io;
+  A.u_in = L.series ? w.u : L.u_io;
   A.s_out = L.s_io;
   A.u_out = L.u_io;
   A.rs_out = L.rs_out;
