@@ -32,7 +32,7 @@ SOURCES = ["cesa_api.cu", "cesa_emicp.cu", "cesa_softassign.cu", "cesa_noalloc.c
            "cesa_softassign_adjoint.cu", "cesa_icp.cu", "cesa_io.cpp", "cesa_softassign_band.cu",
            "cesa_softassign_series.cu"]
 HEADERS = ["cesa_common.cuh", "cesa_sweep.cuh", "cesa_pose.h", "cesa_kernels.h", "cesa_prep.cuh", "cesa_ops.cuh",
-           "cesa_sa_pose.cuh"]
+           "cesa_sa_pose.cuh", "cesa_pose_dd.cuh"]
 
 
 def nvcc():

@@ -28,6 +28,7 @@
 #include "cesa_kernels.h"
 #include "cesa_ops.cuh"
 #include "cesa_pose.h"
+#include "cesa_pose_dd.cuh"
 #include "cesa_prep.cuh"
 
 namespace cesa {
@@ -41,8 +42,8 @@ struct EmicpArgs {
   int nsteps;
   const CenterHdr* hdr;
   float* dRt;           // PoseIO in/out, caller frame
-  float* part;          // row partials [5][S][Mp] (accumulator, column slice, row); ranged: [5][nblk][kmax][128]
-  float4* xs;           // ranged sweeps: X' scaled for the step, [2][N] by step parity
+  float* part;          // row partials [5][S][Mp] (accumulator, column slice, row); ranged: [5][nblk][kmax][kBlockPts]
+  const float4* blk;    // local sweeps: centre and radius of every owned block's rows (null: the plain sweep)
   int Mp;
   df* rbpart;           // [2][grid][kEmNV] moments per block (step parity)
   Ctl* ctl;
@@ -59,17 +60,244 @@ struct EmicpArgs {
   uint64_t timeout_ns;
 };
 
+// ---------------------------------------------------------------- local sweep
+// The E-step sweep on clouds scaled by sc = sqrt(log2(e) / (2 sigma_p2)), each
+// owned block about a centre c' of its own (its posed box centre, scaled):
+//   e = 2^-|x' - z'|^2 = 2^-|z~|^2 2^(2 z~.x~ - |x~|^2),  x~ = x' - c', z~ = z' - c'.
+// The prepare step streams (x~, -|x~|^2), lanes own 2 z~, and the row factor
+// 2^-|z~|^2 multiplies a row's sums once: 3 FFMA for the exponent in place of
+// 3 FADD + FMUL + 2 FFMA, 8 FP32 ops per element in place of 11. It is taken
+// while the block's scaled radius is at most sqrt(kLocalR2), where 2^|z~|^2
+// cannot overflow a sum of e^2 and the rounding of |x~|^2 (of affinities that
+// count, |x~| < 6 + radius) stays at the level of the coordinates' own;
+// otherwise the block sweeps direct differences (EmicpElemScaled). Y is sorted
+// along a Hilbert curve so that blocks are compact: at N = M = 40,097 98% of the
+// default schedule's affinities take the short form, at 8171 points 91%.
+// Bound by the FP32 pipe as before (72% of it busy where every block is short,
+// 23.0 instructions per 128 elements against 29.5): N = M = 40,097 36.3 -> 30.9
+// ms, 17,000 8.75 -> 7.57, 8171 x 6007 1.97 -> 1.86. Not kept: 8 owned points a
+// lane (256 per unit 33.0 ms, or 128 over half-warps 33.4, at their best pair
+// splits), records stored as packed duplicates (35.4), kLocalR2 = 16 (32.1).
+constexpr float kLocalR2 = 48.f;
+
+// Poses of the local form are refined in the last steps, where sigma is small
+// and their errors reach the result (the ones of earlier steps are contracted
+// away): the short form's rounding is then more than made up for. ~2 us a step.
+constexpr int kRefineSteps = 16;
+
+struct EmicpElemLocal {  // q = 2 z~ of two owned points; s = (x~, -|x~|^2)
+  __device__ __forceinline__ void operator()(float2 (&acc)[5], const float2 (&q)[3], float4 s) const {
+    float2 t = __ffma2_rn(q[2], dup2(s.z), dup2(s.w));
+    t = __ffma2_rn(q[1], dup2(s.y), t);
+    const float2 e = ex2_pair(__ffma2_rn(q[0], dup2(s.x), t));
+    acc[0] = __ffma2_rn(e, e, acc[0]);
+    acc[1] = __fadd2_rn(acc[1], e);
+    acc[2] = __ffma2_rn(e, dup2(s.x), acc[2]);
+    acc[3] = __ffma2_rn(e, dup2(s.y), acc[3]);
+    acc[4] = __ffma2_rn(e, dup2(s.z), acc[4]);
+  }
+};
+
+struct LocalSmem {
+  float rho[2][kBlockPts];  // the owned points' |z~|^2, by unit parity
+};
+
+// As sweep_units (deferred), for the EM-ICP E-step: every unit's partial sums
+// of e^2, e and e x' (scaled frame) are stored per (row, slice or slot).
+template <int kLayout>
+__device__ __forceinline__ bool em_local_sweep(SweepSmem& sm, LocalSmem& ls, Pipe& pipe, const SweepGeom& g,
+                                               const StreamSrc& src, const float4* own, const float4* blkinfo,
+                                               const float (&R)[9], const float (&tc)[3], float sc, float* part,
+                                               int part_ld, Ctl* ctl, uint64_t timeout_ns, int where, Timeline& tl,
+                                               OwnCache& oc, const RangedShare* rs) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int G = (int)gridDim.x;
+  constexpr bool ranged = kLayout == 1;
+  pipe.cur = -1;
+  auto task_range = [&](int uu, int ch, int& first, int& len) -> bool {  // as in sweep_units
+    if (ranged) {
+      const int o = rs->o_first + uu;
+      const int o_last = rs->o_last;
+      if (o > o_last) return false;
+      const int c = (uu == 0 ? rs->c_first : 0) + ch;
+      if (c >= (o == o_last ? rs->c_end : g.nch)) return false;
+      first = c * kChunk;
+      len = min(kChunk, g.n_stream - first);
+      return true;
+    }
+    if (uu >= g.units) return false;
+    const int sl = uu % g.slices;
+    const int sb = sl * g.slice_len;
+    const int se = min(sb + g.slice_len, g.n_stream);
+    first = sb + ch * kChunk;
+    if (first >= se) return false;
+    len = min(kChunk, se - first);
+    return true;
+  };
+  const int ustep = ranged ? 1 : G;
+  int u = ranged ? 0 : (int)blockIdx.x;
+  int cur_first = 0, cur_len = 0, cur_ch = 0, cur_stage = 0;
+  unsigned cur_par = 0;
+  bool cur_wait = false;
+  int par = 0, upar = 0;
+  bool have = task_range(u, 0, cur_first, cur_len);
+  if (have) {
+    cur_stage = pipe_issue(pipe, sm, src, cur_first, cur_first, cur_len, cur_wait);
+    cur_par = (pipe.uses[cur_stage] - 1u) & 1u;
+  }
+  while (have) {
+    const int blk = ranged ? rs->o_first + u : u / g.slices, sl = ranged ? u : u % g.slices;
+    float4 ow[kOwnPerLane];
+    load_owned_cached(oc, own, g.n_own, blk, ow);
+    const float4 bi = __ldg(blkinfo + blk);
+    const float cx = R[0] * bi.x + R[1] * bi.y + R[2] * bi.z + tc[0];
+    const float cy = R[3] * bi.x + R[4] * bi.y + R[5] * bi.z + tc[1];
+    const float cz = R[6] * bi.x + R[7] * bi.y + R[8] * bi.z + tc[2];
+    const bool local = bi.w * bi.w * sc * sc <= kLocalR2;  // false for NaN; the same in every thread
+    float2 q[kPairs][3];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+      float p[2][3];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = 2 * k + h, i = lane + 32 * j;
+        p[h][0] = R[0] * ow[j].x + R[1] * ow[j].y + R[2] * ow[j].z + tc[0];
+        p[h][1] = R[3] * ow[j].x + R[4] * ow[j].y + R[5] * ow[j].z + tc[1];
+        p[h][2] = R[6] * ow[j].x + R[7] * ow[j].y + R[8] * ow[j].z + tc[2];
+        if (local) {
+          const bool in = blk * kBlockPts + i < g.n_own;  // padding rows sit at the centre
+          p[h][0] = in ? p[h][0] - cx : 0.f;
+          p[h][1] = in ? p[h][1] - cy : 0.f;
+          p[h][2] = in ? p[h][2] - cz : 0.f;
+          if (warp == 0) ls.rho[upar][i] = fmaf(p[h][2], p[h][2], fmaf(p[h][1], p[h][1], p[h][0] * p[h][0]));
+        }
+      }
+      const float f = local ? 2.f : -1.f;  // the scaled element takes the negated coordinates
+#pragma unroll
+      for (int c = 0; c < 3; ++c) q[k][c] = make_float2(f * p[0][c], f * p[1][c]);
+    }
+    float2 acc[kPairs][5];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+#pragma unroll
+      for (int a = 0; a < 5; ++a) acc[k][a] = make_float2(0.f, 0.f);
+
+    for (;;) {
+      int n_first = 0, n_len = 0, n_u = u, n_ch = cur_ch + 1, n_stage = 0;
+      unsigned n_par = 0;
+      bool n_wait = false;
+      bool have_n = task_range(n_u, n_ch, n_first, n_len);
+      if (!have_n) {
+        n_u = u + ustep;
+        n_ch = 0;
+        have_n = task_range(n_u, 0, n_first, n_len);
+      }
+      pipe.cur = cur_stage;
+      if (have_n) {
+        n_stage = pipe_issue(pipe, sm, src, n_first, n_first, n_len, n_wait);
+        n_par = (pipe.uses[n_stage] - 1u) & 1u;
+      }
+      const bool bad = cur_wait && !mbar_wait(&sm.full[cur_stage], cur_par, ctl, timeout_ns, where);
+      if (cur_ch == 0 && u == (int)blockIdx.x) tl.mark(2);
+      // prepare: double-buffered, one block barrier per chunk (a stage that
+      // timed out is read as it is; the block leaves after the barrier)
+      float4* buf = par ? sm.prep2 : sm.prep;
+      par ^= 1;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = tid + h * kThreads;
+        if (c < cur_len) {
+          const float4 x = sm.raw[cur_stage][c];
+          float4 o;
+          if (local) {
+            o.x = fmaf(x.x, sc, -cx);
+            o.y = fmaf(x.y, sc, -cy);
+            o.z = fmaf(x.z, sc, -cz);
+            o.w = -fmaf(o.z, o.z, fmaf(o.y, o.y, o.x * o.x));
+          } else {
+            o = make_float4(x.x * sc, x.y * sc, x.z * sc, 0.f);
+          }
+          buf[c] = o;
+        }
+      }
+      if (__syncthreads_or(bad)) {
+        // leave only after the prefetched copy (if any) has landed
+        if (have_n && n_wait) mbar_wait(&sm.full[n_stage], n_par, ctl, timeout_ns, where + 1);
+        return false;
+      }
+      if (local) {
+        const EmicpElemLocal elem{};
+#pragma unroll 8
+        for (int c = warp; c < cur_len; c += kWarps) {
+          const float4 a = buf[c];
+#pragma unroll
+          for (int k = 0; k < kPairs; ++k) elem(acc[k], q[k], a);
+        }
+      } else {
+        const EmicpElemScaled elem{};
+#pragma unroll 8
+        for (int c = warp; c < cur_len; c += kWarps) {
+          const float4 a = buf[c];
+#pragma unroll
+          for (int k = 0; k < kPairs; ++k) elem(acc[k], q[k], a, a);
+        }
+      }
+      const bool unit_done = !(have_n && n_u == u);
+      cur_first = n_first;
+      cur_len = n_len;
+      cur_ch = n_ch;
+      cur_stage = n_stage;
+      cur_par = n_par;
+      cur_wait = n_wait;
+      have = have_n;
+      if (unit_done) break;
+    }
+    tl.mark(3);
+    float tot[5];
+    reduce_warps<5>(sm, acc, tot);
+    const int i = blk * kBlockPts + tid;
+    if (tid < kBlockPts && i < g.n_own) {
+      if (local) {  // the row factor, and x~ back to x'
+        const float rho = ex2_approx(-ls.rho[upar][tid]);
+        tot[0] *= rho * rho;
+        tot[1] *= rho;
+        tot[2] = fmaf(tot[1], cx, tot[2] * rho);
+        tot[3] = fmaf(tot[1], cy, tot[3] * rho);
+        tot[4] = fmaf(tot[1], cz, tot[4] * rho);
+      }
+      if (ranged) {  // slot (owned block, j): this block is the j-th to cover it
+        const int j = sl == 0 ? rs->j_first : 0;
+        if (j < g.kmax) {
+#pragma unroll
+          for (int a = 0; a < 5; ++a) __stcg(part + (((size_t)a * g.nblk + blk) * g.kmax + j) * kBlockPts + tid, tot[a]);
+        } else {
+          set_status(ctl, kStatusInternal, where + 3);  // the plan's kmax is inconsistent
+        }
+      } else {
+#pragma unroll
+        for (int a = 0; a < 5; ++a) __stcg(part + ((size_t)a * g.slices + sl) * part_ld + i, tot[a]);
+      }
+    }
+    upar ^= 1;
+    tl.mark(4);
+    u += ustep;
+    cur_ch = 0;
+  }
+  return true;
+}
+
 __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
   __shared__ float s_pose[12];
   __shared__ df s_red[kThreads];
   __shared__ OwnCache oc_rows;
+  __shared__ LocalSmem s_local;
   __shared__ RangedShare rs_rows;  // this block's share of a ranged sweep
   __shared__ int s_pair[3];        // SM pairs: pair index (-1: none), role, parts swapped
   __shared__ uint64_t s_tsweep;    // SM pairs: start of the step's sweep
   __shared__ df s_tot[kEmNV];
-  __shared__ float s_emS[15];  // S, Xc, Yc of the step
+  __shared__ float s_emS[30];  // S, Xc, Yc of the step; their parts below FP32
   __shared__ float s_hdr[12];
 
   const int tid = threadIdx.x;
@@ -119,26 +347,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
   const StreamSrc src{A.cols, nullptr, true};
   float s2 = A.sigma0;
   Timeline tl{A.tl, A.tl_cap, 0};
-  // Ranged sweeps stream X' scaled by sc = sqrt(log2(e) / (2 s2)) (and scale the
-  // owned rows alike), so that an element needs no scale of its own. Each step's
-  // copy is written by all blocks during the previous step's row completion.
-  auto scale_x = [&](float4* dst, float sc) {
-    for (int i = (int)blockIdx.x * kThreads + tid; i < A.N; i += (int)G * kThreads) {
-      const float4 x = ld_cg(A.cols + i);
-      __stcg(dst + i, make_float4(x.x * sc, x.y * sc, x.z * sc, 0.f));
-    }
-  };
-  bool started = true;  // false: the barrier after the first scaled copy gave up
-  if (A.geo.ranged && A.nsteps > 0) {
-    scale_x(A.xs, sqrtf(kLog2e / (2.f * s2)));
-    started = grid_sync(A.ctl, epoch, G, A.timeout_ns, 22);
-  }
-
-  for (int step = 0; step < A.nsteps && started; ++step) {
+  for (int step = 0; step < A.nsteps; ++step) {
     tl.mark(1);
-    // the scaled X' was written by other blocks' ordinary stores, ahead of a
-    // grid barrier; the bulk copies that stream it read through the async proxy
-    if (A.geo.ranged && tid == 0) asm volatile("fence.proxy.async.global;" ::: "memory");
     const float outlier = expf(-A.d_02 / s2);  // src/emicp.cu:489
     float R[9], tc[3];
 #pragma unroll
@@ -150,18 +360,19 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     // e = exp(-d2 / (2 s2)) = 2^(nk d2). Every unit stores its rows' partial
     // sums over its column slice (deferred: no completion counter).
     const float sc = sqrtf(kLog2e / (2.f * s2));
-    if (A.geo.ranged) {
+    if (A.blk) {
       float Rs[9], tcs[3];
 #pragma unroll
       for (int k = 0; k < 9; ++k) Rs[k] = R[k] * sc;
 #pragma unroll
       for (int k = 0; k < 3; ++k) tcs[k] = tc[k] * sc;
-      const StreamSrc xsrc{A.xs + (size_t)(step & 1) * A.N, nullptr, false};
       if (tid == 0 && s_pair[0] >= 0) s_tsweep = global_ns();
-      if (!sweep_units<5, EmicpElemScaled, NoPrep, NoFin, true, 1>(sm, pipe, A.geo, xsrc, A.rows, true, Rs, tcs, 0u,
-                                                                A.part, nullptr, EmicpElemScaled{}, NoPrep{}, NoFin{},
-                                                                A.ctl, A.timeout_ns, 10, tl, A.Mp, &oc_rows, &rs_rows))
-        break;
+      const bool ok = A.geo.ranged
+                          ? em_local_sweep<1>(sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
+                                              A.ctl, A.timeout_ns, 10, tl, oc_rows, &rs_rows)
+                          : em_local_sweep<0>(sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
+                                              A.ctl, A.timeout_ns, 10, tl, oc_rows, nullptr);
+      if (!ok) break;
       if (tid == 0 && s_pair[0] >= 0)
         A.pair_t[2 * s_pair[0] + (s_pair[1] ^ s_pair[2])] = (float)(global_ns() - s_tsweep);
     } else {
@@ -182,10 +393,6 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
         rs_rows = ranged_share(A.geo, 2 * s_pair[0] + (s_pair[1] ^ s_pair[2]), (int)G);
       }
     }
-    // the next step's scaled X' (its buffer was last read by the previous step's sweep)
-    if (A.geo.ranged && step + 1 < A.nsteps)
-      scale_x(A.xs + (size_t)((step + 1) & 1) * A.N, sqrtf(kLog2e / (2.f * (s2 * A.sigma_factor))));
-
     // ---- rows completed, each block a contiguous share of them; its 16
     // moments are one record. Thread t first sums the slice partials of
     // (row, accumulator) pairs t, t + kThreads, ... (loads in flight together),
@@ -193,7 +400,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     df* rb = A.rbpart + (size_t)(step & 1) * G * kEmNV;
     {
       const int S = A.geo.slices;
-      const float inv_sc = 1.f / sc;
+      const float inv_sc = A.blk ? 1.f / sc : 1.f;  // local sweeps: the e x sums are sc times too large
       const int rpc = (A.M + (int)G - 1) / (int)G;
       const int r0 = (int)blockIdx.x * rpc;
       const int nrows = max(0, min(rpc, A.M - r0));
@@ -222,7 +429,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
 #pragma unroll
               for (int q = 0; q < 4; ++q) sum += w[q];
             }
-            stot[rr * 5 + a] = a >= 2 ? sum * inv_sc : sum;  // the scaled coordinates' sums
+            stot[rr * 5 + a] = a >= 2 ? sum * inv_sc : sum;
             continue;
           }
           const float* P = A.part + (size_t)a * S * A.Mp + r0 + c0 + rr;
@@ -242,14 +449,15 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) sum += w[j];  // adding the zeros leaves the sum unchanged
           }
-          stot[rr * 5 + a] = sum;
+          stot[rr * 5 + a] = a >= 2 ? sum * inv_sc : sum;
         }
         __syncthreads();
         if (tid < nr) {
           const int r = r0 + c0 + tid;
           const float tot[5] = {stot[tid * 5], stot[tid * 5 + 1], stot[tid * 5 + 2], stot[tid * 5 + 3],
                                 stot[tid * 5 + 4]};
-          emicp_row_finish(r, tot, ld_cg(A.rows + r), outlier, xm, A.row_out, oX, row_tape, v);
+          const float4 y = ld_cg(A.rows + r);
+          emicp_row_finish(r, __float_as_int(y.w), tot, y, outlier, xm, A.row_out, oX, row_tape, v);
         }
         __syncthreads();
       }
@@ -261,7 +469,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     // ---- grid-wide moments -> pose (every block computes the same pose)
     reduce_block_partials<kEmNV>(rb, (int)G, s_red, s_tot);
     tl.mark(6);
-    em_moments_to_S_block(s_tot, s_emS);
+    const bool refine = A.blk && step + kRefineSteps >= A.nsteps;
+    em_moments_to_S_block(s_tot, s_emS, refine);
     if (tid == 0) {
       float Xc[3], Yc[3], S[9];
       for (int k = 0; k < 9; ++k) S[k] = s_emS[k];
@@ -274,6 +483,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
       // and without a tape, so that both forwards agree bitwise
       horn_quaternion_fast<float>(S, horn, q, &gap, &lmax);
       quat_to_pose<float>(q, Xc, Yc, Rn, tn);
+      if (refine)
+        horn_refine_dd(s_emS, s_emS + 15, s_emS + 9, s_emS + 24, s_emS + 12, s_emS + 27, q, Rn, tn);
       if (A.tape && blockIdx.x == 0) {  // the step's inputs and solve for the adjoint
         // the adjoint's eigenbasis, from a Jacobi solve of the same S on its own
         // state (it does not feed back into the pose)
@@ -335,6 +546,207 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
   }
 }
 
+// ---------------------------------------------------------------- row order
+// Index of a cell of the 32^3 grid along the Hilbert curve, by Skilling's
+// transposition ("Programming the Hilbert curve", AIP Conf. Proc. 707, 2004).
+// Consecutive cells are neighbours, so that 128 consecutive points are compact:
+// at N = 40,097 98% of the default schedule's (block, step) pairs take the short
+// form, against 96% along a Morton curve (8171 points: 91% against 86%).
+__device__ __forceinline__ unsigned hilbert_index(unsigned (&x)[3]) {
+#pragma unroll
+  for (unsigned q = 16; q > 1; q >>= 1) {
+    const unsigned p = q - 1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      if (x[i] & q) {
+        x[0] ^= p;
+      } else {
+        const unsigned t = (x[0] ^ x[i]) & p;
+        x[0] ^= t;
+        x[i] ^= t;
+      }
+    }
+  }
+  x[1] ^= x[0];
+  x[2] ^= x[1];
+  unsigned t = 0;
+#pragma unroll
+  for (unsigned q = 16; q > 1; q >>= 1)
+    if (x[2] & q) t ^= q - 1;
+  unsigned key = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    x[i] ^= t;
+#pragma unroll
+    for (int b = 0; b < 5; ++b) key |= ((x[i] >> b) & 1u) << (3 * b + 2 - i);
+  }
+  return key;
+}
+
+// Order of Y along a Hilbert curve of 32^3 cells over its bounding cube: a
+// stable radix sort of 15-bit keys (two 8-bit digits) by one block, warp w on
+// the w-th contiguous segment, so that the order does not depend on timing.
+// perm receives it (tmp: scratch of M). One block: 40,097 points take about
+// 0.1% of the registration that they are sorted for.
+__global__ void __launch_bounds__(1024) em_sort_kernel(const float* __restrict__ Y, int M, unsigned* keys, int* perm,
+                                                       int* tmp) {
+  constexpr int kW = 32, kDig = 256;
+  __shared__ float s_lo[3][kW], s_hi[3][kW];
+  __shared__ int s_cnt[kDig * kW];  // [digit][warp]
+  __shared__ int s_sum[kW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float lo[3], hi[3];
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = 3.0e38f;
+    hi[k] = -3.0e38f;
+  }
+  for (int i = tid; i < M; i += 1024)
+    for (int k = 0; k < 3; ++k) {
+      const float y = Y[(size_t)k * M + i];
+      lo[k] = fminf(lo[k], y);
+      hi[k] = fmaxf(hi[k], y);
+    }
+  for (int k = 0; k < 3; ++k) {
+    for (int off = 16; off > 0; off >>= 1) {
+      lo[k] = fminf(lo[k], __shfl_down_sync(0xffffffffu, lo[k], off));
+      hi[k] = fmaxf(hi[k], __shfl_down_sync(0xffffffffu, hi[k], off));
+    }
+    if (lane == 0) {
+      s_lo[k][warp] = lo[k];
+      s_hi[k][warp] = hi[k];
+    }
+  }
+  __syncthreads();
+  float ext = 0.f;
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = s_lo[k][0];
+    hi[k] = s_hi[k][0];
+    for (int w = 1; w < kW; ++w) {
+      lo[k] = fminf(lo[k], s_lo[k][w]);
+      hi[k] = fmaxf(hi[k], s_hi[k][w]);
+    }
+    ext = fmaxf(ext, hi[k] - lo[k]);
+  }
+  const float inv = ext > 0.f ? 32.f / ext : 0.f;
+  for (int i = tid; i < M; i += 1024) {
+    unsigned c[3];
+    for (int k = 0; k < 3; ++k)  // (a coordinate that is not finite lands in some cell: only locality is at stake)
+      c[k] = (unsigned)min(31, max(0, (int)((Y[(size_t)k * M + i] - lo[k]) * inv)));
+    keys[i] = hilbert_index(c);
+  }
+  const int seg = ((M + kW - 1) / kW + 31) & ~31;
+  const int sb = min(warp * seg, M), se = min(sb + seg, M);
+  for (int pass = 0; pass < 2; ++pass) {
+    const int shift = 8 * pass;
+    const int* from = pass ? tmp : nullptr;  // pass 0 reads in index order
+    int* to = pass ? perm : tmp;
+    for (int i = tid; i < kDig * kW; i += 1024) s_cnt[i] = 0;
+    __syncthreads();
+    for (int i0 = sb; i0 < se; i0 += 32) {
+      const bool in = i0 + lane < se;
+      const unsigned act = __ballot_sync(0xffffffffu, in);
+      if (in) {
+        const int id = from ? from[i0 + lane] : i0 + lane;
+        const int d = (int)(keys[id] >> shift) & 255;
+        const unsigned same = __match_any_sync(act, d);
+        if (lane == __ffs((int)same) - 1) s_cnt[d * kW + warp] += __popc(same);
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    // exclusive scan over (digit, warp): 8 entries a thread
+    int v[8], sum = 0;
+    for (int k = 0; k < 8; ++k) {
+      v[k] = s_cnt[tid * 8 + k];
+      sum += v[k];
+    }
+    int inc = sum;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += n;
+    }
+    if (lane == 31) s_sum[warp] = inc;
+    __syncthreads();
+    int base = inc - sum;
+    for (int w = 0; w < warp; ++w) base += s_sum[w];
+    for (int k = 0; k < 8; ++k) {
+      s_cnt[tid * 8 + k] = base;
+      base += v[k];
+    }
+    __syncthreads();
+    for (int i0 = sb; i0 < se; i0 += 32) {
+      const bool in = i0 + lane < se;
+      const unsigned act = __ballot_sync(0xffffffffu, in);
+      if (in) {
+        const int id = from ? from[i0 + lane] : i0 + lane;
+        const int d = (int)(keys[id] >> shift) & 255;
+        const unsigned same = __match_any_sync(act, d);
+        const int at = s_cnt[d * kW + warp] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp(act);
+        if (lane == __ffs((int)same) - 1) s_cnt[d * kW + warp] += __popc(same);
+        to[at] = id;
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+  }
+}
+
+// Y' in the order perm (null: as given): (y - o, index in the caller's order).
+__global__ void em_pack_rows_kernel(const float* __restrict__ Y, int M, const CenterHdr* hdr,
+                                    const int* __restrict__ perm, float4* __restrict__ out) {
+  const float* o = hdr->oY;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
+    const int i = perm ? perm[r] : r;
+    out[r] = make_float4(__fsub_rn(Y[i], o[0]), __fsub_rn(Y[M + i], o[1]), __fsub_rn(Y[2 * M + i], o[2]),
+                         __int_as_float(i));
+  }
+}
+
+// Centre of every owned block's bounding box and its points' largest distance
+// from it (NaN where a coordinate is not finite).
+__global__ void __launch_bounds__(kBlockPts) em_block_kernel(const float4* __restrict__ rows, int M,
+                                                            float4* __restrict__ out) {
+  constexpr int kW = kBlockPts / 32;
+  __shared__ float s_lo[3][kW], s_hi[3][kW], s_r[kW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x * kBlockPts + threadIdx.x;
+  const float4 y = rows[min(r, M - 1)];  // the last block's padding repeats its last point
+  float lo[3] = {y.x, y.y, y.z}, hi[3] = {y.x, y.y, y.z};
+  for (int k = 0; k < 3; ++k) {
+    for (int off = 16; off > 0; off >>= 1) {
+      lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], off));
+      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
+    }
+    if (lane == 0) {
+      s_lo[k][warp] = lo[k];
+      s_hi[k][warp] = hi[k];
+    }
+  }
+  __syncthreads();
+  float c[3];
+  for (int k = 0; k < 3; ++k) {
+    float l = s_lo[k][0], h = s_hi[k][0];
+    for (int w = 1; w < kW; ++w) {
+      l = fminf(l, s_lo[k][w]);
+      h = fmaxf(h, s_hi[k][w]);
+    }
+    c[k] = 0.5f * (l + h);
+  }
+  const float dx = y.x - c[0], dy = y.y - c[1], dz = y.z - c[2];
+  float d = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+  for (int off = 16; off > 0; off >>= 1) {
+    const float o = __shfl_xor_sync(0xffffffffu, d, off);
+    d = (o > d || o != o) ? o : d;
+  }
+  if (lane == 0) s_r[warp] = d;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kW; ++w) d = (s_r[w] > d || s_r[w] != s_r[w]) ? s_r[w] : d;
+    out[blockIdx.x] = make_float4(c[0], c[1], c[2], d);
+  }
+}
+
 // ------------------------------------------------------------------ host side
 
 namespace {
@@ -355,14 +767,23 @@ struct EmicpPlan {
   int grid;
   SweepGeom geo;
   size_t smem;
+  bool local;  // sorted Y, local sweeps
 };
 
 size_t sweep_smem() { return sizeof(SweepSmem); }
+
+// The local sweep (and the sort that it wants) from 2.4e7 affinities a step on:
+// below, a step is mostly latency and the prepare step's barrier per chunk
+// costs as much as the shorter element gives (4001^2: 1.045 -> 1.043 ms, 3000^2
+// 0.878 -> 0.897, 1007^2 0.576 -> 0.624; 6000 x 5000 1.46 -> 1.41, 12,000^2
+// 4.47 -> 4.01, 17,000^2 8.75 -> 7.75).
+bool emicp_local_pays(int N, int M) { return (double)N * (double)M >= 2.4e7; }
 
 EmicpPlan plan_emicp(int N, int M, int device) {
   EmicpPlan P;
   P.smem = sweep_smem();
   const int limit = persistent_grid_limit(device, (const void*)emicp_kernel, P.smem);
+  P.local = emicp_local_pays(N, M);
   const SweepGeomH h = plan_sweep(M, N, limit);
   P.geo = SweepGeom{h.n_own, h.n_stream, h.nblk, h.slices, h.slice_len, h.units, 0, 0, 0, 0};
   P.grid = h.units < limit ? h.units : limit;
@@ -370,7 +791,7 @@ EmicpPlan plan_emicp(int N, int M, int device) {
   // chunk of 512 streamed points, instead of units dealt in waves; with two
   // blocks on every SM, each SM's pair splits its range 13 : 3, the larger
   // part to the block the SM favours.
-  if (ranged_pays(h.nblk, N, limit)) {
+  if (P.local && ranged_pays(h.nblk, N, limit)) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const char* ev = getenv("CESA_SM_PAIRS");  // "0": equal shares (for comparisons)
@@ -386,7 +807,9 @@ struct EmicpCarved {
   CenterHdr* hdr;
   float4* rows;
   float4* cols;
-  float4* xs;
+  float4* blk;
+  unsigned* keys;
+  int* perm;
   float* part;
   df* rbpart;
   unsigned* pair_tab;
@@ -402,7 +825,9 @@ EmicpCarved carve_emicp(void* base, const EmicpPlan& P, int N, int M, size_t* to
   w.hdr = c.take<CenterHdr>(1);
   w.rows = c.take<float4>((size_t)M);
   w.cols = c.take<float4>((size_t)N);
-  w.xs = c.take<float4>(P.geo.ranged ? (size_t)2 * N : 0);
+  w.blk = c.take<float4>(P.local ? (size_t)P.geo.nblk : 0);
+  w.keys = c.take<unsigned>(P.local ? (size_t)M : 0);
+  w.perm = c.take<int>(P.local ? (size_t)2 * M : 0);
   w.part = c.take<float>(P.geo.ranged ? (size_t)5 * P.geo.nblk * P.geo.kmax * kBlockPts
                                       : (size_t)5 * P.geo.slices * w.Mp);
   w.rbpart = c.take<df>((size_t)2 * P.grid * kEmNV);
@@ -448,7 +873,13 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   prep_center_kernel<<<1, 1024, 0, st>>>(L.dX, L.N, L.dY, L.M, w.hdr);
   const int pb = 256, pg_x = (L.N + pb - 1) / pb, pg_y = (L.M + pb - 1) / pb;
   prep_pack_kernel<<<pg_x < 1024 ? pg_x : 1024, pb, 0, st>>>(L.dX, L.N, w.hdr, 0, 0.f, w.cols);
-  prep_pack_kernel<<<pg_y < 1024 ? pg_y : 1024, pb, 0, st>>>(L.dY, L.M, w.hdr, 1, 0.f, w.rows);
+  if (P.local) {
+    em_sort_kernel<<<1, 1024, 0, st>>>(L.dY, L.M, w.keys, w.perm, w.perm + L.M);
+    em_pack_rows_kernel<<<pg_y < 1024 ? pg_y : 1024, pb, 0, st>>>(L.dY, L.M, w.hdr, w.perm, w.rows);
+    em_block_kernel<<<P.geo.nblk, kBlockPts, 0, st>>>(w.rows, L.M, w.blk);
+  } else {
+    em_pack_rows_kernel<<<pg_y < 1024 ? pg_y : 1024, pb, 0, st>>>(L.dY, L.M, w.hdr, nullptr, w.rows);
+  }
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   if (L.nsteps <= 0) return 0;
@@ -466,7 +897,7 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   A.hdr = w.hdr;
   A.dRt = L.dRt;
   A.part = w.part;
-  A.xs = w.xs;
+  A.blk = P.local ? w.blk : nullptr;
   A.Mp = w.Mp;
   A.rbpart = w.rbpart;
   A.ctl = w.ctl;

@@ -635,7 +635,10 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
 }
 
 // float4 accumulators -> caller SoA [x..., y..., z...]
-__global__ void adjoint_unpack_kernel(const float4* gX, int N, float* oX, const float4* gY, int M, float* oY) {
+// Gradients to the caller's SoA layout; the rows carry their index in the
+// caller's order (the forward may have sorted them).
+__global__ void adjoint_unpack_kernel(const float4* gX, int N, float* oX, const float4* gY, const float4* rows, int M,
+                                      float* oY) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < N) {
     const float4 v = gX[i];
@@ -645,9 +648,10 @@ __global__ void adjoint_unpack_kernel(const float4* gX, int N, float* oX, const 
   } else if (i < N + M) {
     const int r = i - N;
     const float4 v = gY[r];
-    oY[r] = v.x;
-    oY[M + r] = v.y;
-    oY[2 * M + r] = v.z;
+    const int i = __float_as_int(rows[r].w);
+    oY[i] = v.x;
+    oY[M + i] = v.y;
+    oY[2 * M + i] = v.z;
   }
 }
 
@@ -813,7 +817,7 @@ int enqueue_emicp_adjoint(const EmicpAdjointLaunch& L, void* ws, size_t ws_bytes
     if (e != cudaSuccess) return (int)e;
   }
   // SoA outputs
-  adjoint_unpack_kernel<<<(L.N + L.M + 255) / 256, 256, 0, st>>>(gX, L.N, L.gX, gY, L.M, L.gY);
+  adjoint_unpack_kernel<<<(L.N + L.M + 255) / 256, 256, 0, st>>>(gX, L.N, L.gX, gY, L.rows, L.M, L.gY);
   if (e == cudaSuccess) e = cudaMemcpyAsync(L.g_in, g_in, sizeof(float) * 12, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaGetLastError();
   return (int)e;

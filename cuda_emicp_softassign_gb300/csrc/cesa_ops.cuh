@@ -63,8 +63,9 @@ struct EmicpElemScaled {
 // One row's finalize: from its sums tot = (sum e^2, sum e, sum e x) to C_r,
 // lambda_r, u_r = lambda_r X'_r (src/emicp.cu:489-549: C_r <= 1e-6 gives
 // A = 1/N, lambda = 1, X' = mean(X)), the optional row records, and the row's
-// contribution to the 16 moments (added to v).
-__device__ __forceinline__ void emicp_row_finish(int r, const float (&tot)[5], float4 y, float outlier,
+// contribution to the 16 moments (added to v). r: the row's place in the tape;
+// r_out: its index in the caller's order.
+__device__ __forceinline__ void emicp_row_finish(int r, int r_out, const float (&tot)[5], float4 y, float outlier,
                                                  const float (&xm)[3], float* row_out, const float (&oX)[3],
                                                  float* row_tape, df (&v)[kEmNV]) {
   const float C = tot[0] + outlier;
@@ -90,7 +91,7 @@ __device__ __forceinline__ void emicp_row_finish(int r, const float (&tot)[5], f
     o[4] = uu[2];
   }
   if (row_out) {
-    float* o = row_out + (size_t)r * 5;
+    float* o = row_out + (size_t)r_out * 5;
     o[0] = C;
     o[1] = lam;
     o[2] = fmaf(lam, oX[0], uu[0]);
@@ -129,7 +130,7 @@ struct EmicpFin {
     for (int k = 0; k < kEmNV; ++k) v[k] = df_make(0.f);
     const int r = blk * kBlockPts + (int)threadIdx.x;
     if (threadIdx.x < kBlockPts && r < M)
-      emicp_row_finish(r, tot, ld_cg(rows + r), outlier, xm, row_out, oX, row_tape, v);
+      emicp_row_finish(r, r, tot, ld_cg(rows + r), outlier, xm, row_out, oX, row_tape, v);
     owned_block_sum<kEmNV>(v, scratch, rbpart + (size_t)blk * kEmNV);
   }
 };
@@ -192,12 +193,12 @@ __device__ __forceinline__ df dsub(df a, const df& b) {
 // centres the first-order rounding terms cancel and L dXc dYc^T remains, so a
 // cloud that sits off the origin (raw moments thousands of times S) keeps S
 // to FP32 precision; S = sum u y^T - L Xc Yc^T with rounded Xc would not.
-__device__ __forceinline__ float em_S_entry(const df* tot, int i, int j, float xi, float yj) {
+__device__ __forceinline__ df em_S_entry(const df* tot, int i, int j, float xi, float yj) {
   df a = tot[7 + i + 3 * j];
   df_add(a, dmul(tot[4 + j], -xi));
   df_add(a, dmul(tot[1 + i], -yj));
   df_add(a, dmul(dmul(tot[0], xi), yj));
-  return df_val(a);
+  return a;
 }
 
 // One thread forms everything (the adjoint's recomputation of a step).
@@ -208,22 +209,31 @@ __device__ __forceinline__ void em_moments_to_S(const df* tot, float Xc[3], floa
     Yc[i] = df_val(tot[4 + i]) / L;
   }
   for (int j = 0; j < 3; ++j)
-    for (int i = 0; i < 3; ++i) S[i + 3 * j] = em_S_entry(tot, i, j, Xc[i], Yc[j]);
+    for (int i = 0; i < 3; ++i) S[i + 3 * j] = df_val(em_S_entry(tot, i, j, Xc[i], Yc[j]));
 }
 
 // Block-wide (every thread calls it), bitwise the same values: thread i + 3 j
 // (< 9) forms S_ij, threads 9..14 the centres, into out[0..8] = S,
-// out[9..11] = Xc, out[12..14] = Yc (shared). The nine df chains then run side
+// out[9..11] = Xc, out[12..14] = Yc (shared); with `pairs` also their parts
+// below FP32 into out[15..29]. The nine df chains then run side
 // by side instead of one after another in one thread. Synchronises the block.
-__device__ __forceinline__ void em_moments_to_S_block(const df* tot, float* out) {
+__device__ __forceinline__ void em_moments_to_S_block(const df* tot, float* out, bool pairs = false) {
   const int t = threadIdx.x;
   if (t < 15) {
     const float L = df_val(tot[0]);
     if (t < 9) {
       const int i = t % 3, j = t / 3;
-      out[t] = em_S_entry(tot, i, j, df_val(tot[1 + i]) / L, df_val(tot[4 + j]) / L);
+      const df s = em_S_entry(tot, i, j, df_val(tot[1 + i]) / L, df_val(tot[4 + j]) / L);
+      out[t] = df_val(s);
+      if (pairs) out[15 + t] = dd_fast(s.hi, s.lo).lo;
     } else {
       out[t] = df_val(tot[t - 8]) / L;  // t = 9..11: tot[1..3] (Xc); 12..14: tot[4..6] (Yc)
+      if (pairs) {  // the quotient's remainder over L
+        df r = tot[t - 8];
+        df_add_prod(r, -out[t], tot[0].hi);
+        r.lo = __fmaf_rn(-out[t], tot[0].lo, r.lo);
+        out[15 + t] = __fdividef(df_val(r), L);
+      }
     }
   }
   __syncthreads();

@@ -4,20 +4,21 @@
 #pragma once
 #include "cesa_ops.cuh"
 #include "cesa_pose.h"
+#include "cesa_pose_dd.cuh"
 #include "cesa_prep.cuh"
 
 namespace cesa {
 
 struct SaPoseScratch {
-  float S[9], Sl[9], xcp[3], yd[3], xc[3], yc[3];  // Sl: S below FP32 (pairs only)
+  float S[9], xcp[3], yd[3], xc[3], yc[3];
+  float Sl[9], xcl[3], ydl[3];  // S, xcp and yd below FP32 (pairs only)
 };
 
 // sa_moments_to_S with the centres, alpha and beta as (hi, lo) pairs too. Two
 // clouds of unequal counts give sum V a part that S must cancel, against which
 // FP32 rounding of a centre shows.
 __device__ __forceinline__ void sa_moments_to_S_dd(int tid, const df* s_tot, const float* oX, const float* oY,
-                                                   const float* yh, float* s_S, float* s_Sl, float* s_xcp,
-                                                   float* s_yd, float* s_xc, float* s_yc) {
+                                                   const float* yh, SaPoseScratch& ps) {
   const df A1 = dd_fast(s_tot[0].hi, s_tot[0].lo);
   const float inv = dd_inv(A1);
   auto over = [&](int k) { return dd_div(dd_fast(s_tot[k].hi, s_tot[k].lo), A1, inv); };
@@ -45,16 +46,18 @@ __device__ __forceinline__ void sa_moments_to_S_dd(int tid, const df* s_tot, con
     df_add(sij, dd_mul(dd_mul(minus(T9, T5), al), o));
     df_add(sij, dd_mul(dd_mul(minus(T7, A1), be), o));
     sij = dd_fast(sij.hi, sij.lo);
-    s_S[i + 3 * j] = sij.hi;
-    s_Sl[i + 3 * j] = sij.lo;
+    ps.S[i + 3 * j] = sij.hi;
+    ps.Sl[i + 3 * j] = sij.lo;
   } else {
-    s_xcp[i] = df_val(xi);
-    s_yd[i] = df_val(yd);
+    ps.xcp[i] = xi.hi;
+    ps.xcl[i] = xi.lo;
+    ps.yd[i] = yd.hi;
+    ps.ydl[i] = yd.lo;
     df xc = xi, yc = yd;
     df_add(xc, oX[i]);
     df_add(yc, oY[i]);
-    s_xc[i] = df_val(xc);
-    s_yc[i] = df_val(yc);
+    ps.xc[i] = df_val(xc);
+    ps.yc[i] = df_val(yc);
   }
 }
 
@@ -64,46 +67,6 @@ __device__ __forceinline__ void sa_moments_to_S_dd(int tid, const df* s_tot, con
 static __device__ __noinline__ void horn_fast_call(const float* S, HornState<float>* st, float* q, float* gap,
                                                    float* lmax) {
   horn_quaternion_fast<float>(S, *st, q, gap, lmax);
-}
-
-// The last pose of a schedule from the paired S: one inverse iteration in FP64
-// from the FP32 solve's quaternion (the shift, 2e-6 max|N| above its Rayleigh
-// quotient, leaves an error of ~1e-11; the FP32 solve's is ~1e-6 where the
-// eigenvalues lie close). Keeps q where the shifted matrix is not positive definite.
-static __device__ __noinline__ void horn_refine_call(const float* S, const float* Sl, const float* q, const float* Xc,
-                                                     const float* Yc, float* R, float* t) {
-  double Sd[9], N[4][4], A[4][4], L[4][4], rd[4], qd[4], x[4], Xd[3], Yd[3], Rd[9], td[3];
-  for (int k = 0; k < 9; ++k) Sd[k] = (double)S[k] + (double)Sl[k];
-  horn_matrix<double>(Sd, N);
-  double lam = 0.0, scale = 0.0, n2 = 0.0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) qd[i] = q[i];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    n2 += qd[i] * qd[i];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      lam += qd[i] * N[i][j] * qd[j];
-      scale = t_abs(N[i][j]) > scale ? t_abs(N[i][j]) : scale;
-    }
-  }
-  const double sigma = lam / n2 + 2e-6 * scale;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) A[i][j] = (i == j ? sigma : 0.0) - N[i][j];
-  if (!chol4<double>(A, L, rd)) return;
-  chol4_solve_unit<double>(L, rd, qd, x);
-  bool ok = true;
-  for (int i = 0; i < 4; ++i) ok = ok && t_finite(x[i]);
-  if (!ok) return;
-  for (int k = 0; k < 3; ++k) {
-    Xd[k] = Xc[k];
-    Yd[k] = Yc[k];
-  }
-  quat_to_pose<double>(x, Xd, Yd, Rd, td);
-  for (int k = 0; k < 9; ++k) R[k] = (float)Rd[k];
-  for (int k = 0; k < 3; ++k) t[k] = (float)td[k];
 }
 
 // Block-wide (every thread calls it). s_tot: the 32 moments; s_hdr: oX, oY,
@@ -125,7 +88,7 @@ __device__ __forceinline__ void sa_pose_update(const df* s_tot, const float* s_h
   const int tid = threadIdx.x;
   if (kPairs) {
     if (tid < 12)
-      sa_moments_to_S_dd(tid, s_tot, &s_hdr[0], &s_hdr[3], &s_hdr[6], ps.S, ps.Sl, ps.xcp, ps.yd, ps.xc, ps.yc);
+      sa_moments_to_S_dd(tid, s_tot, &s_hdr[0], &s_hdr[3], &s_hdr[6], ps);
   } else if (tid < 12) sa_moments_to_S(tid, s_tot, &s_hdr[0], &s_hdr[3], &s_hdr[6], ps.S, ps.xcp, ps.yd, ps.xc, ps.yc);
   __syncthreads();
   if (tl) tl->mark(13);
@@ -147,7 +110,7 @@ __device__ __forceinline__ void sa_pose_update(const df* s_tot, const float* s_h
       horn_quaternion<float>(S, horn, q, &gap, &lmax);
     // centred-frame translation t' = Xc' - R (Yc - oY)
     quat_to_pose<float>(q, Xcp, Yd, Rn, tn);
-    if (kPairs && last) horn_refine_call(ps.S, ps.Sl, q, Xcp, Yd, Rn, tn);
+    if (kPairs && last) horn_refine_dd(ps.S, ps.Sl, ps.xcp, ps.xcl, ps.yd, ps.ydl, q, Rn, tn);
     for (int k = 0; k < 9; ++k) s_pose[k] = Rn[k];
     for (int k = 0; k < 3; ++k) s_pose[9 + k] = tn[k];
     if (leads) {
