@@ -21,21 +21,23 @@
 // Coordinates are centred by exact offsets before the loop (S is translation
 // invariant; Xc, Yc and t are shifted back).
 //
-// Grid search (phase A alternative, from 4096 target points on by default):
-// the target cloud is bucketed once per registration into a uniform grid of
-// about n/4 cells (counting sort: bin, exclusive scan, scatter). A query scans
-// the cells in Chebyshev rings around its own cell and stops once the box of
-// rings visited is farther from it, on every side, than its best distance
-// (with a relative margin for rounding). Candidates are compared on
+// Grid search (phase A alternative, for large clouds by default): the target
+// cloud is bucketed once per registration into a uniform grid of two cells per
+// point (counting sort: bin, exclusive scan, scatter). A query starts from a
+// real candidate, the previous iteration's match (in the first iteration the
+// nearest of a sample of the target), and looks only at the cells that meet the
+// ball of the candidate's distance, with margins for rounding: per (x, y) column
+// the run of z cells, whose points are contiguous. Candidates are compared on
 // (distance, index), so the match is the same as the exhaustive search's and
-// the whole registration is bitwise the same. A thread searches its query
-// within a work budget; the queries that run over it (far from the target:
-// outliers, early misaligned iterations) are searched again after a grid
-// barrier by a whole warp each, its lanes splitting every ring's cells. From
-// the second iteration on every search starts from the query's previous match
-// (a real candidate, so the search stays exact): the pose changes little, so
-// the bound starts close to the answer and prunes most cells.
+// the whole registration is bitwise the same. 8 lanes share a query (its
+// columns are dealt over them: the chain of dependent loads, not the points, is
+// what a query takes), and the few queries with wide balls are searched after a
+// grid barrier by a warp each. N = M = 40,097, 30 iterations: 4.6 ms with one
+// thread per query going through rings of coarser cells (its slowest threads
+// took 150-240 us of each iteration), 2.7 ms with one thread per ball, 1.7 ms.
+// The queries run in the spatial order of their starting positions.
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/cesa.h"
 #include "cesa_kernels.h"
@@ -49,7 +51,8 @@ namespace {
 constexpr int kIcpRows = kThreads * 4;  // source points per unit (4 per thread)
 constexpr int kIcpTile = 1024;          // target points per shared-memory tile (16 KB)
 constexpr int kIcpNV = 16;              // moments: sum x (3), sum x yd^T (9), sum yd (3), sum d2
-constexpr int kIcpBudget = 1536;        // per-thread search work (points + 4 x cells) before a warp takes over
+constexpr int kIcpBudget = 1536;        // ring search: per-thread work (points + 4 x cells) before a warp takes over
+constexpr int kIcpColumns = 256;        // ball search: columns of cells searched by 8 lanes, more by a warp
 
 // Uniform grid over the (centred) target cloud.
 struct IcpGrid {
@@ -242,6 +245,100 @@ __device__ void grid_nearest_warp(const IcpGrid& g, const int* start, const floa
   bi_out = bi;
 }
 
+// ---- Searches from a candidate. With a real candidate at squared distance
+// `best`, only the cells that meet the ball of that radius can hold a nearer
+// point (or an equal one of lower index): the (x, y) columns of cells within it,
+// and in each the run of z cells, whose points lie next to one another in the
+// sorted array. Margins as in cell_may_hold.
+
+// A column's run of points [p, e) within the ball of radius B (cell units)
+// around f; false when it misses the ball or the grid.
+__device__ __forceinline__ bool column_run(const IcpGrid& g, const int* start, const float (&f)[3], float B, int ix,
+                                           int iy, int& p, int& e) {
+  const float gx = fmaxf(fmaxf((float)ix - f[0], f[0] - (float)(ix + 1)), 0.f);
+  const float gy = fmaxf(fmaxf((float)iy - f[1], f[1] - (float)(iy + 1)), 0.f);
+  const float rest = fmaf(-gy, gy, fmaf(-gx, gx, B * B));
+  if (!(rest >= 0.f)) return false;
+  const float dz = sqrtf(rest) + 1e-5f;
+  const float z0 = fmaxf(floorf(f[2] - dz), 0.f), z1 = fminf(floorf(f[2] + dz), (float)(g.dim[2] - 1));
+  if (!(z0 <= z1)) return false;
+  const int row = (ix * g.dim[1] + iy) * g.dim[2];
+  p = __ldg(start + row + (int)z0);
+  e = __ldg(start + row + (int)z1 + 1);
+  return true;
+}
+
+__device__ __forceinline__ void scan_run(const float4* sorted, int p, int e, float zx, float zy, float zz, float& best,
+                                         int& bi) {
+  for (; p + 4 <= e; p += 4) {
+    const float4 q0 = __ldg(sorted + p), q1 = __ldg(sorted + p + 1), q2 = __ldg(sorted + p + 2),
+                 q3 = __ldg(sorted + p + 3);
+    consider(q0, zx, zy, zz, best, bi);
+    consider(q1, zx, zy, zz, best, bi);
+    consider(q2, zx, zy, zz, best, bi);
+    consider(q3, zx, zy, zz, best, bi);
+  }
+  for (; p < e; ++p) consider(__ldg(sorted + p), zx, zy, zz, best, bi);
+}
+
+// The lexicographic minimum of (distance, index) over groups of W lanes.
+template <int W>
+__device__ __forceinline__ void group_min(float& best, int& bi) {
+#pragma unroll
+  for (int off = W / 2; off > 0; off >>= 1) {
+    const float ob = __shfl_xor_sync(0xffffffffu, best, off);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+    if (ob < best || (ob == best && oi < bi)) {
+      best = ob;
+      bi = oi;
+    }
+  }
+}
+
+struct BallBox {
+  float f[3], B;
+  int x0, x1, y0, y1;
+};
+
+__device__ __forceinline__ float ball_radius(const IcpGrid& g, float best) {
+  return fmaf(sqrtf(best * (1.f + 1e-5f)), g.inv_h, 1e-4f);
+}
+
+__device__ __forceinline__ BallBox ball_box(const IcpGrid& g, float zx, float zy, float zz, float best) {
+  BallBox q;
+  q.f[0] = (zx - g.lo[0]) * g.inv_h;
+  q.f[1] = (zy - g.lo[1]) * g.inv_h;
+  q.f[2] = (zz - g.lo[2]) * g.inv_h;
+  q.B = ball_radius(g, best);
+  q.x0 = (int)fminf(fmaxf(floorf(q.f[0] - q.B), 0.f), (float)g.dim[0]);
+  q.x1 = (int)fmaxf(fminf(floorf(q.f[0] + q.B), (float)(g.dim[0] - 1)), -1.f);
+  q.y0 = (int)fminf(fmaxf(floorf(q.f[1] - q.B), 0.f), (float)g.dim[1]);
+  q.y1 = (int)fmaxf(fminf(floorf(q.f[1] + q.B), (float)(g.dim[1] - 1)), -1.f);
+  return q;
+}
+
+// W consecutive lanes (8, or a whole warp) search one query, its columns dealt
+// over them; every lane of the warp calls it (`live`: this group has a query
+// whose box is small enough). All of the group's lanes return the match.
+template <int W>
+__device__ __forceinline__ void ball_nearest(const IcpGrid& g, const int* start, const float4* sorted,
+                                             const BallBox& q, bool live, float zx, float zy, float zz, float& best,
+                                             int& bi) {
+  if (live) {
+    const int ny = q.y1 - q.y0 + 1, n = (q.x1 - q.x0 + 1) * ny;
+    float B = q.B;
+    for (int k = (int)(threadIdx.x & (W - 1)); k < n; k += W) {
+      int p, e;
+      if (column_run(g, start, q.f, B, q.x0 + k / ny, q.y0 + k % ny, p, e)) {
+        const float was = best;
+        scan_run(sorted, p, e, zx, zy, zz, best, bi);
+        if (best < was) B = ball_radius(g, best);
+      }
+    }
+  }
+  group_min<W>(best, bi);
+}
+
 // One block: the bounding box of the target and the grid (about one cell per
 // four target points over the bounding box, at most cap cells).
 __global__ void __launch_bounds__(1024) k_icp_grid_setup(const float4* X, int N, int cap, IcpGrid* g) {
@@ -282,7 +379,7 @@ __global__ void __launch_bounds__(1024) k_icp_grid_setup(const float4* X, int N,
   }
   if (!(emax > 0.0)) emax = 1.0;
   for (int a = 0; a < 3; ++a) E[a] = fmax(E[a], 1e-3 * emax);
-  const double target = fmax(1.0, fmin((double)cap, N / 4.0));
+  const double target = fmax(1.0, (double)cap);
   double h = cbrt(E[0] * E[1] * E[2] / target);
   int d[3];
   for (int it = 0; it < 64; ++it) {
@@ -328,32 +425,63 @@ __global__ void k_icp_bin(const float4* X, int N, const IcpGrid* gp, int* cell, 
   }
 }
 
-// One block: exclusive scan of the cell counts into start[0..ncells], and a
-// copy into the scatter cursors.
-__global__ void __launch_bounds__(1024) k_icp_scan(const IcpGrid* gp, const int* count, int* start, int* cursor) {
-  __shared__ int s_part[1024];
-  const int n = gp->ncells;
-  const int per = (n + blockDim.x - 1) / blockDim.x;
-  const int b = threadIdx.x * per, e = min(b + per, n);
-  int sum = 0;
-  for (int i = b; i < e; ++i) sum += count[i];
-  s_part[threadIdx.x] = sum;
+// Exclusive scan of the cell counts into start[0..ncells] and the scatter
+// cursors: per-block sums of kScanPer cells, then every block adds the sums
+// before it and scans its own cells.
+constexpr int kScanPer = 4096;
+__global__ void __launch_bounds__(1024) k_icp_scan_sums(const IcpGrid* gp, const int* count, int* sums) {
+  __shared__ int s_w[32];
+  const int n = gp->ncells, b = blockIdx.x * kScanPer;
+  int v = 0;
+  for (int k = 0; k < kScanPer / 1024; ++k) {
+    const int i = b + k * 1024 + (int)threadIdx.x;
+    v += i < n ? count[i] : 0;
+  }
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int k = 0; k < (int)blockDim.x; ++k) {
-      const int v = s_part[k];
-      s_part[k] = run;
-      run += v;
-    }
-    start[n] = run;
+  if (threadIdx.x < 32) {
+    v = __reduce_add_sync(0xffffffffu, s_w[threadIdx.x]);
+    if (threadIdx.x == 0) sums[blockIdx.x] = v;
+  }
+}
+
+__global__ void __launch_bounds__(1024) k_icp_scan(const IcpGrid* gp, const int* count, const int* sums, int* start,
+                                                   int* cursor) {
+  __shared__ int s_w[32], s_base;
+  const int n = gp->ncells, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int v = 0;  // the blocks before this one
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += 1024) v += sums[k];
+  v = __reduce_add_sync(0xffffffffu, v);
+  if (lane == 0) s_w[warp] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = __reduce_add_sync(0xffffffffu, s_w[lane]);
+    if (lane == 0) s_base = v;
   }
   __syncthreads();
-  int run = s_part[threadIdx.x];
-  for (int i = b; i < e; ++i) {
-    start[i] = run;
-    cursor[i] = run;
-    run += count[i];
+  constexpr int kPer = kScanPer / 1024;
+  const int i0 = blockIdx.x * kScanPer + (int)threadIdx.x * kPer;
+  int c[kPer], sum = 0;
+  for (int k = 0; k < kPer; ++k) {
+    c[k] = i0 + k < n ? count[i0 + k] : 0;
+    sum += c[k];
+  }
+  int inc = sum;
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += o;
+  }
+  if (lane == 31) s_w[warp] = inc;
+  __syncthreads();
+  int run = s_base + inc - sum;
+  for (int w = 0; w < warp; ++w) run += s_w[w];
+  for (int k = 0; k < kPer; ++k) {
+    if (i0 + k <= n) {  // entry n: the total
+      start[i0 + k] = run;
+      if (i0 + k < n) cursor[i0 + k] = run;
+    }
+    run += c[k];
   }
 }
 
@@ -398,7 +526,11 @@ struct IcpArgs {
 };
 
 __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
-  __shared__ float4 s_x[kIcpTile];
+  // target points staged in phase A, the rows' moments in phase B
+  __shared__ __align__(16) unsigned char s_buf[sizeof(df) * kIcpNV * (kThreads + kThreads / kIcpNV)];
+  static_assert(sizeof(s_buf) >= sizeof(float4) * kIcpTile && kIcpNV == kEmNV, "shared buffer");
+  float4* s_x = reinterpret_cast<float4*>(s_buf);
+  __shared__ float s_S[12];
   __shared__ float s_pose[12];
   __shared__ float s_hdr[9];  // oX, oY, mean of Y'
   __shared__ df s_red[kThreads];
@@ -436,20 +568,68 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
       const IcpGrid g = *A.grid;
       const int warp = tid >> 5, lane = tid & 31;
       const int nchunks = (A.M + 31) >> 5;
-      // warp-sized chunks of spatially ordered rows, dealt round-robin over the blocks
-      for (int ch = blockIdx.x + (int)G * warp; ch < nchunks; ch += (int)G * kWarps) {
-        const int j = (ch << 5) + lane;
-        if (j >= A.M) continue;
-        const int r = __ldg(A.qorder + j);
-        float z[3];
-        move_point(R, tc, ld_cg(A.rows + r), z);
-        float best, sd;
-        int bi, si;
-        seed_of(A.cols, iter > 0 ? A.prev_nn : nullptr, r, A.N, z[0], z[1], z[2], sd, si);
-        if (grid_nearest(g, A.cell_start, A.sorted, z[0], z[1], z[2], kIcpBudget, sd, si, best, bi))
-          __stcg(A.part + r, make_float2(best, __int_as_float(bi)));
-        else
-          A.heavy[atomicAdd(A.heavy_n, 1)] = r;
+      // A grid over a bounding box that is not finite keeps the ring searches.
+      const bool ball = g.inv_h > 0.f && g.inv_h < 1e30f && fabsf(g.lo[0]) < 1e30f && fabsf(g.lo[1]) < 1e30f &&
+                        fabsf(g.lo[2]) < 1e30f;
+      const int* prev = iter > 0 ? A.prev_nn : nullptr;
+      // The first iteration's candidates: the nearest of a sample of the target
+      // (every N / kIcpTile-th point of the sorted array, which runs through the
+      // occupied cells); later ones start from the previous match.
+      const int nsamp = min(A.N, kIcpTile);
+      if (ball && !prev) {
+        for (int k = tid; k < nsamp; k += kThreads)
+          s_x[k] = __ldg(A.sorted + (int)((long)k * A.N / nsamp));
+        __syncthreads();
+      }
+      // candidate of row r at z (a real point, or +inf and no index), by a group of W lanes
+      auto candidate = [&](auto W, int r, const float (&z)[3], float& best, int& bi) {
+        seed_of(A.cols, prev, r, A.N, z[0], z[1], z[2], best, bi);
+        if (ball && !prev) {
+          for (int k = (int)(threadIdx.x & (W.value - 1)); k < nsamp; k += W.value)
+            consider(s_x[k], z[0], z[1], z[2], best, bi);
+          group_min<W.value>(best, bi);
+        }
+      };
+      if (ball) {
+        // Four spatially neighbouring queries a warp, 8 lanes each; one whose
+        // box holds over kIcpColumns columns is left to a whole warp.
+        using W8 = std::integral_constant<int, 8>;
+        const int nquads = (A.M + 3) >> 2;
+        for (int ch = blockIdx.x + (int)G * warp; ch < nquads; ch += (int)G * kWarps) {
+          const int j = (ch << 2) + (lane >> 3);
+          const int r = __ldg(A.qorder + min(j, A.M - 1));
+          float z[3];
+          move_point(R, tc, ld_cg(A.rows + r), z);
+          float best;
+          int bi;
+          candidate(W8{}, r, z, best, bi);
+          const bool found = best < 1e30f;  // else a coordinate is not finite: no match (phase B takes the first point)
+          const BallBox q = ball_box(g, z[0], z[1], z[2], found ? best : 0.f);
+          const bool small = (q.x1 - q.x0 + 1) * (q.y1 - q.y0 + 1) <= kIcpColumns;
+          ball_nearest<8>(g, A.cell_start, A.sorted, q, found && small && j < A.M, z[0], z[1], z[2], best, bi);
+          if ((lane & 7) == 0 && j < A.M) {
+            if (small || !found)
+              __stcg(A.part + r, make_float2(best, __int_as_float(bi)));
+            else
+              A.heavy[atomicAdd(A.heavy_n, 1)] = r;
+          }
+        }
+      } else {
+        // warp-sized chunks of spatially ordered rows, dealt round-robin over the blocks
+        for (int ch = blockIdx.x + (int)G * warp; ch < nchunks; ch += (int)G * kWarps) {
+          const int j = (ch << 5) + lane;
+          if (j >= A.M) continue;
+          const int r = __ldg(A.qorder + j);
+          float z[3];
+          move_point(R, tc, ld_cg(A.rows + r), z);
+          float best, sd;
+          int bi, si;
+          seed_of(A.cols, prev, r, A.N, z[0], z[1], z[2], sd, si);
+          if (grid_nearest(g, A.cell_start, A.sorted, z[0], z[1], z[2], kIcpBudget, sd, si, best, bi))
+            __stcg(A.part + r, make_float2(best, __int_as_float(bi)));
+          else
+            A.heavy[atomicAdd(A.heavy_n, 1)] = r;
+        }
       }
       if (!grid_sync(A.ctl, epoch, G, A.timeout_ns, 69)) {
         ok = false;
@@ -460,10 +640,18 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
         const int r = __ldcg(A.heavy + h);
         float z[3];
         move_point(R, tc, ld_cg(A.rows + r), z);
-        float best, sd;
-        int bi, si;
-        seed_of(A.cols, iter > 0 ? A.prev_nn : nullptr, r, A.N, z[0], z[1], z[2], sd, si);
-        grid_nearest_warp(g, A.cell_start, A.sorted, z[0], z[1], z[2], sd, si, best, bi);
+        float best;
+        int bi;
+        if (ball) {
+          candidate(std::integral_constant<int, 32>{}, r, z, best, bi);
+          ball_nearest<32>(g, A.cell_start, A.sorted, ball_box(g, z[0], z[1], z[2], best), true, z[0], z[1], z[2], best,
+                           bi);
+        } else {
+          float sd;
+          int si;
+          seed_of(A.cols, prev, r, A.N, z[0], z[1], z[2], sd, si);
+          grid_nearest_warp(g, A.cell_start, A.sorted, z[0], z[1], z[2], sd, si, best, bi);
+        }
         if (lane == 0) __stcg(A.part + r, make_float2(best, __int_as_float(bi)));
       }
     }
@@ -538,7 +726,9 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
       df v[kIcpNV];
 #pragma unroll
       for (int k = 0; k < kIcpNV; ++k) v[k] = df_make(0.f);
-      for (int r = blockIdx.x * kThreads + tid; r < A.M; r += G * kThreads) {
+      const int rpb = (A.M + (int)G - 1) / (int)G;  // an even share of the rows
+      const int rb0 = min((int)blockIdx.x * rpb, A.M), rb1 = min(rb0 + rpb, A.M);
+      for (int r = rb0 + tid; r < rb1; r += kThreads) {
         float best = __int_as_float(0x7f800000);
         int bi = 0;
         for (int s = 0; s < A.S; ++s) {
@@ -566,11 +756,7 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
         }
         df_add(v[15], best);
       }
-      block_reduce_df<kIcpNV>(v, s_red);
-      if (tid == 0)
-#pragma unroll
-        for (int k = 0; k < kIcpNV; ++k)
-          __stcg(reinterpret_cast<float2*>(mom + (size_t)blockIdx.x * kIcpNV + k), make_float2(v[k].hi, v[k].lo));
+      em_block_moments(v, min(rb1 - rb0, kThreads), reinterpret_cast<df*>(s_buf), mom + (size_t)blockIdx.x * kIcpNV);
     }
     if (!grid_sync(A.ctl, epoch, G, A.timeout_ns, 72)) {
       ok = false;
@@ -578,19 +764,29 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
     }
     // ---- the pose (every block computes the same one)
     reduce_block_partials<kIcpNV>(mom, (int)G, s_red, s_tot);
+    // S = sum (x - Xc)(y - Yc)^T = sum x yd^T - Xc (sum yd)^T: thread i + 3 j its
+    // entry, threads 9-11 the centre
+    if (tid < 12) {
+      const int i = tid < 9 ? tid % 3 : tid - 9, j = tid / 3;
+      const float mh = (float)A.M;
+      const df m{mh, (float)(A.M - (int)mh)};
+      const float xc = df_val(dd_div(dd_fast(s_tot[i].hi, s_tot[i].lo), m, dd_inv(m)));
+      if (tid < 9) {
+        df a = s_tot[3 + i + 3 * j];
+        df_add_prod(a, -xc, df_val(s_tot[12 + j]));
+        s_S[tid] = df_val(a);
+      } else {
+        s_S[tid] = xc;
+      }
+    }
+    __syncthreads();
     if (tid == 0) {
       float Xc[3], Ym[3], S[9];
+      for (int i = 0; i < 9; ++i) S[i] = s_S[i];
       for (int i = 0; i < 3; ++i) {
-        Xc[i] = (float)(df_dbl(s_tot[i]) / (double)A.M);
+        Xc[i] = s_S[9 + i];
         Ym[i] = s_hdr[6 + i];
       }
-      // S = sum (x - Xc)(y - Yc)^T = sum x yd^T - Xc (sum yd)^T
-      for (int j = 0; j < 3; ++j)
-        for (int i = 0; i < 3; ++i) {
-          df a = s_tot[3 + i + 3 * j];
-          df_add_prod(a, -Xc[i], df_val(s_tot[12 + j]));
-          S[i + 3 * j] = df_val(a);
-        }
       float q[4], gap = 0.f, lmax = 0.f, Rn[9], tn[3];
       horn_quaternion_fast<float>(S, horn, q, &gap, &lmax);
       quat_to_pose<float>(q, Xc, Ym, Rn, tn);  // centred frame: t' = Xc' - R Ym
@@ -659,8 +855,14 @@ struct IcpPlan {
 IcpPlan plan_icp(int N, int M, int device, int search) {
   IcpPlan P;
   const int limit = persistent_grid_limit(device, (const void*)icp_kernel, 0);
-  P.use_grid = search == CESA_ICP_SEARCH_GRID || (search == CESA_ICP_SEARCH_AUTO && N >= 4096);
-  P.cap = std::max(64, N / 4);
+  P.use_grid = search == CESA_ICP_SEARCH_GRID || 
+               // below ~6500^2 pairs every point is scanned sooner (5000^2: 0.71 ms against 0.82;
+               // 8000^2: 1.00 against 0.90)
+               (search == CESA_ICP_SEARCH_AUTO && N >= 4096 && (double)N * (double)M >= 4e7);
+  // Two cells per target point (scans are points of a surface: ~20 to an
+  // occupied cell): N = M = 40,097 1.70 ms, with 1/2, 1, 4 and 8 cells 2.02,
+  // 1.76, 2.03, 2.25; 10,007 x 9001 0.88, with 1 and 4 0.94 and 0.92.
+  P.cap = std::max(64, (int)std::min(2.0 * N, std::max(4.2e6, N / 4.0)));
   if (P.use_grid) {  // one slice: every row is searched whole by one thread
     P.nrb = (M + kIcpRows - 1) / kIcpRows;
     P.S = 1;
@@ -700,7 +902,7 @@ struct IcpCarved {
   float2* part;
   df* rbpart;
   IcpGrid* grid;  // grid search only
-  int *count, *start, *cursor, *cell;
+  int *count, *start, *cursor, *cell, *sums;
   float4* sorted;
   int* qorder;
   int* heavy;
@@ -723,6 +925,7 @@ IcpCarved carve_icp(void* base, const IcpPlan& P, int N, int M, size_t* total) {
     w.start = c.take<int>((size_t)P.cap + 1);
     w.cursor = c.take<int>((size_t)P.cap + 1);
     w.cell = c.take<int>((size_t)std::max(N, M));
+    w.sums = c.take<int>((size_t)P.cap / kScanPer + 1);
     w.sorted = c.take<float4>((size_t)N);
     w.qorder = c.take<int>((size_t)M);
     w.heavy = c.take<int>((size_t)M);
@@ -764,7 +967,9 @@ int enqueue_icp(const IcpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, 
     k_icp_grid_setup<<<1, 1024, 0, st>>>(w.cols, L.N, P.cap, w.grid);
     const int gb = std::min((L.N + pb - 1) / pb, 1024);
     k_icp_bin<<<gb, pb, 0, st>>>(w.cols, L.N, w.grid, w.cell, w.count);
-    k_icp_scan<<<1, 1024, 0, st>>>(w.grid, w.count, w.start, w.cursor);
+    const int sb = P.cap / kScanPer + 1;  // covers entry ncells <= cap
+    k_icp_scan_sums<<<sb, 1024, 0, st>>>(w.grid, w.count, w.sums);
+    k_icp_scan<<<sb, 1024, 0, st>>>(w.grid, w.count, w.sums, w.start, w.cursor);
     k_icp_scatter<<<gb, pb, 0, st>>>(w.cols, L.N, w.cell, w.cursor, w.sorted);
     // the source rows in the spatial order of their starting positions (a rigid
     // motion keeps neighbours together, so a warp's queries stay coherent)
@@ -772,7 +977,8 @@ int enqueue_icp(const IcpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, 
     if (e != cudaSuccess) return (int)e;
     const int gy = std::min((L.M + pb - 1) / pb, 1024);
     k_icp_bin<<<gy, pb, 0, st>>>(w.rows, L.M, w.grid, w.cell, w.count);
-    k_icp_scan<<<1, 1024, 0, st>>>(w.grid, w.count, w.cursor, w.cursor);
+    k_icp_scan_sums<<<sb, 1024, 0, st>>>(w.grid, w.count, w.sums);
+    k_icp_scan<<<sb, 1024, 0, st>>>(w.grid, w.count, w.sums, w.cursor, w.cursor);
     k_icp_scatter_order<<<gy, pb, 0, st>>>(L.M, w.cell, w.cursor, w.qorder);
   }
   e = cudaGetLastError();

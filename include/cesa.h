@@ -92,9 +92,9 @@ typedef struct cesa_params {
 
 /* ICP nearest-neighbour search (cesa_params.icp_search). Both are exact and
  * give the same matches (the first of equal distances in X order). */
-#define CESA_ICP_SEARCH_AUTO 0       /* uniform grid from 4096 target points on, else exhaustive */
+#define CESA_ICP_SEARCH_AUTO 0       /* uniform grid from 4096 target points and N x M = 4e7 on, else exhaustive */
 #define CESA_ICP_SEARCH_EXHAUSTIVE 1 /* every target point, tiled through shared memory */
-#define CESA_ICP_SEARCH_GRID 2       /* uniform grid over the target, rings of cells around each query */
+#define CESA_ICP_SEARCH_GRID 2       /* uniform grid over the target, the cells within reach of a candidate */
 
 /*
  * Optional per-call report (may be NULL). trace, when non-NULL, receives one
