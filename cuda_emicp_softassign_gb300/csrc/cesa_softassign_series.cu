@@ -906,26 +906,34 @@ __device__ __forceinline__ void series_run(const SeriesArgs& A) {
 
 __global__ void __launch_bounds__(kSerThreads, 1) softassign_series_kernel(const SeriesArgs A) { series_run(A); }
 
+// A batch's launches (one per cluster size) run side by side: each may start
+// once all CTAs of the one before have started, and none completes before it.
 __global__ void __launch_bounds__(kSerThreads, 1) softassign_series_batch_kernel(const SeriesArgs* tab) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   series_run(tab[cluster_id_x()]);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ------------------------------------------------------------------ host side
 namespace {
 constexpr size_t kSerSmemMax = 220 * 1024;  // of 227 KB; the rest is static
+constexpr int kSerBatchPts = 1536;          // most points per CTA in a batch
+static_assert(sizeof(float) * ((size_t)kLState + (size_t)(kRowArr + kColArr) * kSerBatchPts) <= kSerSmemMax, "fits");
 
 struct SeriesPlan {
   int CS = 0, nr = 0, nc = 0;
   size_t smem = 0;
 };
 
-SeriesPlan plan_series(int N, int M) {
+// The least power of two of CTAs that leaves each at most `pts` points of a
+// cloud (0: the choice for one pair alone).
+SeriesPlan plan_series(int N, int M, int pts = 0) {
   SeriesPlan P;
   const int n = N > M ? N : M;
   int CS = 1;
-  // points a CTA: 128 up to 512 points (7.0 against 7.2 ms with 256 at N = M =
+  // one pair: 128 up to 512 points (7.0 against 7.2 ms with 256 at N = M =
   // 413), else 256 (7.7 against 7.7 with 128 and 9.0 with 512 at 2000)
-  const int pts = n <= 512 ? 128 : 256;
+  if (pts == 0) pts = n <= 512 ? 128 : 256;
   while (CS < kSerMaxCS && (n + CS - 1) / CS > pts) CS *= 2;
   const int nr = (N + CS - 1) / CS, nc = (M + CS - 1) / CS;
   const size_t smem =
@@ -944,7 +952,8 @@ bool softassign_series_fits(int N, int M) {
 }
 
 namespace {
-cudaError_t launch_series(const void* k, int clusters, int CS, size_t smem, void** args, cudaStream_t st) {
+cudaError_t launch_series(const void* k, int clusters, int CS, size_t smem, void** args, cudaStream_t st,
+                          bool beside = false) {
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerSmemMax);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
@@ -953,13 +962,15 @@ cudaError_t launch_series(const void* k, int clusters, int CS, size_t smem, void
   cfg.blockDim = dim3(kSerThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = CS;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = beside ? 2 : 1;
   return cudaLaunchKernelExC(&cfg, k, args);
 }
 }  // namespace
@@ -1000,7 +1011,29 @@ int enqueue_softassign_series(const SoftassignLaunch& L, const float4* rows, con
 
 size_t softassign_series_table_bytes(int njobs) { return sizeof(SeriesArgs) * (size_t)njobs; }
 
+// Points per CTA for a batch: the fewest for which all clusters run at once.
+// One pair (60 temperatures) takes little longer on fewer CTAs (its updates
+// are latency: N = M = 1000 on 4 CTAs 4.6 ms, on 1 6.0; 4000 on 16 5.1, on 4
+// 6.6), a second wave of clusters twice as long: 20 pairs of 500-20,000 points
+// take 15.9 / 11.7 / 6.8 / 8.2 ms with 256 / 512 / 1024 / 1536 points (276 / 210
+// / 129 / 105 CTAs) and 25 ms one cluster size after the other. Clusters of 16 leave SMs
+// of their GPCs over, so 7/8 of the SMs count (154 CTAs did not fit 152 SMs:
+// 12.5 ms; 129 did).
+int batch_points(const SeriesJob* jobs, int njobs, int sms) {
+  for (int pts = 256; pts <= 1024; pts *= 2) {
+    long ctas = 0;
+    for (int i = 0; i < njobs; ++i) ctas += plan_series(jobs[i].N, jobs[i].M, pts).CS;
+    if (ctas <= (long)sms * 7 / 8) return pts;
+  }
+  return kSerBatchPts;
+}
+
 int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_table, void* ctl, cudaStream_t st) {
+  int device = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess) return (int)e;
+  const int pts = batch_points(jobs, njobs, sms);
   // one launch per cluster size, its pairs in the order given
   std::vector<SeriesArgs> tab;
   tab.reserve((size_t)njobs);
@@ -1013,7 +1046,7 @@ int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_
     Group g{CS, (int)tab.size(), 0, 0};
     for (int i = 0; i < njobs; ++i) {
       const SeriesJob& J = jobs[i];
-      const SeriesPlan P = plan_series(J.N, J.M);
+      const SeriesPlan P = plan_series(J.N, J.M, pts);
       if (P.CS != CS) continue;
       SeriesArgs A{};
       A.rows = J.rows;
@@ -1045,11 +1078,12 @@ int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_
     if (g.n > 0) groups.push_back(g);
   }
   if (tab.empty()) return 0;
-  cudaError_t e = cudaMemcpyAsync(dev_table, tab.data(), sizeof(SeriesArgs) * tab.size(), cudaMemcpyHostToDevice, st);
+  e = cudaMemcpyAsync(dev_table, tab.data(), sizeof(SeriesArgs) * tab.size(), cudaMemcpyHostToDevice, st);
   for (size_t i = 0; i < groups.size() && e == cudaSuccess; ++i) {
     const SeriesArgs* t = static_cast<const SeriesArgs*>(dev_table) + groups[i].first;
     void* args[] = {(void*)&t};
-    e = launch_series((const void*)softassign_series_batch_kernel, groups[i].n, groups[i].CS, groups[i].smem, args, st);
+    e = launch_series((const void*)softassign_series_batch_kernel, groups[i].n, groups[i].CS, groups[i].smem, args, st,
+                      i > 0);
   }
   return (int)e;
 }

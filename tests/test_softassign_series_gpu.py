@@ -87,3 +87,20 @@ def test_batch_takes_up_where_the_series_stops(cesa):
         Rs, ts = (cesa.softassign if algo == cesa.ALGO_SOFTASSIGN else cesa.emicp)(X, Y, param=p)
         assert rot_err_deg(R, Rs) < 2e-3
         assert np.abs(t - ts).max() < 1e-4 * float(np.ptp(X, 0).max())
+
+
+@pytest.mark.parametrize("sizes", [[33, 257, 1025], [513] * 40 + [1535, 1536, 1537, 3073, 24001],
+                                   [20011, 16385, 16384, 12289] * 3 + [129] * 30])
+def test_batches_of_several_cluster_sizes(cesa, sizes):
+    """All clusters at once with few, more and most points per CTA, and more
+    clusters than fit: the pairs agree with single calls, both in the series
+    (its sums in another order), within the batch's tolerance."""
+    p = cesa.Params.default(JMAX=12)
+    pairs = [(cesa.ALGO_SOFTASSIGN, *_pair(n, n, k % 7), p) for k, n in enumerate(sizes)]
+    single = {}
+    for (_, X, Y, _), (R, t), key in zip(pairs, cesa.register_batch(pairs), [(n, k % 7) for k, n in enumerate(sizes)]):
+        if key not in single:
+            single[key] = cesa.softassign(X, Y, param=p)
+        Rs, ts = single[key]
+        assert rot_err_deg(R, Rs) < 2e-3
+        assert np.abs(t - ts).max() < 1e-4 * float(np.ptp(X, 0).max())
