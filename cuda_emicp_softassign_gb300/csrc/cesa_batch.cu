@@ -1,15 +1,20 @@
 // Batched registration for sm_103a: many (X, Y) pairs of uneven sizes, EM-ICP
-// and Softassign mixed, in one persistent cooperative launch.
+// and Softassign mixed.
 //
-// Every pair follows its own schedule (the sigma loop of src/emicp.cu:443-669
-// or the JMAX x I0 x I1 loops of src/softassign.cu:486-822), and all pairs
-// advance in lock step, one phase per round:
-//   EM-ICP      E (E-step sweep)  Z (moments -> S -> Horn pose)
-//   Softassign  R_0 C_0 ... R_{I1-1} C_{I1-1} F Z
-// with R_k / C_k the Sinkhorn row / column passes and F the final sweep. A
-// sweep phase is split into (pair, tile) units of 128 owned points x one slice
-// of the streamed points; a Z phase is one unit. The units of all pairs in a
-// round form one work list, taken round-robin by the blocks of the grid, and
+// The EM-ICP pairs run in one launch in which every pair has a team of blocks of
+// its own (emicp_teams_kernel). The Softassign pairs run their leading updates
+// in the series form, a cluster per pair (softassign_series_batch_kernel); what
+// is left of their schedules, and the pairs whose form is set, run here in one
+// persistent cooperative launch:
+//
+// Every pair follows its own schedule (the JMAX x I0 x I1 loops of
+// src/softassign.cu:486-822), and all pairs advance in lock step, one phase per
+// round:
+//   R_0 C_0 ... R_{I1-1} C_{I1-1} F Z
+// with R_k / C_k the Sinkhorn row / column passes, F the final sweep and Z the
+// pose. A sweep phase is split into (pair, tile) units of 128 owned points x one
+// slice of the streamed points; a Z phase is one unit. The units of all pairs in
+// a round form one work list, taken round-robin by the blocks of the grid, and
 // the round ends at a grid barrier. With hundreds of pairs a round holds
 // thousands of units, so the barrier is amortised and the small pairs (which
 // alone could not fill 152 SMs) run alongside the large ones.
@@ -35,11 +40,10 @@
 namespace cesa {
 namespace {
 
-constexpr int kPhIdle = 0, kPhEmE = 1, kPhEmZ = 2, kPhSaRow = 3, kPhSaCol = 4, kPhSaFin = 5, kPhSaZ = 6;
+constexpr int kPhIdle = 0, kPhSaRow = 1, kPhSaCol = 2, kPhSaFin = 3, kPhSaZ = 4;
 
 // Per-pair state block (floats): [0..8] R, [9..11] t' (centred frame),
-// [12] sigma_p2 (EM-ICP) or T (Softassign), [16..35] Horn eigenbasis and
-// last quaternion.
+// [12] T, [16..35] Horn eigenbasis and last quaternion.
 constexpr int kStateFloats = 64;
 constexpr int kStateHorn = 16;
 static_assert(sizeof(HornState<float>) == 20 * sizeof(float), "Horn state layout");
@@ -52,19 +56,18 @@ constexpr double kUnitsPerBlock = 8.0;
 struct BPair {
   int algo;  // 0 EM-ICP, 1 Softassign
   int N, M;
-  SweepGeom g0;  // EM-ICP: own Y' stream X'; Softassign row sweeps: own X' stream Y'
-  SweepGeom g1;  // Softassign column sweeps: own Y' stream X'
-  int rounds;
-  int nsteps;  // sigma steps or pose updates (JMAX * I0)
+  SweepGeom g0;  // Softassign row sweeps: own X' stream Y'
+  SweepGeom g1;  // column sweeps: own Y' stream X'
+  int rounds;    // (EM-ICP: as reported, the steps run in teams of their own)
+  int nsteps;    // sigma steps or pose updates (JMAX * I0)
   int I0, I1;
-  float init;  // sigma_p2 or T_0
-  float sigma_factor, d_02;
+  float init;  // T_0
   float alpha, TFACTOR, moutlier;
   const float* X;  // caller SoA (device)
   const float* Y;
   float* dRt;  // caller pose (device), written after the last step
-  float4* own0;  // EM-ICP: Y' (M); Softassign: X' (N)
-  float4* own1;  // EM-ICP: X' (N); Softassign: Y' (M)
+  float4* own0;  // X' (N)
+  float4* own1;  // Softassign: Y' (M)
   CenterHdr* hdr;
   float* part;
   unsigned* cnt0;
@@ -88,7 +91,7 @@ struct BatchArgs {
 };
 
 struct Sched {
-  int algo, rounds, I1, units0, units1;
+  int rounds, I1, units0, units1;
   int done;  // pose updates the series kernel ran
 };
 
@@ -100,12 +103,6 @@ struct Ph {
 __device__ __forceinline__ Ph phase_of(const Sched& s, int r) {
   Ph p{kPhIdle, 0, 0, 0u};
   if (r >= s.rounds) return p;
-  if (s.algo == 0) {
-    p.step = r >> 1;
-    p.phase = (r & 1) ? kPhEmZ : kPhEmE;
-    p.geo_round = (unsigned)p.step;
-    return p;
-  }
   const int per = 2 * s.I1 + 2;
   const int upd = r / per, k = r - upd * per;
   p.step = upd + s.done;
@@ -129,13 +126,11 @@ __device__ __forceinline__ Ph phase_of(const Sched& s, int r) {
 
 __device__ __forceinline__ int phase_units(const Sched& s, int phase) {
   switch (phase) {
-    case kPhEmE:
     case kPhSaRow:
     case kPhSaFin:
       return s.units0;
     case kPhSaCol:
       return s.units1;
-    case kPhEmZ:
     case kPhSaZ:
       return 1;
     default:
@@ -231,10 +226,6 @@ __device__ __forceinline__ UnitRef resolve(const BPair* pairs, const Sched* sche
   U.state = P.state;
   U.hdr = P.hdr;
   switch (U.ph.phase) {
-    case kPhEmE:
-      U.src = P.own1;
-      U.own = P.own0;
-      break;
     case kPhSaRow:
       U.src = P.own1;
       U.own = P.own0;
@@ -402,16 +393,6 @@ __device__ bool run_sweep_unit(SweepSmem& sm, Ring& rg, const UnitRef& U, bool x
 // phases fold 2^c0 (wsc) into the streamed weights, so that the elements are
 // EmicpElemScaled / SinkElemScaled / FinalElemScaled.
 
-// E-step: the streamed X' times sc.
-__device__ __forceinline__ PrepOut prep_scaled(SweepSmem& sm, int stage, int len, float sc) {
-  for (int c = threadIdx.x; c < len; c += kThreads) {
-    const float4 x = sm.raw[stage][c];
-    sm.prep[c] = make_float4(x.x * sc, x.y * sc, x.z * sc, 0.f);
-  }
-  __syncthreads();
-  return PrepOut{sm.prep, sm.prep};
-}
-
 // Streamed Y' posed by (R, t') = meta[0..11]: sc (R y' + t') and w wsc, with w
 // from the stage's weights, or 1.
 __device__ __forceinline__ PrepOut prep_posed(SweepSmem& sm, int stage, int len, const float* m, bool unit_weight,
@@ -517,27 +498,6 @@ struct BColFin {
 
 // Per-phase operations of a sweep unit. meta: state floats [0..15] (R, t',
 // sigma_p2 or T at [12]), centring header [16..31] (oX, oY, xmean, ymean).
-// e = exp(-d^2 / (2 sigma_p2)) = 2^-|sc x - sc z|^2, sc = sqrt(log2(e) / (2 sigma_p2))
-__device__ __forceinline__ float em_scale(float s2) { return sqrtf(kLog2e / (2.f * s2)); }
-
-struct EmOps {  // EM-ICP E-step
-  using Elem = EmicpElemScaled;
-  const BPair* P;
-  df* scratch;
-  __device__ __forceinline__ Elem elem(const float*) const { return Elem{}; }
-  __device__ __forceinline__ float scale(const float* m) const { return em_scale(m[12]); }
-  __device__ __forceinline__ PrepOut prep(SweepSmem& sm, int stage, int len, const float* m) const {
-    return prep_scaled(sm, stage, len, em_scale(m[12]));
-  }
-  __device__ __forceinline__ void fin(int blk, const float (&tot)[5], const float* m) const {
-    const float inv_sc = 1.f / em_scale(m[12]);  // the e x sums came out sc times too large
-    const float t5[5] = {tot[0], tot[1], tot[2] * inv_sc, tot[3] * inv_sc, tot[4] * inv_sc};
-    const EmicpFin f{P->own0, P->M, expf(-P->d_02 / m[12]),  // src/emicp.cu:489
-                     {m[24], m[25], m[26]}, nullptr, {m[16], m[17], m[18]}, scratch, P->rec};
-    f(blk, t5);
-  }
-};
-
 // K = exp((alpha - d^2)/T) / sqrt(T) = 2^c0 2^-|sc x - sc y|^2, sc = sqrt(log2(e) / T)
 __device__ __forceinline__ float sa_scale(float T) { return sqrtf(kLog2e / T); }
 __device__ __forceinline__ float sa_wscale(float alpha, float T) {
@@ -614,23 +574,6 @@ __device__ __noinline__ void horn_update(const BPair& P, const float S[9], const
   (void)step;
 }
 
-__device__ __noinline__ void em_finalize(const BPair& P, const Ph& ph, df* s_red, df* s_tot) {
-  __shared__ float s_emS[15];
-  reduce_block_partials<kEmNV>(P.rec, P.g0.nblk, s_red, s_tot);
-  em_moments_to_S_block(s_tot, s_emS);
-  if (threadIdx.x == 0) {
-    float Xc[3], Yc[3], S[9];
-    for (int k = 0; k < 9; ++k) S[k] = s_emS[k];
-    for (int k = 0; k < 3; ++k) {
-      Xc[k] = s_emS[9 + k];
-      Yc[k] = s_emS[12 + k];
-    }
-    horn_update(P, S, Xc, Yc, ph.step, ph.step + 1 == P.nsteps);
-    __stcg(P.state + 12, __ldcg(P.state + 12) * P.sigma_factor);  // FP32, src/emicp.cu:668
-  }
-  __syncthreads();
-}
-
 __device__ __noinline__ void sa_finalize(const BPair& P, const Ph& ph, df* s_red, df* s_tot, float* s_S, float* s_v) {
   reduce_block_partials<kSaNV>(P.rec, P.g0.nblk + P.g1.nblk, s_red, s_tot);
   if (threadIdx.x < 12) {
@@ -675,8 +618,7 @@ __global__ void __launch_bounds__(kThreads, 2) batch_kernel(const BatchArgs A) {
   for (int p = tid; p < A.npairs; p += kThreads) {
     const BPair& P = A.pairs[p];
     const int done = P.hand ? P.hand->titer * P.I0 + P.hand->iter0 : 0;
-    s_sched[p] = Sched{P.algo, P.algo == 0 ? P.rounds : P.rounds - done * (2 * P.I1 + 2), P.I1, P.g0.units, P.g1.units,
-                       done};
+    s_sched[p] = Sched{P.algo == 0 ? 0 : P.rounds - done * (2 * P.I1 + 2), P.I1, P.g0.units, P.g1.units, done};
     atomicMax(&s_rounds, s_sched[p].rounds);
   }
   __syncthreads();
@@ -726,20 +668,16 @@ __global__ void __launch_bounds__(kThreads, 2) batch_kernel(const BatchArgs A) {
         const Task& tn = s_tn;
         const BPair& P = A.pairs[cur.p];
         Slot ns{0, 0u, false};
-        if (cur.ph.phase == kPhEmZ || cur.ph.phase == kPhSaZ) {
+        if (cur.ph.phase == kPhSaZ) {
           if (tn.src) ns = ring_issue(rg, sm, tn);  // lands while the pose is solved
-          if (cur.ph.phase == kPhEmZ) em_finalize(P, cur.ph, s_red, s_tot);
-          else sa_finalize(P, cur.ph, s_red, s_tot, s_S, s_v);
+          sa_finalize(P, cur.ph, s_red, s_tot, s_S, s_v);
         } else {
           df* scratch = reinterpret_cast<df*>(sm.prep);
           static_assert(offsetof(SweepSmem, full) - offsetof(SweepSmem, prep) >= 32 * (kBlockPts + 8) * sizeof(df),
                         "moment scratch does not fit");
           const BPair* PP = &A.pairs[cur.p];
           const int k = cur.ph.k;
-          if (cur.ph.phase == kPhEmE)
-            ok = run_sweep_unit<5>(sm, rg, cur, true, slot, tn, ns, P.part, P.cnt0, EmOps{PP, scratch}, s_meta,
-                                   A.ctl, A.timeout_ns, 10);
-          else if (cur.ph.phase == kPhSaRow)
+          if (cur.ph.phase == kPhSaRow)
             ok = run_sweep_unit<1>(sm, rg, cur, false, slot, tn, ns, P.part, P.cnt0, RowOps{PP, k == 0}, s_meta,
                                    A.ctl, A.timeout_ns, 30);
           else if (cur.ph.phase == kPhSaCol)
@@ -773,18 +711,17 @@ __global__ void __launch_bounds__(1024) batch_center_kernel(const BPair* pairs) 
 __global__ void batch_pack_kernel(const BPair* pairs) {
   const BPair& P = pairs[blockIdx.y];
   const CenterHdr* h = P.hdr;
-  float4* xo = P.algo == 0 ? P.own1 : P.own0;
-  float4* yo = P.algo == 0 ? P.own0 : P.own1;
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.N; i += stride) {
-    xo[i] = make_float4(__fsub_rn(P.X[i], h->oX[0]), __fsub_rn(P.X[P.N + i], h->oX[1]),
+    P.own0[i] = make_float4(__fsub_rn(P.X[i], h->oX[0]), __fsub_rn(P.X[P.N + i], h->oX[1]),
                         __fsub_rn(P.X[2 * P.N + i], h->oX[2]), 0.f);
     if (P.algo == 1) P.s[i] = P.moutlier;
   }
+  if (P.algo == 0) return;  // Y is packed in its sorted order, the pose read by the team
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.M; i += stride) {
-    yo[i] = make_float4(__fsub_rn(P.Y[i], h->oY[0]), __fsub_rn(P.Y[P.M + i], h->oY[1]),
+    P.own1[i] = make_float4(__fsub_rn(P.Y[i], h->oY[0]), __fsub_rn(P.Y[P.M + i], h->oY[1]),
                         __fsub_rn(P.Y[2 * P.M + i], h->oY[2]), 0.f);
-    if (P.algo == 1) P.u[i] = P.moutlier;
+    P.u[i] = P.moutlier;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     float R[9], t[3], tc[3];
@@ -831,11 +768,12 @@ SweepGeom batch_geom(int n_own, int n_stream, int slice) {
 // launch), the pair table, then each pair's buffers. With base == nullptr
 // only sizes are computed.
 // Slice length for a batch on a grid of G blocks: the largest sweep round
-// (sum of N M over the pairs) in about kUnitsPerBlock * G units of 128 owned
+// (sum of N M over the Softassign pairs) in about kUnitsPerBlock * G units of 128 owned
 // points, in whole TMA chunks.
 int batch_slice(const BatchLaunchPair* in, int npairs, int G) {
   double work = 0.0;
-  for (int i = 0; i < npairs; ++i) work += (double)in[i].N * (double)in[i].M;
+  for (int i = 0; i < npairs; ++i)
+    if (in[i].algo != 0) work += (double)in[i].N * (double)in[i].M;
   double chunks = work / (kUnitsPerBlock * (double)G * kBlockPts * kChunk);
   int c = (int)(chunks + 0.5);
   if (c < 1) c = 1;
@@ -847,8 +785,9 @@ int batch_slice(const BatchLaunchPair* in, int npairs, int G) {
 // counters (cleared per launch), the pair table, then each pair's buffers.
 // The pair table is ordered by decreasing size, so the largest units of a
 // round are handed out first. With base == nullptr only sizes are computed.
-size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std::vector<BPair>* out, Ctl** ctl,
-                   size_t* zero_bytes, BPair** dpairs, int* rounds, unsigned** rctr, void** series_tab) {
+size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std::vector<BPair>* out,
+                   std::vector<EmTeamJob>* teams, Ctl** ctl, size_t* zero_bytes, BPair** dpairs, int* rounds,
+                   unsigned** rctr, void** series_tab) {
   Carve c(base);
   *ctl = c.take<Ctl>(1);
   const int slice = batch_slice(in, npairs, G);
@@ -868,13 +807,9 @@ size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std
     P.N = L.N;
     P.M = L.M;
     if (L.algo == 0) {
-      P.g0 = batch_geom(L.M, L.N, slice);
-      P.g1 = SweepGeom{0, 0, 0, 1, 0, 0};
+      P.g0 = P.g1 = SweepGeom{0, 0, 0, 1, 0, 0};
       P.nsteps = L.nsteps;
       P.rounds = 2 * L.nsteps;
-      P.init = L.sigma_p2;
-      P.sigma_factor = L.sigma_factor;
-      P.d_02 = L.d_02;
       P.I0 = 1;
       P.I1 = 1;
     } else {
@@ -905,34 +840,37 @@ size_t carve_batch(void* base, const BatchLaunchPair* in, int npairs, int G, std
   size_t co = 0;
   for (int i = 0; i < npairs; ++i) {
     BPair& P = v[(size_t)i];
-    const int n0 = P.algo == 0 ? P.M : P.N;
-    const int n1 = P.algo == 0 ? P.N : P.M;
     P.cnt0 = cnt ? cnt + co : nullptr;
     co += (size_t)P.g0.nblk;
     P.cnt1 = cnt ? cnt + co : nullptr;
     co += (size_t)P.g1.nblk;
     P.hdr = c.take<CenterHdr>(1);
-    P.own0 = c.take<float4>((size_t)n0);
-    P.own1 = c.take<float4>((size_t)n1);
+    P.own0 = c.take<float4>((size_t)P.N);
+    if (P.algo == 0) {
+      const BatchLaunchPair& L = in[order[(size_t)i]];
+      if (P.nsteps > 0)
+        teams->push_back(EmTeamJob{P.N, P.M, P.nsteps, L.sigma_p2, L.sigma_factor, L.d_02, P.Y, P.own0, P.hdr, P.dRt});
+      continue;
+    }
+    P.own1 = c.take<float4>((size_t)P.M);
     const size_t part0 = (size_t)P.g0.units * 5 * kBlockPts;
     const size_t part1 = (size_t)P.g1.units * 1 * kBlockPts;
     P.part = c.take<float>(part0 > part1 ? part0 : part1);
     P.rec = c.take<df>((size_t)(P.g0.nblk + P.g1.nblk) * 32);
-    if (P.algo == 1) {
-      // padded to 4 floats: weight copies are whole 16-byte groups
-      const size_t Np = ((size_t)P.N + 3) & ~size_t(3), Mp = ((size_t)P.M + 3) & ~size_t(3);
-      P.a = c.take<float>(Np);
-      P.s = c.take<float>(Np);
-      P.rs = c.take<float>(Np);
-      P.b = c.take<float>(Mp);
-      P.u = c.take<float>(Mp);
-      P.cs = c.take<float>(Mp);
-      if (P.nsteps > 0 && P.series) P.hand = hand ? hand + i : nullptr;
-    }
+    // padded to 4 floats: weight copies are whole 16-byte groups
+    const size_t Np = ((size_t)P.N + 3) & ~size_t(3), Mp = ((size_t)P.M + 3) & ~size_t(3);
+    P.a = c.take<float>(Np);
+    P.s = c.take<float>(Np);
+    P.rs = c.take<float>(Np);
+    P.b = c.take<float>(Mp);
+    P.u = c.take<float>(Mp);
+    P.cs = c.take<float>(Mp);
+    if (P.nsteps > 0 && P.series) P.hand = hand ? hand + i : nullptr;
     P.state = c.take<float>(kStateFloats);
   }
   if (out) out->swap(v);
   *rounds = rmax;
+  c.take<char>(0);  // the teams' workspace begins where a part would
   return c.off;
 }
 
@@ -950,7 +888,9 @@ size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device) {
   unsigned* rctr = nullptr;
   void* stab = nullptr;
   const int G = persistent_grid_limit(device, (const void*)batch_kernel, batch_smem(npairs));
-  return carve_batch(nullptr, pairs, npairs, G, nullptr, &ctl, &zb, &dp, &rounds, &rctr, &stab);
+  std::vector<EmTeamJob> teams;
+  const size_t own = carve_batch(nullptr, pairs, npairs, G, nullptr, &teams, &ctl, &zb, &dp, &rounds, &rctr, &stab);
+  return own + emicp_teams_ws_need(teams.data(), (int)teams.size(), device);
 }
 
 int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint64_t timeout_ns, void* ws,
@@ -968,8 +908,10 @@ int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint6
   void* stab = nullptr;
   const size_t smem = batch_smem(npairs);
   const int limit = persistent_grid_limit(device, (const void*)batch_kernel, smem);
-  const size_t need = carve_batch(ws, pairs, npairs, limit, &host, &ctl, &zero_bytes, &dpairs, &rounds, &rctr, &stab);
-  if (need > ws_bytes) return (int)cudaErrorInvalidValue;
+  std::vector<EmTeamJob> teams;
+  const size_t own =
+      carve_batch(ws, pairs, npairs, limit, &host, &teams, &ctl, &zero_bytes, &dpairs, &rounds, &rctr, &stab);
+  if (own > ws_bytes) return (int)cudaErrorInvalidValue;
   if (rounds_out) *rounds_out = rounds;
   e = cudaMemsetAsync(ws, 0, zero_bytes, st);
   if (e == cudaSuccess)
@@ -981,9 +923,12 @@ int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint6
   if (e != cudaSuccess) return (int)e;
   if (grid_used) *grid_used = limit;
   if (rounds == 0) return 0;
+  const int te = enqueue_emicp_teams(teams.data(), (int)teams.size(), static_cast<char*>(ws) + own, ws_bytes - own, ctl,
+                                     timeout_ns, st);
+  if (te) return te;
   // The leading updates of the Softassign pairs, as far as a short series
   // represents their affinities: a cluster per pair, before the lock-step
-  // rounds (which then hold the EM-ICP pairs and what is left).
+  // rounds (which then hold what is left).
   std::vector<SeriesJob> jobs;
   for (const BPair& P : host)
     if (P.hand)

@@ -22,8 +22,11 @@
 // Coordinates are centred on the device (FP32 offsets oX, oY) before the
 // loop. EM-ICP's S is translation invariant, so only Xc, Yc and t are shifted
 // back; the pose enters and leaves in the caller's frame.
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
+#include <vector>
 
 #include "cesa_kernels.h"
 #include "cesa_ops.cuh"
@@ -105,13 +108,12 @@ struct LocalSmem {
 // As sweep_units (deferred), for the EM-ICP E-step: every unit's partial sums
 // of e^2, e and e x' (scaled frame) are stored per (row, slice or slot).
 template <int kLayout>
-__device__ __forceinline__ bool em_local_sweep(SweepSmem& sm, LocalSmem& ls, Pipe& pipe, const SweepGeom& g,
+__device__ __forceinline__ bool em_local_sweep(const int& bid, const int& G, SweepSmem& sm, LocalSmem& ls, Pipe& pipe, const SweepGeom& g,
                                                const StreamSrc& src, const float4* own, const float4* blkinfo,
                                                const float (&R)[9], const float (&tc)[3], float sc, float* part,
                                                int part_ld, Ctl* ctl, uint64_t timeout_ns, int where, Timeline& tl,
                                                OwnCache& oc, const RangedShare* rs) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = (int)gridDim.x;
   constexpr bool ranged = kLayout == 1;
   pipe.cur = -1;
   auto task_range = [&](int uu, int ch, int& first, int& len) -> bool {  // as in sweep_units
@@ -135,7 +137,7 @@ __device__ __forceinline__ bool em_local_sweep(SweepSmem& sm, LocalSmem& ls, Pip
     return true;
   };
   const int ustep = ranged ? 1 : G;
-  int u = ranged ? 0 : (int)blockIdx.x;
+  int u = ranged ? 0 : bid;
   int cur_first = 0, cur_len = 0, cur_ch = 0, cur_stage = 0;
   unsigned cur_par = 0;
   bool cur_wait = false;
@@ -198,7 +200,7 @@ __device__ __forceinline__ bool em_local_sweep(SweepSmem& sm, LocalSmem& ls, Pip
         n_par = (pipe.uses[n_stage] - 1u) & 1u;
       }
       const bool bad = cur_wait && !mbar_wait(&sm.full[cur_stage], cur_par, ctl, timeout_ns, where);
-      if (cur_ch == 0 && u == (int)blockIdx.x) tl.mark(2);
+      if (cur_ch == 0 && u == bid) tl.mark(2);
       // prepare: double-buffered, one block barrier per chunk (a stage that
       // timed out is read as it is; the block leaves after the barrier)
       float4* buf = par ? sm.prep2 : sm.prep;
@@ -286,9 +288,17 @@ __device__ __forceinline__ bool em_local_sweep(SweepSmem& sm, LocalSmem& ls, Pip
   return true;
 }
 
-__global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
+// A block's part in emicp_teams_kernel: jobs [first, first + njobs), block
+// `rank` of the `size` blocks that run them.
+struct TeamBlock {
+  int first, njobs, rank, size;
+};
+
+// One registration by blocks 0 .. G - 1, this one block bid; false after a
+// failure (status set). kTeam: one of several in the launch (local sweeps, no
+// tape); the caller has initialised the stage barriers and the pipe.
+template <bool kTeam>
+__device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pipe& pipe, const int& bid, const int& G) {
   __shared__ float s_pose[12];
   __shared__ df s_red[kThreads];
   __shared__ OwnCache oc_rows;
@@ -301,11 +311,12 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
   __shared__ float s_hdr[12];
 
   const int tid = threadIdx.x;
-  const unsigned G = gridDim.x;
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
-    mbar_init_fence();
+    if (!kTeam) {
+      for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
+      mbar_init_fence();
+    }
     for (int k = 0; k < 3; ++k) {
       s_hdr[k] = A.hdr->oX[k];
       s_hdr[3 + k] = A.hdr->oY[k];
@@ -318,11 +329,15 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     for (int k = 0; k < 9; ++k) s_pose[k] = R[k];
     for (int k = 0; k < 3; ++k) s_pose[9 + k] = tc[k];
     oc_rows.blk = -1;
-    int vb = (int)blockIdx.x;  // the virtual block whose share this block sweeps
+    int vb = bid;  // the virtual block whose share this block sweeps
     s_pair[0] = -1;
-    if (A.geo.pair_num) {
+    if (kTeam && A.geo.pair_num) {  // ranks 2 d and 2 d + 1 share an SM
+      s_pair[0] = bid >> 1;
+      s_pair[1] = bid & 1;
+      s_pair[2] = 0;
+    } else if (A.geo.pair_num) {
       const int2 pr = join_sm_pair(A.pair_tab, A.timeout_ns);
-      if (pr.x >= 0 && pr.x < (int)G / 2) {
+      if (pr.x >= 0 && pr.x < G / 2) {
         s_pair[0] = pr.x;
         s_pair[1] = pr.y;
         s_pair[2] = 0;
@@ -331,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
         set_status(A.ctl, kStatusInternal, 23);  // the launch ends at its first grid barrier
       }
     }
-    rs_rows = A.geo.pair_num && s_pair[0] < 0 ? RangedShare{0, -1, 0, 0, 0} : ranged_share(A.geo, vb, (int)G);
+    rs_rows = A.geo.pair_num && s_pair[0] < 0 ? RangedShare{0, -1, 0, 0, 0} : ranged_share(A.geo, vb, G);
   }
   __syncthreads();
 
@@ -341,12 +356,12 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     horn.reset();
     horn_tape.reset();
   }
-  Pipe pipe;
-  pipe_init(pipe);
+  if (!kTeam) pipe_init(pipe);
   unsigned epoch = 0;
   const StreamSrc src{A.cols, nullptr, true};
   float s2 = A.sigma0;
-  Timeline tl{A.tl, A.tl_cap, 0};
+  Timeline tl{kTeam ? nullptr : A.tl, A.tl_cap, 0};
+  bool good = true;
   for (int step = 0; step < A.nsteps; ++step) {
     tl.mark(1);
     const float outlier = expf(-A.d_02 / s2);  // src/emicp.cu:489
@@ -360,37 +375,45 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     // e = exp(-d2 / (2 s2)) = 2^(nk d2). Every unit stores its rows' partial
     // sums over its column slice (deferred: no completion counter).
     const float sc = sqrtf(kLog2e / (2.f * s2));
-    if (A.blk) {
+    if (kTeam || A.blk) {
       float Rs[9], tcs[3];
 #pragma unroll
       for (int k = 0; k < 9; ++k) Rs[k] = R[k] * sc;
 #pragma unroll
       for (int k = 0; k < 3; ++k) tcs[k] = tc[k] * sc;
       if (tid == 0 && s_pair[0] >= 0) s_tsweep = global_ns();
-      const bool ok = A.geo.ranged
-                          ? em_local_sweep<1>(sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
+      const bool ok = kTeam || A.geo.ranged
+                          ? em_local_sweep<1>(bid, G, sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
                                               A.ctl, A.timeout_ns, 10, tl, oc_rows, &rs_rows)
-                          : em_local_sweep<0>(sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
+                          : em_local_sweep<0>(bid, G, sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
                                               A.ctl, A.timeout_ns, 10, tl, oc_rows, nullptr);
-      if (!ok) break;
+      if (!ok) {
+        good = false;
+        break;
+      }
       if (tid == 0 && s_pair[0] >= 0)
         A.pair_t[2 * s_pair[0] + (s_pair[1] ^ s_pair[2])] = (float)(global_ns() - s_tsweep);
     } else {
       const EmicpElem elem{-kLog2e / (2.f * s2)};
       if (!sweep_units<5, EmicpElem, NoPrep, NoFin, true, 0>(sm, pipe, A.geo, src, A.rows, true, R, tc, 0u, A.part,
                                                            nullptr, elem, NoPrep{}, NoFin{}, A.ctl, A.timeout_ns, 10,
-                                                           tl, A.Mp, &oc_rows))
+                                                           tl, A.Mp, &oc_rows)) {
+        good = false;
         break;
+      }
     }
-    if (!grid_sync(A.ctl, epoch, G, A.timeout_ns, 20)) break;
+    if (!grid_sync(A.ctl, epoch, (unsigned)G, A.timeout_ns, 20)) {
+      good = false;
+      break;
+    }
     tl.mark(5);
     if (tid == 0 && s_pair[0] >= 0) {  // SM pairs: the parts change blocks when the times show the other favoured
       long lo = 0, sp = 0, hi = 0;
-      ranged_tasks(A.geo, 2 * s_pair[0], (int)G, lo, sp);
-      ranged_tasks(A.geo, 2 * s_pair[0] + 1, (int)G, sp, hi);
+      ranged_tasks(A.geo, 2 * s_pair[0], G, lo, sp);
+      ranged_tasks(A.geo, 2 * s_pair[0] + 1, G, sp, hi);
       if (pair_swap(lo, sp, hi, A.pair_t, s_pair[0])) {
         s_pair[2] ^= 1;
-        rs_rows = ranged_share(A.geo, 2 * s_pair[0] + (s_pair[1] ^ s_pair[2]), (int)G);
+        rs_rows = ranged_share(A.geo, 2 * s_pair[0] + (s_pair[1] ^ s_pair[2]), G);
       }
     }
     // ---- rows completed, each block a contiguous share of them; its 16
@@ -400,9 +423,9 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     df* rb = A.rbpart + (size_t)(step & 1) * G * kEmNV;
     {
       const int S = A.geo.slices;
-      const float inv_sc = A.blk ? 1.f / sc : 1.f;  // local sweeps: the e x sums are sc times too large
-      const int rpc = (A.M + (int)G - 1) / (int)G;
-      const int r0 = (int)blockIdx.x * rpc;
+      const float inv_sc = kTeam || A.blk ? 1.f / sc : 1.f;  // local sweeps: the e x sums are sc times too large
+      const int rpc = (A.M + G - 1) / G;
+      const int r0 = bid * rpc;
       const int nrows = max(0, min(rpc, A.M - r0));
       float* stot = reinterpret_cast<float*>(&sm.raw2[0][0]);  // [kThreads][5]; raw2 carries no stream here
       static_assert(sizeof(sm.raw2) >= sizeof(float) * 5 * kThreads, "row sums scratch");
@@ -418,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
         const int nr = min(kThreads, nrows - c0);
         for (int pq = tid; pq < 5 * nr; pq += kThreads) {
           const int a = pq % 5, rr = pq / 5;
-          if (A.geo.ranged) {  // the kmax slots of the row's owned block, in task order
+          if (kTeam || A.geo.ranged) {  // the kmax slots of the row's owned block, in task order
             const int kmax = A.geo.kmax;
             const float* P = A.part + (size_t)a * A.geo.nblk * kmax * kBlockPts + ranged_slot0(r0 + c0 + rr, kmax);
             float sum = 0.f;
@@ -461,15 +484,18 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
         }
         __syncthreads();
       }
-      em_block_moments(v, min(nrows, kThreads), reinterpret_cast<df*>(sm.prep), rb + (size_t)blockIdx.x * kEmNV);
+      em_block_moments(v, min(nrows, kThreads), reinterpret_cast<df*>(sm.prep), rb + (size_t)bid * kEmNV);
     }
-    if (!grid_sync(A.ctl, epoch, G, A.timeout_ns, 21)) break;
+    if (!grid_sync(A.ctl, epoch, (unsigned)G, A.timeout_ns, 21)) {
+      good = false;
+      break;
+    }
     tl.mark(8);
 
     // ---- grid-wide moments -> pose (every block computes the same pose)
-    reduce_block_partials<kEmNV>(rb, (int)G, s_red, s_tot);
+    reduce_block_partials<kEmNV>(rb, G, s_red, s_tot);
     tl.mark(6);
-    const bool refine = A.blk && step + kRefineSteps >= A.nsteps;
+    const bool refine = (kTeam || A.blk) && step + kRefineSteps >= A.nsteps;
     em_moments_to_S_block(s_tot, s_emS, refine);
     if (tid == 0) {
       float Xc[3], Yc[3], S[9];
@@ -485,7 +511,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
       quat_to_pose<float>(q, Xc, Yc, Rn, tn);
       if (refine)
         horn_refine_dd(s_emS, s_emS + 15, s_emS + 9, s_emS + 24, s_emS + 12, s_emS + 27, q, Rn, tn);
-      if (A.tape && blockIdx.x == 0) {  // the step's inputs and solve for the adjoint
+      if (!kTeam && A.tape && bid == 0) {  // the step's inputs and solve for the adjoint
         // the adjoint's eigenbasis, from a Jacobi solve of the same S on its own
         // state (it does not feed back into the pose)
         float qj[4], gj = 0.f, lj = 0.f;
@@ -503,8 +529,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
       }
       for (int k = 0; k < 9; ++k) s_pose[k] = Rn[k];
       for (int k = 0; k < 3; ++k) s_pose[9 + k] = tn[k];
-      if (blockIdx.x == 0) {
-        if (A.trace && step < A.trace_cap) {
+      if (bid == 0) {
+        if (!kTeam && A.trace && step < A.trace_cap) {
           double* rec = A.trace + (size_t)step * 32;
           float to[3];
           pose_from_centred(Rn, tn, &s_hdr[0], &s_hdr[3], to);
@@ -531,7 +557,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     s2 *= A.sigma_factor;  // FP32, src/emicp.cu:668
   }
 
-  if (blockIdx.x == 0 && tid == 0) {
+  if (bid == 0 && tid == 0) {
     const int st = ld_status(A.ctl);
     if (st == kStatusOk) {
       float R[9], tc[3], t[3];
@@ -543,6 +569,72 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
     }
     if (A.d_status) *A.d_status = st;
     if (A.tl) A.ctl->pad[0] = (unsigned)tl.n;
+  }
+  return good;
+}
+
+__global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Pipe pipe;
+  emicp_run<false>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// Many registrations in one cooperative launch, each by a team of blocks of
+// its own: a team goes through its registrations one after the other and waits
+// for nobody else, so that pairs of any sizes fill the chip without a step of
+// one being a step of all (plan_teams). All sweeps are local and ranged: one
+// sweep loop (with the slice layout beside it ptxas made it 8% slower), its
+// arguments in shared memory. In lock step over all pairs, with direct
+// differences, a step paid two grid barriers and a last wave of units; lock step
+// -> teams: one pair of 600 x 500 1.58 -> 1.00 ms, 20 of 2000 x 2000 4.47 ->
+// 3.04, 60 9.43 -> 6.97, 20 of 6000 x 6000 20.8 -> 17.2, 20 of 500-20,000 points
+// 8.8 / 16.3 / 12.3 -> 6.2 / 13.4 / 9.9 (three sets). Bound by the FP32 pipe and, in
+// small pairs, by a step's latency; the teams' sizes are even numbers of
+// blocks, which leaves up to 8% of the chip idle (20 x 14 of 304 blocks).
+__global__ void __launch_bounds__(kThreads, 2) emicp_teams_kernel(const EmicpArgs* __restrict__ jobs,
+                                                                  const TeamBlock* __restrict__ blocks, Ctl* ctl,
+                                                                  unsigned* pair_tab, uint64_t timeout_ns) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
+  __shared__ EmicpArgs s_args;
+  static_assert(sizeof(EmicpArgs) % 4 == 0 && sizeof(EmicpArgs) / 4 <= kThreads, "copied by one word a thread");
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
+    mbar_init_fence();
+  }
+  __shared__ int s_vb;
+  __shared__ TeamBlock s_team;
+  if (tid == 0) {  // SM pairs: virtual blocks 2 d and 2 d + 1 are an SM's two
+    int vb = (int)blockIdx.x;
+    if (pair_tab) {
+      const int2 pr = join_sm_pair(pair_tab, timeout_ns);
+      vb = pr.x >= 0 && pr.x < (int)gridDim.x / 2 ? 2 * pr.x + pr.y : -1;
+      if (vb < 0) set_status(ctl, kStatusInternal, 25);
+    }
+    s_vb = vb;
+  }
+  Pipe pipe;
+  pipe_init(pipe);
+  __syncthreads();
+  if (s_vb < 0) return;
+  const int vb = s_vb;
+  if (tid == 0) s_team = blocks[vb];
+  for (;;) {
+    __syncthreads();
+    if (s_team.njobs <= 0) return;
+    if (tid < (int)(sizeof(EmicpArgs) / 4))
+      reinterpret_cast<unsigned*>(&s_args)[tid] = reinterpret_cast<const unsigned*>(jobs + s_team.first)[tid];
+    __syncthreads();
+    if (!emicp_run<true>(s_args, sm, pipe, s_team.rank, s_team.size)) {
+      if (tid == 0) set_status(ctl, ld_status(s_args.ctl), 24);
+      return;
+    }
+    if (tid == 0) {
+      s_team.first += 1;
+      s_team.njobs -= 1;
+    }
+    for (int s = 0; s < kStages; ++s) pipe.tag[s] = -1;  // the next pair's chunks are others
   }
 }
 
@@ -588,8 +680,7 @@ __device__ __forceinline__ unsigned hilbert_index(unsigned (&x)[3]) {
 // the w-th contiguous segment, so that the order does not depend on timing.
 // perm receives it (tmp: scratch of M). One block: 40,097 points take about
 // 0.1% of the registration that they are sorted for.
-__global__ void __launch_bounds__(1024) em_sort_kernel(const float* __restrict__ Y, int M, unsigned* keys, int* perm,
-                                                       int* tmp) {
+__device__ __forceinline__ void em_sort(const float* __restrict__ Y, int M, unsigned* keys, int* perm, int* tmp) {
   constexpr int kW = 32, kDig = 256;
   __shared__ float s_lo[3][kW], s_hi[3][kW];
   __shared__ int s_cnt[kDig * kW];  // [digit][warp]
@@ -692,9 +783,14 @@ __global__ void __launch_bounds__(1024) em_sort_kernel(const float* __restrict__
   }
 }
 
+__global__ void __launch_bounds__(1024) em_sort_kernel(const float* __restrict__ Y, int M, unsigned* keys, int* perm,
+                                                       int* tmp) {
+  em_sort(Y, M, keys, perm, tmp);
+}
+
 // Y' in the order perm (null: as given): (y - o, index in the caller's order).
-__global__ void em_pack_rows_kernel(const float* __restrict__ Y, int M, const CenterHdr* hdr,
-                                    const int* __restrict__ perm, float4* __restrict__ out) {
+__device__ __forceinline__ void em_pack_rows(const float* __restrict__ Y, int M, const CenterHdr* hdr,
+                                             const int* __restrict__ perm, float4* __restrict__ out) {
   const float* o = hdr->oY;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
     const int i = perm ? perm[r] : r;
@@ -703,10 +799,14 @@ __global__ void em_pack_rows_kernel(const float* __restrict__ Y, int M, const Ce
   }
 }
 
-// Centre of every owned block's bounding box and its points' largest distance
-// from it (NaN where a coordinate is not finite).
-__global__ void __launch_bounds__(kBlockPts) em_block_kernel(const float4* __restrict__ rows, int M,
-                                                            float4* __restrict__ out) {
+__global__ void em_pack_rows_kernel(const float* __restrict__ Y, int M, const CenterHdr* hdr,
+                                    const int* __restrict__ perm, float4* __restrict__ out) {
+  em_pack_rows(Y, M, hdr, perm, out);
+}
+
+// Centre of an owned block's (blockIdx.x) bounding box and its points' largest
+// distance from it (NaN where a coordinate is not finite).
+__device__ __forceinline__ void em_block(const float4* __restrict__ rows, int M, float4* __restrict__ out) {
   constexpr int kW = kBlockPts / 32;
   __shared__ float s_lo[3][kW], s_hi[3][kW], s_r[kW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -747,6 +847,37 @@ __global__ void __launch_bounds__(kBlockPts) em_block_kernel(const float4* __res
   }
 }
 
+__global__ void __launch_bounds__(kBlockPts) em_block_kernel(const float4* __restrict__ rows, int M,
+                                                            float4* __restrict__ out) {
+  em_block(rows, M, out);
+}
+
+// The same for the pairs of a batch.
+struct TeamPrep {
+  const float* Y;
+  int M;
+  const CenterHdr* hdr;
+  unsigned* keys;
+  int* perm;
+  float4* rows;
+  float4* blk;
+};
+
+__global__ void __launch_bounds__(1024) em_sort_teams_kernel(const TeamPrep* __restrict__ tab) {
+  const TeamPrep P = tab[blockIdx.x];
+  em_sort(P.Y, P.M, P.keys, P.perm, P.perm + P.M);
+}
+
+__global__ void em_pack_teams_kernel(const TeamPrep* __restrict__ tab) {
+  const TeamPrep P = tab[blockIdx.y];
+  em_pack_rows(P.Y, P.M, P.hdr, P.perm, P.rows);
+}
+
+__global__ void __launch_bounds__(kBlockPts) em_block_teams_kernel(const TeamPrep* __restrict__ tab) {
+  const TeamPrep P = tab[blockIdx.y];
+  if ((int)blockIdx.x * kBlockPts < P.M) em_block(P.rows, P.M, P.blk);
+}
+
 // ------------------------------------------------------------------ host side
 
 namespace {
@@ -772,6 +903,8 @@ struct EmicpPlan {
 
 size_t sweep_smem() { return sizeof(SweepSmem); }
 
+constexpr int kEmPairNum = 208;  // SM pairs: the favoured block's share, 13 / 16
+
 // The local sweep (and the sort that it wants) from 2.4e7 affinities a step on:
 // below, a step is mostly latency and the prepare step's barrier per chunk
 // costs as much as the shorter element gives (4001^2: 1.045 -> 1.043 ms, 3000^2
@@ -795,7 +928,7 @@ EmicpPlan plan_emicp(int N, int M, int device) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const char* ev = getenv("CESA_SM_PAIRS");  // "0": equal shares (for comparisons)
-    if (sms > 0 && limit == 2 * sms && !(ev && ev[0] == '0')) P.geo.pair_num = 208;  // 13 / 16
+    if (sms > 0 && limit == 2 * sms && !(ev && ev[0] == '0')) P.geo.pair_num = kEmPairNum;
     make_ranged(P.geo, limit);
     P.grid = limit;
   }
@@ -916,6 +1049,208 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   e = cudaLaunchCooperativeKernel((const void*)emicp_kernel, dim3(P.grid), dim3(kThreads), args,
                                   P.smem, st);
   return (int)e;
+}
+
+namespace {
+// A batch's registrations over the launch's blocks. A registration takes about
+// nsteps (kTeamStepNs + M (N kTeamElemNs + kTeamRowNs) / g) on g blocks (an
+// element of a block that shares its SM: 0.096-0.098 measured for M <= 5120; a
+// row's sums and completion; the barriers and the pose of a step). For the least
+// t that the blocks can keep, every one that needs more than a block gets the
+// fewest that hold it to t, and the others go to single blocks, as many on one
+// as stay below t. Teams of whole SMs come first (their pairs of blocks split
+// the sweep by pair_num); an odd number of blocks, or one, takes kTeamOdd times
+// as long for the lack of that. The blocks of a pair depend on t and its own
+// size, not on where it stands in the batch.
+constexpr double kTeamElemNs = 0.095, kTeamRowNs = 30.0, kTeamStepNs = 8000.0, kTeamOdd = 1.2;
+
+struct TeamPlan {
+  std::vector<TeamBlock> blocks;
+  std::vector<int> order;  // job -> index in the caller's list
+  std::vector<int> size;   // blocks of every job
+};
+
+TeamPlan plan_teams(const EmTeamJob* jobs, int n, int G) {
+  TeamPlan P;
+  std::vector<double> cost((size_t)n), need((size_t)n);  // need: time on one block
+  P.order.resize((size_t)n);
+  P.size.resize((size_t)n);
+  double sum = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double steps = (double)jobs[i].nsteps;
+    P.order[(size_t)i] = i;
+    cost[(size_t)i] = steps * (double)jobs[i].M * ((double)jobs[i].N * kTeamElemNs + kTeamRowNs);
+    need[(size_t)i] = kTeamOdd * cost[(size_t)i] + steps * kTeamStepNs;
+    sum += need[(size_t)i];
+  }
+  std::stable_sort(P.order.begin(), P.order.end(), [&](int a, int b) { return need[(size_t)a] > need[(size_t)b]; });
+  // sizes for a time t, and the blocks they take (more than G: not kept)
+  auto fill = [&](double t) -> long {
+    long used = 0;
+    double left = 0.0;
+    for (int j = 0; j < n && used <= G; ++j) {
+      const size_t i = (size_t)P.order[(size_t)j];
+      const double run = t - jobs[i].nsteps * kTeamStepNs;
+      int g = 1;
+      if (need[i] > t) {
+        const double e = run > 0.0 ? std::ceil(0.5 * cost[i] / run) * 2.0 : 2.0 * G;
+        const double o = run > 0.0 ? std::ceil(kTeamOdd * cost[i] / run) : 2.0 * G;
+        g = (int)std::min(std::min(e, o), 2.0 * G);
+        used += g;
+      } else if (left >= need[i]) {
+        left -= need[i];
+      } else {
+        left = t - need[i];
+        used += 1;
+      }
+      P.size[(size_t)j] = g;
+    }
+    return used;
+  };
+  double lo = 0.0, hi = sum;  // all on one block
+  for (int k = 0; k < 24; ++k) {
+    const double t = 0.5 * (lo + hi);
+    if (fill(t) <= G) hi = t;
+    else lo = t;
+  }
+  fill(hi);
+  for (int odd = 0; odd < 2; ++odd)
+    for (int j = 0; j < n; ++j) {
+      const int g = P.size[(size_t)j];
+      if (g > 1 && (g & 1) == odd)
+        for (int r = 0; r < g; ++r) P.blocks.push_back(TeamBlock{j, 1, r, g});
+    }
+  double left = -1.0;
+  for (int j = 0; j < n; ++j) {  // single blocks: consecutive in the order
+    if (P.size[(size_t)j] > 1) continue;
+    const double w = need[(size_t)P.order[(size_t)j]];
+    if (left >= w) {
+      left -= w;
+      P.blocks.back().njobs += 1;
+    } else {
+      left = hi - w;
+      P.blocks.push_back(TeamBlock{j, 1, 0, 1});
+    }
+  }
+  if ((int)P.blocks.size() < G) P.blocks.resize((size_t)G, TeamBlock{0, 0, 0, 0});  // the rest idle
+  return P;
+}
+
+struct TeamsCarved {
+  Ctl* ctl;  // one per job; cleared, as are the ranged partials behind them
+  unsigned* pair_tab;
+  size_t zero_bytes, total;
+  EmicpArgs* args;
+  TeamPrep* prep;
+  TeamBlock* blocks;
+  std::vector<EmicpArgs> hargs;
+  std::vector<TeamPrep> hprep;
+};
+
+TeamsCarved carve_teams(void* base, const EmTeamJob* jobs, int n, const TeamPlan& P, bool pairs,
+                        uint64_t timeout_ns) {
+  TeamsCarved w;
+  Carve c(base);
+  w.ctl = c.take<Ctl>((size_t)n);
+  w.pair_tab = c.take<unsigned>(pairs ? 2 * kPairCap + 1 : 0);
+  if (!pairs) w.pair_tab = nullptr;
+  w.hargs.resize((size_t)n);
+  w.hprep.resize((size_t)n);
+  for (int j = 0; j < n; ++j) {
+    const EmTeamJob& J = jobs[P.order[(size_t)j]];
+    EmicpArgs& A = w.hargs[(size_t)j];
+    A = EmicpArgs{};
+    const int g = P.size[(size_t)j];
+    const SweepGeomH h = plan_sweep(J.M, J.N, g);
+    A.geo = SweepGeom{h.n_own, h.n_stream, h.nblk, h.slices, h.slice_len, h.units, 0, 0, 0, 0};
+    {
+      if (pairs && g % 2 == 0) A.geo.pair_num = kEmPairNum;
+      make_ranged(A.geo, g);
+    }
+    A.cols = J.cols;
+    A.M = J.M;
+    A.N = J.N;
+    A.sigma0 = J.sigma_p2;
+    A.sigma_factor = J.sigma_factor;
+    A.d_02 = J.d_02;
+    A.nsteps = J.nsteps;
+    A.hdr = J.hdr;
+    A.dRt = J.dRt;
+    A.Mp = (J.M + 3) & ~3;
+    A.ctl = w.ctl ? w.ctl + j : nullptr;
+    A.timeout_ns = timeout_ns;
+    if (A.geo.ranged) A.part = c.take<float>((size_t)5 * A.geo.nblk * A.geo.kmax * kBlockPts);
+  }
+  w.zero_bytes = c.off;
+  w.args = c.take<EmicpArgs>((size_t)n);
+  w.prep = c.take<TeamPrep>((size_t)n);
+  w.blocks = c.take<TeamBlock>(P.blocks.size());
+  for (int j = 0; j < n; ++j) {
+    const EmTeamJob& J = jobs[P.order[(size_t)j]];
+    EmicpArgs& A = w.hargs[(size_t)j];
+    if (!A.geo.ranged) A.part = c.take<float>((size_t)5 * A.geo.slices * A.Mp);
+    A.rbpart = c.take<df>((size_t)2 * P.size[(size_t)j] * kEmNV);
+    A.pair_t = c.take<float>((size_t)P.size[(size_t)j]);
+    float4* blk = c.take<float4>((size_t)A.geo.nblk);
+    unsigned* keys = c.take<unsigned>((size_t)J.M);
+    int* perm = c.take<int>((size_t)2 * J.M);
+    float4* rows = c.take<float4>((size_t)J.M);
+    A.rows = rows;
+    A.blk = blk;
+    w.hprep[(size_t)j] = TeamPrep{J.dY, J.M, J.hdr, keys, perm, rows, blk};
+  }
+  w.total = c.off;
+  return w;
+}
+
+int teams_grid(int device, bool* pairs) {
+  const int G = persistent_grid_limit(device, (const void*)emicp_teams_kernel, sweep_smem());
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  *pairs = sms > 0 && G == 2 * sms;
+  return G;
+}
+}  // namespace
+
+size_t emicp_teams_ws_need(const EmTeamJob* jobs, int n, int device) {
+  if (n < 1) return 0;
+  bool pairs = false;
+  const TeamPlan P = plan_teams(jobs, n, teams_grid(device, &pairs));
+  return carve_teams(nullptr, jobs, n, P, pairs, 0).total;
+}
+
+int enqueue_emicp_teams(const EmTeamJob* jobs, int n, void* ws, size_t ws_bytes, void* ctl, uint64_t timeout_ns,
+                        cudaStream_t st) {
+  if (n < 1) return 0;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  bool pairs = false;
+  const int G = teams_grid(device, &pairs);
+  const TeamPlan P = plan_teams(jobs, n, G);
+  TeamsCarved w = carve_teams(ws, jobs, n, P, pairs, timeout_ns);
+  if (w.total > ws_bytes || (int)P.blocks.size() != G) return (int)cudaErrorInvalidValue;
+  int max_blk = 1;
+  for (const EmicpArgs& A : w.hargs) max_blk = A.geo.nblk > max_blk ? A.geo.nblk : max_blk;
+  e = cudaMemsetAsync(ws, 0, w.zero_bytes, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(w.args, w.hargs.data(), sizeof(EmicpArgs) * (size_t)n, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(w.prep, w.hprep.data(), sizeof(TeamPrep) * (size_t)n, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(w.blocks, P.blocks.data(), sizeof(TeamBlock) * P.blocks.size(), cudaMemcpyHostToDevice, st);
+  if (e != cudaSuccess) return (int)e;
+  em_sort_teams_kernel<<<n, 1024, 0, st>>>(w.prep);
+  em_pack_teams_kernel<<<dim3(16, n), 256, 0, st>>>(w.prep);
+  em_block_teams_kernel<<<dim3(max_blk, n), kBlockPts, 0, st>>>(w.prep);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;
+  const EmicpArgs* jobs_d = w.args;
+  const TeamBlock* blocks_d = w.blocks;
+  Ctl* main_ctl = static_cast<Ctl*>(ctl);
+  void* args[] = {(void*)&jobs_d, (void*)&blocks_d, (void*)&main_ctl, (void*)&w.pair_tab, (void*)&timeout_ns};
+  return (int)cudaLaunchCooperativeKernel((const void*)emicp_teams_kernel, dim3(G), dim3(kThreads), args, sweep_smem(),
+                                          st);
 }
 
 int read_ws_status(void* ws, cudaStream_t st, int* status, int* steps, int* tl_written) {

@@ -185,7 +185,21 @@ bool softassign_band_preferred(int N, int M, int device);
 size_t softassign_band_ws_need(int N, int M, int device);
 int enqueue_softassign_band(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, int* grid_used);
 
-// Batched registration: all pairs in one persistent launch.
+// The EM-ICP registrations of a batch in one persistent launch, each by a team
+// of blocks. ctl: where a failure is recorded.
+struct EmTeamJob {
+  int N, M, nsteps;
+  float sigma_p2, sigma_factor, d_02;
+  const float* dY;       // SoA, M
+  const float4* cols;    // X' centred (N)
+  const CenterHdr* hdr;
+  float* dRt;            // PoseIO in/out (device)
+};
+size_t emicp_teams_ws_need(const EmTeamJob* jobs, int n, int device);
+int enqueue_emicp_teams(const EmTeamJob* jobs, int n, void* ws, size_t ws_bytes, void* ctl, uint64_t timeout_ns,
+                        cudaStream_t st);
+
+// Batched registration.
 size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device);
 int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint64_t timeout_ns, void* ws,
                   size_t ws_bytes, cudaStream_t st, int* grid_used, int* rounds_out);

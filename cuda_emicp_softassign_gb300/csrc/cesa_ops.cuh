@@ -111,30 +111,6 @@ __device__ __forceinline__ void emicp_row_finish(int r, int r_out, const float (
     for (int i = 0; i < 3; ++i) df_add_prod(v[7 + i + 3 * j], uu[i], yy[j]);
 }
 
-// Row finalize of a split-completed owned block (the batched kernel): every
-// row's emicp_row_finish, then the block's 16 moments (block accumulator,
-// compensated).
-struct EmicpFin {
-  const float4* rows;
-  int M;
-  float outlier;
-  float xm[3];
-  float* row_out;  // caller frame: u = lambda X' + lambda oX
-  float oX[3];
-  df* scratch;     // shared, >= 17 * 128 dfs
-  df* rbpart;      // this step's [nblk][kEmNV]
-  float* row_tape; // optional: this step's [M][5] (C, lambda, u) in the centred frame
-  __device__ void operator()(int blk, const float (&tot)[5]) const {
-    df v[kEmNV];
-#pragma unroll
-    for (int k = 0; k < kEmNV; ++k) v[k] = df_make(0.f);
-    const int r = blk * kBlockPts + (int)threadIdx.x;
-    if (threadIdx.x < kBlockPts && r < M)
-      emicp_row_finish(r, r, tot, ld_cg(rows + r), outlier, xm, row_out, oX, row_tape, v);
-    owned_block_sum<kEmNV>(v, scratch, rbpart + (size_t)blk * kEmNV);
-  }
-};
-
 // Sum over the block of the 16 moments held by threads 0..active-1 (active <=
 // kThreads), through shared memory in a fixed order: value k of thread i at
 // scratch[k * kThreads + i]; thread (k, g) = (tid % 16, tid / 16) adds entries
