@@ -13,11 +13,14 @@
 // A = e^2 and sqrt(A / C) = e / sqrt(C). Per row, three running sums over the
 // columns give everything: sum e^2, sum e, sum e*x. Then
 //   C_r = sum e^2 + outlier,  lambda_r = sum e / sqrt(C_r),  lambda_r X'_r = sum e x / sqrt(C_r).
-// Per element that is 3 FADD (direct differences), FMUL + 2 FFMA (d^2),
-// FMUL (scale), 1 MUFU ex2, and FFMA + FADD + 3 FFMA (accumulators): 12 FP32
-// pipe ops + 1 MUFU op. Large clouds take the ranged sweep on clouds scaled by
-// sqrt(log2(e) / (2 sigma_p2)) (a scaled copy of X' per step), which drops the
-// scale multiply: 11 FP32 ops.
+// Three forms, by size (plan_emicp):
+//   small clouds    whole rows to a block, X in shared memory, one grid barrier a
+//                   step: direct differences on scaled coordinates, 11 FP32 pipe ops
+//                   + 1 MUFU per element;
+//   large clouds    the local sweep: Y sorted, every unit about a centre of its
+//                   own, 8 ops + 1 MUFU;
+//   what is left    (few rows against many columns) (row block, column slice)
+//                   units, direct differences and a scale: 12 ops + 1 MUFU.
 //
 // Coordinates are centred on the device (FP32 offsets oX, oY) before the
 // loop. EM-ICP's S is translation invariant, so only Xc, Yc and t are shifted
@@ -288,6 +291,134 @@ __device__ __forceinline__ bool em_local_sweep(const int& bid, const int& G, Swe
   return true;
 }
 
+// ---------------------------------------------------------------- small clouds
+// A step of small clouds is a chain of latencies, of which the general path's
+// two grid barriers are the largest. Here a block owns whole rows (up to 32)
+// and holds all of X in shared memory: its rows' sums are complete within the
+// block, and a step has one grid barrier (for the moments). A thread takes every
+// 256th pair of columns against 4 rows at a time: direct differences, 11
+// FP32 ops per element (the scale rides on the difference's FFMA). Bound by that
+// chain (about 5.7 us a step) up to 2000 points, by the FP32 pipe from 5000 on:
+// N = M = 1007 591 -> 426 us, 8171 x 6007 1897 -> 1679 (device call).
+constexpr int kRowsOwn = 32;                // most rows of a block
+constexpr int kRowsMaxN = 8192;             // X in shared memory, two blocks to an SM
+constexpr int kRowsPad = 2 * kThreads;      // columns are padded to this
+struct RowsSmem {
+  float4 y[kRowsOwn];                       // this block's rows
+  float4 nz[kRowsOwn];                      // -z of the step, scaled
+  float part[kRowsOwn / 4][kWarps][4][5];   // per-warp sums of (pass, row, accumulator)
+  df mom[kEmNV][kRowsOwn + 1];
+};
+__host__ __device__ constexpr size_t rows_smem(int N) {
+  return sizeof(RowsSmem) + sizeof(float) * 3 * (size_t)((N + kRowsPad - 1) / kRowsPad * kRowsPad);
+}
+
+__device__ __forceinline__ void rows_load(const EmicpArgs& A, RowsSmem& rs, float* xs, int r0, int nrows) {
+  const int Np = (A.N + kRowsPad - 1) / kRowsPad * kRowsPad;
+  for (int i = threadIdx.x; i < Np; i += kThreads) {
+    // padding columns: far away, affinity 0
+    const float4 x = i < A.N ? ld_cg(A.cols + i) : make_float4(1e18f, 1e18f, 1e18f, 0.f);
+    xs[i] = x.x;
+    xs[Np + i] = x.y;
+    xs[2 * Np + i] = x.z;
+  }
+  if ((int)threadIdx.x < kRowsOwn)
+    rs.y[threadIdx.x] = (int)threadIdx.x < nrows ? ld_cg(A.rows + r0 + threadIdx.x) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Every row's sums of e^2, e and e x over all columns, per warp, into rs.part.
+__device__ __forceinline__ void rows_sweep(const EmicpArgs& A, RowsSmem& rs, const float* xs, float sc, int nrows) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int Np2 = (A.N + kRowsPad - 1) / kRowsPad * kThreads;  // pairs of columns
+  const float2* x2 = reinterpret_cast<const float2*>(xs);
+  const float2 sc2 = make_float2(sc, sc);
+  for (int p = 0; 4 * p < nrows; ++p) {
+    float2 q[4][3], acc[4][5];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float4 z = rs.nz[4 * p + r];
+      q[r][0] = dup2(z.x);
+      q[r][1] = dup2(z.y);
+      q[r][2] = dup2(z.z);
+#pragma unroll
+      for (int a = 0; a < 5; ++a) acc[r][a] = make_float2(0.f, 0.f);
+    }
+#pragma unroll 2
+    for (int i = tid; i < Np2; i += kThreads) {
+      const float2 x = x2[i], y = x2[Np2 + i], z = x2[2 * Np2 + i];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 dx = __ffma2_rn(x, sc2, q[r][0]), dy = __ffma2_rn(y, sc2, q[r][1]), dz = __ffma2_rn(z, sc2, q[r][2]);
+        const float2 e = ex2_neg_pair(__ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx))));
+        acc[r][0] = __ffma2_rn(e, e, acc[r][0]);
+        acc[r][1] = __fadd2_rn(acc[r][1], e);
+        acc[r][2] = __ffma2_rn(e, x, acc[r][2]);
+        acc[r][3] = __ffma2_rn(e, y, acc[r][3]);
+        acc[r][4] = __ffma2_rn(e, z, acc[r][4]);
+      }
+    }
+    // the warp's sums: lanes 8 r .. 8 r + 7 end with row r's
+    float v[4][5], w[2][5], u[5];
+    const bool up = (lane & 16) != 0, od = (lane & 8) != 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int a = 0; a < 5; ++a) v[r][a] = acc[r][a].x + acc[r][a].y;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int a = 0; a < 5; ++a) {
+        const float give = up ? v[r][a] : v[r + 2][a], keep = up ? v[r + 2][a] : v[r][a];
+        w[r][a] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+      }
+#pragma unroll
+    for (int a = 0; a < 5; ++a) {
+      const float give = od ? w[0][a] : w[1][a], keep = od ? w[1][a] : w[0][a];
+      u[a] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+      for (int a = 0; a < 5; ++a) u[a] += __shfl_xor_sync(0xffffffffu, u[a], off);
+    if ((lane & 7) == 0)
+#pragma unroll
+      for (int a = 0; a < 5; ++a) rs.part[p][warp][lane >> 3][a] = u[a];
+  }
+}
+
+// The rows completed (by warp 0, after a block barrier) and their 16 moments,
+// added in row order by halves, stored as this block's record.
+__device__ __forceinline__ void rows_finish(const EmicpArgs& A, RowsSmem& rs, int r0, int nrows, float outlier,
+                                            const float* hdr, float* row_tape, df* rec) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x >= 32) return;
+  df v[kEmNV];
+#pragma unroll
+  for (int k = 0; k < kEmNV; ++k) v[k] = df_make(0.f);
+  if (lane < nrows) {
+    float tot[5];
+#pragma unroll
+    for (int a = 0; a < 5; ++a) {
+      float t = rs.part[lane >> 2][0][lane & 3][a];
+#pragma unroll
+      for (int w = 1; w < kWarps; ++w) t += rs.part[lane >> 2][w][lane & 3][a];
+      tot[a] = t;
+    }
+    const float xm[3] = {hdr[6], hdr[7], hdr[8]}, oX[3] = {hdr[0], hdr[1], hdr[2]};
+    const float4 y = rs.y[lane];
+    emicp_row_finish(r0 + lane, __float_as_int(y.w), tot, y, outlier, xm, A.row_out, oX, row_tape, v);
+#pragma unroll
+    for (int k = 0; k < kEmNV; ++k) rs.mom[k][lane] = v[k];
+  }
+  __syncwarp();
+  const int k = lane & 15;
+  df s = df_make(0.f);
+  for (int i = lane >> 4; i < nrows; i += 2) df_add(s, rs.mom[k][i]);
+  const df o = df_shfl_down(s, 16);
+  df_add(s, o);
+  if (lane < 16) __stcg(reinterpret_cast<float2*>(rec + k), make_float2(s.hi, s.lo));
+}
+
 // A block's part in emicp_teams_kernel: jobs [first, first + njobs), block
 // `rank` of the `size` blocks that run them.
 struct TeamBlock {
@@ -296,9 +427,13 @@ struct TeamBlock {
 
 // One registration by blocks 0 .. G - 1, this one block bid; false after a
 // failure (status set). kTeam: one of several in the launch (local sweeps, no
-// tape); the caller has initialised the stage barriers and the pipe.
-template <bool kTeam>
-__device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pipe& pipe, const int& bid, const int& G) {
+// tape); the caller has initialised the stage barriers and the pipe. kRows:
+// small clouds, whole rows to a block (sm and pipe unused).
+constexpr int kPlain = 0, kTeams = 1, kSmall = 2;
+template <int kMode>
+__device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pipe& pipe, const int& bid, const int& G,
+                                          RowsSmem* rs = nullptr, float* xs = nullptr) {
+  constexpr bool kTeam = kMode == kTeams, kRows = kMode == kSmall;
   __shared__ float s_pose[12];
   __shared__ df s_red[kThreads];
   __shared__ OwnCache oc_rows;
@@ -313,7 +448,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
   const int tid = threadIdx.x;
 
   if (tid == 0) {
-    if (!kTeam) {
+    if (kMode == kPlain) {
       for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
       mbar_init_fence();
     }
@@ -328,14 +463,14 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     pose_to_centred(R, t, &s_hdr[0], &s_hdr[3], tc);
     for (int k = 0; k < 9; ++k) s_pose[k] = R[k];
     for (int k = 0; k < 3; ++k) s_pose[9 + k] = tc[k];
-    oc_rows.blk = -1;
+    if (!kRows) oc_rows.blk = -1;
     int vb = bid;  // the virtual block whose share this block sweeps
     s_pair[0] = -1;
     if (kTeam && A.geo.pair_num) {  // ranks 2 d and 2 d + 1 share an SM
       s_pair[0] = bid >> 1;
       s_pair[1] = bid & 1;
       s_pair[2] = 0;
-    } else if (A.geo.pair_num) {
+    } else if (!kRows && A.geo.pair_num) {
       const int2 pr = join_sm_pair(A.pair_tab, A.timeout_ns);
       if (pr.x >= 0 && pr.x < G / 2) {
         s_pair[0] = pr.x;
@@ -346,7 +481,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
         set_status(A.ctl, kStatusInternal, 23);  // the launch ends at its first grid barrier
       }
     }
-    rs_rows = A.geo.pair_num && s_pair[0] < 0 ? RangedShare{0, -1, 0, 0, 0} : ranged_share(A.geo, vb, G);
+    if (!kRows) rs_rows = A.geo.pair_num && s_pair[0] < 0 ? RangedShare{0, -1, 0, 0, 0} : ranged_share(A.geo, vb, G);
   }
   __syncthreads();
 
@@ -356,12 +491,15 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     horn.reset();
     horn_tape.reset();
   }
-  if (!kTeam) pipe_init(pipe);
+  if (kMode == kPlain) pipe_init(pipe);
   unsigned epoch = 0;
   const StreamSrc src{A.cols, nullptr, true};
   float s2 = A.sigma0;
   Timeline tl{kTeam ? nullptr : A.tl, A.tl_cap, 0};
   bool good = true;
+  const int own_rows = kRows ? A.geo.slice_len : 0;  // small clouds: rows of a block
+  const int own_r0 = bid * own_rows, own_n = max(0, min(own_rows, A.M - own_r0));
+  if (kRows) rows_load(A, *rs, xs, own_r0, own_n);
   for (int step = 0; step < A.nsteps; ++step) {
     tl.mark(1);
     const float outlier = expf(-A.d_02 / s2);  // src/emicp.cu:489
@@ -370,12 +508,26 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     for (int k = 0; k < 9; ++k) R[k] = s_pose[k];
 #pragma unroll
     for (int k = 0; k < 3; ++k) tc[k] = s_pose[9 + k];
+    if (kRows) {
+      __syncthreads();  // (the first step: the rows are there)
+      const float scr = sqrtf(kLog2e / (2.f * s2));
+      if (tid < kRowsOwn) {
+        const float4 y = rs->y[tid];
+        rs->nz[tid] = make_float4(-scr * (R[0] * y.x + R[1] * y.y + R[2] * y.z + tc[0]),
+                                  -scr * (R[3] * y.x + R[4] * y.y + R[5] * y.z + tc[1]),
+                                  -scr * (R[6] * y.x + R[7] * y.y + R[8] * y.z + tc[2]), 0.f);
+      }
+    }
     __syncthreads();
 
     // e = exp(-d2 / (2 s2)) = 2^(nk d2). Every unit stores its rows' partial
     // sums over its column slice (deferred: no completion counter).
     const float sc = sqrtf(kLog2e / (2.f * s2));
-    if (kTeam || A.blk) {
+    if (kRows) {
+      rows_sweep(A, *rs, xs, sc, own_n);
+      tl.mark(4);
+      __syncthreads();
+    } else if (kTeam || A.blk) {
       float Rs[9], tcs[3];
 #pragma unroll
       for (int k = 0; k < 9; ++k) Rs[k] = R[k] * sc;
@@ -402,18 +554,20 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
         break;
       }
     }
-    if (!grid_sync(A.ctl, epoch, (unsigned)G, A.timeout_ns, 20)) {
-      good = false;
-      break;
-    }
-    tl.mark(5);
-    if (tid == 0 && s_pair[0] >= 0) {  // SM pairs: the parts change blocks when the times show the other favoured
-      long lo = 0, sp = 0, hi = 0;
-      ranged_tasks(A.geo, 2 * s_pair[0], G, lo, sp);
-      ranged_tasks(A.geo, 2 * s_pair[0] + 1, G, sp, hi);
-      if (pair_swap(lo, sp, hi, A.pair_t, s_pair[0])) {
-        s_pair[2] ^= 1;
-        rs_rows = ranged_share(A.geo, 2 * s_pair[0] + (s_pair[1] ^ s_pair[2]), G);
+    if (!kRows) {
+      if (!grid_sync(A.ctl, epoch, (unsigned)G, A.timeout_ns, 20)) {
+        good = false;
+        break;
+      }
+      tl.mark(5);
+      if (tid == 0 && s_pair[0] >= 0) {  // SM pairs: the parts change blocks when the times show the other favoured
+        long lo = 0, sp = 0, hi = 0;
+        ranged_tasks(A.geo, 2 * s_pair[0], G, lo, sp);
+        ranged_tasks(A.geo, 2 * s_pair[0] + 1, G, sp, hi);
+        if (pair_swap(lo, sp, hi, A.pair_t, s_pair[0])) {
+          s_pair[2] ^= 1;
+          rs_rows = ranged_share(A.geo, 2 * s_pair[0] + (s_pair[1] ^ s_pair[2]), G);
+        }
       }
     }
     // ---- rows completed, each block a contiguous share of them; its 16
@@ -421,7 +575,10 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     // (row, accumulator) pairs t, t + kThreads, ... (loads in flight together),
     // then row threads finish their rows (emicp_row_finish).
     df* rb = A.rbpart + (size_t)(step & 1) * G * kEmNV;
-    {
+    if (kRows) {
+      rows_finish(A, *rs, own_r0, own_n, outlier, s_hdr, A.row_tape ? A.row_tape + (size_t)step * A.M * 5 : nullptr,
+                  rb + (size_t)bid * kEmNV);
+    } else {
       const int S = A.geo.slices;
       const float inv_sc = kTeam || A.blk ? 1.f / sc : 1.f;  // local sweeps: the e x sums are sc times too large
       const int rpc = (A.M + G - 1) / G;
@@ -576,7 +733,14 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
 __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Pipe pipe;
-  emicp_run<false>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x);
+  emicp_run<kPlain>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) emicp_rows_kernel(const EmicpArgs A) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Pipe pipe;
+  emicp_run<kSmall>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x,
+                    reinterpret_cast<RowsSmem*>(smem_raw), reinterpret_cast<float*>(smem_raw + sizeof(RowsSmem)));
 }
 
 // Many registrations in one cooperative launch, each by a team of blocks of
@@ -626,7 +790,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_teams_kernel(const EmicpArg
     if (tid < (int)(sizeof(EmicpArgs) / 4))
       reinterpret_cast<unsigned*>(&s_args)[tid] = reinterpret_cast<const unsigned*>(jobs + s_team.first)[tid];
     __syncthreads();
-    if (!emicp_run<true>(s_args, sm, pipe, s_team.rank, s_team.size)) {
+    if (!emicp_run<kTeams>(s_args, sm, pipe, s_team.rank, s_team.size)) {
       if (tid == 0) set_status(ctl, ld_status(s_args.ctl), 24);
       return;
     }
@@ -899,23 +1063,49 @@ struct EmicpPlan {
   SweepGeom geo;
   size_t smem;
   bool local;  // sorted Y, local sweeps
+  bool rows;   // small clouds: whole rows to a block, X in shared memory
 };
 
 size_t sweep_smem() { return sizeof(SweepSmem); }
 
 constexpr int kEmPairNum = 208;  // SM pairs: the favoured block's share, 13 / 16
 
-// The local sweep (and the sort that it wants) from 2.4e7 affinities a step on:
-// below, a step is mostly latency and the prepare step's barrier per chunk
+// Of the others, the local sweep (and the sort that it wants) is taken from 2.4e7
+// affinities a step on: below, a step is mostly latency and the prepare step's barrier per chunk
 // costs as much as the shorter element gives (4001^2: 1.045 -> 1.043 ms, 3000^2
 // 0.878 -> 0.897, 1007^2 0.576 -> 0.624; 6000 x 5000 1.46 -> 1.41, 12,000^2
 // 4.47 -> 4.01, 17,000^2 8.75 -> 7.75).
 bool emicp_local_pays(int N, int M) { return (double)N * (double)M >= 2.4e7; }
 
+// Rows of a block in the small clouds' form, 0 where it is not taken: X has to
+// fit shared memory beside a second block's, and up to 7e7 affinities a step the
+// barrier that it saves is worth more than the local sweep's shorter element
+// (general or local form -> this, us: 100^2 664 -> 379, 600 x 500 581 -> 410,
+// 1007^2 591 -> 426, 2000^2 734 -> 568, 4001^2 1086 -> 996, 6000 x 5000 1475 ->
+// 1386, 8171 x 6007 1897 -> 1679; 8000 x 9000 2401 -> 2420). A whole number of
+// passes of 4 rows; 8 rather than 4 where that leaves one block to an SM (1007:
+// 448 -> 426).
+int emicp_small_rows(int N, int M, int limit) {
+  if (N > kRowsMaxN || (double)N * (double)M >= 7e7) return 0;
+  int own = (M + 4 * limit - 1) / (4 * limit) * 4;
+  if (own == 4 && M > 2 * limit) own = 8;
+  return own <= kRowsOwn ? own : 0;
+}
+
 EmicpPlan plan_emicp(int N, int M, int device) {
   EmicpPlan P;
   P.smem = sweep_smem();
   const int limit = persistent_grid_limit(device, (const void*)emicp_kernel, P.smem);
+  P.local = P.rows = false;
+  const int own =
+      emicp_small_rows(N, M, persistent_grid_limit(device, (const void*)emicp_rows_kernel, rows_smem(kRowsMaxN)));
+  if (own > 0) {
+    P.rows = true;
+    P.smem = rows_smem(N);
+    P.grid = (M + own - 1) / own;
+    P.geo = SweepGeom{M, N, 0, 0, own, 0, 0, 0, 0, 0};
+    return P;
+  }
   P.local = emicp_local_pays(N, M);
   const SweepGeomH h = plan_sweep(M, N, limit);
   P.geo = SweepGeom{h.n_own, h.n_stream, h.nblk, h.slices, h.slice_len, h.units, 0, 0, 0, 0};
@@ -1046,7 +1236,7 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   A.tl_cap = L.timeline_cap;
   A.timeout_ns = L.timeout_ns;
   void* args[] = {(void*)&A};
-  e = cudaLaunchCooperativeKernel((const void*)emicp_kernel, dim3(P.grid), dim3(kThreads), args,
+  e = cudaLaunchCooperativeKernel(P.rows ? (const void*)emicp_rows_kernel : (const void*)emicp_kernel, dim3(P.grid), dim3(kThreads), args,
                                   P.smem, st);
   return (int)e;
 }
