@@ -27,10 +27,10 @@
 // final sweep and the pose are those of the affinity kernels
 // (src/softassign.cu:494-798), the scalings and the slack as (hi, lo) pairs.
 // What bounds it is latency: an update is a chain of ~8 exchanges and the
-// fixed-order sums before and after each (~15 us up to 4000 points, D <= 4;
+// fixed-order sums before and after each (~14 us up to 4000 points, D <= 4;
 // ~32 us at D = 8), not its arithmetic (2 P FMAs per point and pass). Default
-// schedule, one box, affinity kernels -> this: N = M = 413 20.1 -> 7.2 ms, 2000
-// 12.9 -> 7.8, 20,000 461 -> 14.0; 30 updates from T = 0.1 at 7001 x 6007 4.25
+// schedule, one box, affinity kernels -> this: N = M = 413 20.1 -> 6.6 ms, 2000
+// 12.9 -> 7.4, 20,000 461 -> 13.5; 30 updates from T = 0.1 at 7001 x 6007 4.25
 // -> 1.13.
 #include <vector>
 
@@ -365,6 +365,9 @@ __device__ __forceinline__ void ser_sync(const Ser& S) {
     __syncthreads();
 }
 
+// Threads that share a term's remote stores (each adds its sum itself).
+__host__ __device__ constexpr int push_threads(int P) { return 2 * P <= kSerThreads ? 2 : 1; }
+
 // Moments of one pass over this CTA's points, all CTAs' added in rank order
 // and divided by k!: the polynomial's coefficients in L.m. The constant term is
 // kept apart (returned; its place in L.m is 0) and to more than FP32: its
@@ -381,12 +384,17 @@ __device__ __forceinline__ df pass_moments(Ser& S, int n, int ntot, int which, c
   __syncthreads();
   float* slots = at(kLSlot) + S.par * kSerMaxCS * kSerPs;
   S.par ^= 1u;
-  if (t < P) {  // into this CTA's slot of every CTA
-    const float s = sum16(ws + t, kSerPf);
-    const float* dst = slots + S.rank * kSerPs + t;
-#pragma unroll
-    for (int r = 0; r < kSerMaxCS; ++r)
-      if (r < S.CS) st_dsmem(dst, (unsigned)r, s);
+  // into this CTA's slot of every CTA: kPush threads to a term, each for every
+  // kPush-th CTA, as a loop: unrolled over 16 CTAs the stores were mostly code to
+  // fetch (100 points 6.37 -> 5.45 ms, 413 7.09 -> 6.52, 2000 7.83 -> 7.40, 20,000
+  // 14.1 -> 13.7; with 16 or 4 threads to a term 20,000 took 14.4 and 13.8)
+  constexpr int kPush = push_threads(P);
+  if (t < P * kPush) {
+    const int k = t / kPush;
+    const float s = sum16(ws + k, kSerPf);
+    const float* dst = slots + S.rank * kSerPs + k;
+#pragma unroll 1
+    for (int r = t % kPush; r < S.CS; r += kPush) st_dsmem(dst, (unsigned)r, s);
   }
   ser_sync(S);
   float* m = at(kLM);
@@ -697,11 +705,11 @@ __device__ __noinline__ void series_update(Ser& Sg, df wsc, int I1, float lam, f
   }
   __syncthreads();
   float* slotD = at(kLSlotD);
-  if (tid < 32) {
-    const df s = sum16d(wd + 2 * tid);
-#pragma unroll
-    for (int r = 0; r < kSerMaxCS; ++r)
-      if (r < S.CS) st_dsmem2(slotD + (S.rank * 32 + tid) * 2, (unsigned)r, s.hi, s.lo);
+  if (tid < 32 * 4) {
+    const int k = tid & 31;
+    const df s = sum16d(wd + 2 * k);
+#pragma unroll 1
+    for (int r = tid >> 5; r < S.CS; r += 4) st_dsmem2(slotD + (S.rank * 32 + k) * 2, (unsigned)r, s.hi, s.lo);
   }
   ser_sync(S);
   if (tid < 32) reinterpret_cast<df*>(at(kLTot))[tid] = sum16d(slotD + 2 * tid);
