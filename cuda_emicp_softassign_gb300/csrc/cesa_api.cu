@@ -819,7 +819,7 @@ int cesa_emicp_backward_device(int N, int M, const cesa_params* p, const void* t
   cudaStream_t st = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lock(g_mu);
   StreamCtx& C = ctx_for(dev, st);
-  cudaError_t e = C.ws.ensure(emicp_adjoint_ws_need(N, M, dev, p->emicp_backward_layout));
+  cudaError_t e = C.ws.ensure(emicp_adjoint_ws_need(N, M, nsteps, dev, p->emicp_backward_layout));
   if (e != cudaSuccess) return map_cuda(e);
   const TapeLayout T = tape_layout(N, M, nsteps);
   const char* tb = static_cast<const char*>(tape);

@@ -8,7 +8,9 @@
 //      eigenvector of Horn's N (sum over the other eigenvectors of
 //      (v_j . gq) / (l_0 - l_j) v_j q^T), of N(S) and of the moment algebra,
 //      giving dL/d(L, U, P, Q) for L = sum lambda, U = sum u, P = sum lambda y,
-//      Q = sum u y^T;
+//      Q = sum u y^T. It is linear in dL/d(R, t') and otherwise the tape's: a
+//      kernel before the walk forms every step's 16 x 12 matrix (all steps at
+//      once), and the walk multiplies by it;
 //   2. one sweep that recomputes the affinities e_rc = exp(-|x_c - z_r|^2 / 2 s2)
 //      (z_r = R y_r + t) over (column block, row slice) units. A lane owns 6
 //      X columns; Y rows stream through shared memory as records of packed
@@ -49,7 +51,9 @@
 namespace cesa {
 namespace {
 
-constexpr int kAdjCols = 6;                       // owned X columns per lane
+// Owned X columns per lane: 6, or 2 for clouds whose units of 6 would leave most
+// blocks without one (plan_adj).
+constexpr int kAdjCols = 6, kAdjColsSmall = 2;
 constexpr int kAdjColBlk = kThreads * kAdjCols;   // owned columns per unit
 constexpr int kAdjRows = kThreads;                // streamed Y rows per chunk (one record per thread)
 constexpr int kAdjRP = kAdjRows / 2;              // row pairs per chunk
@@ -97,7 +101,7 @@ struct EmAdjArgs {
   int M, N;
   AdjGeom geo;
   int nsteps;
-  const float* tape;      // [nsteps][kEmTape]
+  const float* steps;     // [nsteps][kAdjStep]: the step's map, then its input pose and sigma_p2
   const float* row_tape;  // [nsteps][M][5]
   const float* g_out;     // dL/d(R, t) of the final pose (device, caller frame)
   const CenterHdr* hdr;   // centring offsets (t' = t + R oY - oX)
@@ -146,6 +150,28 @@ __device__ void em_step_adjoint(const float* rec, const float (&gRo)[9], const f
     gL -= (gXc[i] * Xc[i] + gYc[i] * Yc[i]) / L;
   }
   coef[0] = gL;
+}
+
+// Every step's adjoint as a matrix (coefficient i, entry j of dL/d(R', t')), one
+// thread per column, with the step's pose and sigma_p2. By one thread of the
+// walk the chain took 3 us of each step (N = M = 100, 66 steps: backward 1.66 ->
+// 1.47 ms; 10,007 x 9001 6.42 -> 6.32).
+constexpr int kAdjMap = 16 * 12, kAdjStep = kAdjMap + 16;
+static_assert(kAdjMap + 13 <= kThreads, "a step's record is loaded by one thread a value");
+
+__global__ void adjoint_map_kernel(const float* __restrict__ tape, float* __restrict__ steps) {
+  const float* rec = tape + (size_t)blockIdx.x * kEmTape;
+  float* out = steps + (size_t)blockIdx.x * kAdjStep;
+  const int j = threadIdx.x;
+  if (j < 12) {
+    float gR[9], gt[3], coef[16];
+    for (int i = 0; i < 9; ++i) gR[i] = i == j ? 1.f : 0.f;
+    for (int i = 0; i < 3; ++i) gt[i] = 9 + i == j ? 1.f : 0.f;
+    em_step_adjoint(rec, gR, gt, coef);
+    for (int i = 0; i < 16; ++i) out[i * 12 + j] = coef[i];
+  } else if (j < 25) {
+    out[kAdjMap + j - 12] = rec[j - 12];
+  }
 }
 
 // Per row: z (posed), and the row-sum adjoints gA, gB[3], gC (zero for
@@ -255,10 +281,13 @@ __device__ __forceinline__ void complete_chunk_rows(const AdjSmem& sm, int buf, 
   __stcg(A.part_z + (size_t)cb * A.M + r, make_float4(gz[0], gz[1], gz[2], 0.f));
 }
 
+template <int kCols>
 __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjArgs A) {
+  constexpr int kColBlk = kThreads * kCols;  // owned columns per unit
   extern __shared__ __align__(128) unsigned char smem_raw[];
   AdjSmem& sm = *reinterpret_cast<AdjSmem*>(smem_raw);
   __shared__ float s_g[12];     // dL/d(R, t') of the current step's output pose
+  __shared__ float s_step[kAdjMap + 13];  // the step's map, pose and sigma_p2
   __shared__ float s_coef[16];  // moment adjoints of the current step
   __shared__ float s_pose[13];  // the step's input pose and sigma_p2
   __shared__ df s_red[kThreads];
@@ -292,16 +321,16 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
   __syncthreads();
   unsigned epoch = 0;
   bool ok = true;
+  if (tid < kAdjMap + 13) s_step[tid] = __ldcg(A.steps + (size_t)(A.nsteps - 1) * kAdjStep + tid);
+  __syncthreads();
   for (int k = A.nsteps - 1; k >= 0 && ok; --k) {
     const int par = k & 1;
-    const float* rec = A.tape + (size_t)k * kEmTape;
-    if (tid == 0) {
-      float gRo[9], gto[3], coef[16];
-      for (int i = 0; i < 9; ++i) gRo[i] = s_g[i];
-      for (int i = 0; i < 3; ++i) gto[i] = s_g[9 + i];
-      em_step_adjoint(rec, gRo, gto, coef);
-      for (int i = 0; i < 16; ++i) s_coef[i] = coef[i];
-      for (int i = 0; i < 13; ++i) s_pose[i] = rec[i];
+    if (tid < 16) {
+      df c = df_make(0.f);
+      for (int j = 0; j < 12; ++j) df_add_prod(c, s_step[tid * 12 + j], s_g[j]);
+      s_coef[tid] = df_val(c);
+    } else if (tid >= 32 && tid < 45) {
+      s_pose[tid - 32] = s_step[kAdjMap + tid - 32];
     }
     __syncthreads();
     // the step's pose and coefficients stay in shared memory (read per row record)
@@ -313,7 +342,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
     const float sc = sqrtf(kLog2e / (2.f * s2)), inv_sc = 1.f / sc;  // coordinate scale
     const float* rtape = A.row_tape + (size_t)k * A.M * 5;
     df* recs = A.rec + (size_t)par * G * 16;
-    const size_t px_len = g.ranged ? (size_t)g.nb * g.kmax * kAdjColBlk : (size_t)g.S * A.N;
+    const size_t px_len = g.ranged ? (size_t)g.nb * g.kmax * kColBlk : (size_t)g.S * A.N;
     float4* px = A.part_x + (size_t)par * px_len;
 
     int u_begin = (int)blockIdx.x, u_end = g.units, u_step = (int)G;
@@ -345,20 +374,20 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
         const int j = u == 0 ? rsh.j_first : 0;
         // the slot must exist: an inconsistent plan records an error and
         // stores nothing (px_dst = nullptr) rather than writing past the array
-        px_dst = j < g.kmax && cb < g.nb ? px + ((size_t)cb * g.kmax + j) * kAdjColBlk : nullptr;
+        px_dst = j < g.kmax && cb < g.nb ? px + ((size_t)cb * g.kmax + j) * kColBlk : nullptr;
         if (!px_dst && tid == 0) set_status(A.ctl, kStatusInternal, 104);
       } else {
         const int sl = u / g.nb;
         cb = u - sl * g.nb;
         rb = sl * g.len;
         re = min(rb + g.len, A.M);
-        px_dst = px + (size_t)sl * A.N + (size_t)cb * kAdjColBlk;
+        px_dst = px + (size_t)sl * A.N + (size_t)cb * kColBlk;
       }
       // owned columns, duplicated into both halves of a packed pair
-      float2 xd[kAdjCols][3], gx[kAdjCols][3];
+      float2 xd[kCols][3], gx[kCols][3];
 #pragma unroll
-      for (int j = 0; j < kAdjCols; ++j) {
-        const int c = cb * kAdjColBlk + j * kThreads + tid;
+      for (int j = 0; j < kCols; ++j) {
+        const int c = cb * kColBlk + j * kThreads + tid;
         const float4 x = c < A.N ? ld_cg(A.cols + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         xd[j][0] = dup2(c < A.N ? x.x * sc : kPadScaled);
         xd[j][1] = dup2(c < A.N ? x.y * sc : kPadScaled);
@@ -431,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
             const float2 gB2 = make_float2(a5.x, a5.y);
             float2 gz0 = gz[g2][0], gz1 = gz[g2][1], gz2 = gz[g2][2];  // sum of e gB - w (x - z)
 #pragma unroll
-            for (int j = 0; j < kAdjCols; ++j) {
+            for (int j = 0; j < kCols; ++j) {
               const float2 dx = __fadd2_rn(xd[j][0], nz0);
               const float2 dy = __fadd2_rn(xd[j][1], nz1);
               const float2 dz = __fadd2_rn(xd[j][2], nz2);
@@ -482,8 +511,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
       }
       // this unit's dL/dx of the owned columns
 #pragma unroll
-      for (int j = 0; j < kAdjCols; ++j) {
-        const int c = cb * kAdjColBlk + j * kThreads + tid;
+      for (int j = 0; j < kCols; ++j) {
+        const int c = cb * kColBlk + j * kThreads + tid;
         if (c < A.N && px_dst)
           __stcg(px_dst + j * kThreads + tid,
                  make_float4((gx[j][0].x + gx[j][0].y) * inv_sc, (gx[j][1].x + gx[j][1].y) * inv_sc,
@@ -512,6 +541,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
         if (g.pair_num) rsh = ranged_share(adj_tasks(g), 2 * s_pair[0] + (s_pair[1] ^ s_pair[2]), (int)G);
       }
     }
+    // (the next step's record is on its way while the rows complete)
+    const float next = k > 0 && tid < kAdjMap + 13 ? __ldcg(A.steps + (size_t)(k - 1) * kAdjStep + tid) : 0.f;
     // Rows completed, each block a contiguous share of them (all blocks in
     // parallel, no serial tail): the column blocks' dL/dz partials summed in
     // column-block order, dL/dy = R^T dL/dz + lambda_r gP + gQ^T u_r, and the
@@ -578,6 +609,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
       em_block_moments(vv, min(kThreads, nrows), reinterpret_cast<df*>(&sm.wsum[0][0][0][0]),
                        recs + (size_t)blockIdx.x * 16);
     }
+    if (tid < kAdjMap + 13) s_step[tid] = next;
     if (!grid_sync(A.ctl, epoch, G, A.timeout_ns, 103)) {
       ok = false;
       break;
@@ -592,9 +624,9 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_adjoint_kernel(const EmAdjA
     // kmax slot) partials in order
     for (int c = blockIdx.x * kThreads + tid; c < A.N; c += G * kThreads) {
       float sx = gxb[0], sy = gxb[1], sz = gxb[2];
-      const int cbk = c / kAdjColBlk;
-      const float4* src = g.ranged ? px + (size_t)cbk * g.kmax * kAdjColBlk + (c - cbk * kAdjColBlk) : px + c;
-      const size_t stride = g.ranged ? (size_t)kAdjColBlk : (size_t)A.N;
+      const int cbk = c / kColBlk;
+      const float4* src = g.ranged ? px + (size_t)cbk * g.kmax * kColBlk + (c - cbk * kColBlk) : px + c;
+      const size_t stride = g.ranged ? (size_t)kColBlk : (size_t)A.N;
       const int np = g.ranged ? g.kmax : g.S;
       int b = 0;
       for (; b + 16 <= np; b += 16) {  // 16 loads in flight, summed in order
@@ -673,17 +705,15 @@ struct AdjPlan {
   AdjGeom geo;
   size_t smem;
   int pairs;  // slice units dealt to SM pairs
+  int cols;   // owned columns per lane
 };
 
-// Column blocks of kAdjColBlk columns and row slices of an even number of rows,
-// as many slices as fill whole waves of the co-resident grid best (up to 4 waves;
-// at least 64 rows per slice).
-AdjPlan plan_adj(int N, int M, int device, int layout) {
-  AdjPlan P;
-  P.smem = sizeof(AdjSmem);
-  const int limit = persistent_grid_limit(device, (const void*)emicp_adjoint_kernel, P.smem);
-  AdjGeom g;
-  g.nb = (N + kAdjColBlk - 1) / kAdjColBlk;
+// Column blocks of kThreads * cols columns and row slices of an even number of
+// rows, as many slices as fill whole waves of the co-resident grid best (up to 4
+// waves; at least 64 rows per slice).
+AdjGeom adj_slices(int N, int M, int limit, int cols) {
+  AdjGeom g{};
+  g.nb = (N + kThreads * cols - 1) / (kThreads * cols);
   const int max_s = (M + 63) / 64;  // at least 64 rows per slice
   int bestS = 1;
   double best = -1.0;
@@ -706,6 +736,35 @@ AdjPlan plan_adj(int N, int M, int device, int layout) {
   g.len += g.len & 1;
   g.S = (M + g.len - 1) / g.len;
   g.units = g.nb * g.S;
+  return g;
+}
+
+const void* adj_kernel(int cols) {
+  return cols == kAdjCols ? (const void*)emicp_adjoint_kernel<kAdjCols>
+                          : (const void*)emicp_adjoint_kernel<kAdjColsSmall>;
+}
+
+AdjPlan plan_adj(int N, int M, int device, int layout) {
+  AdjPlan P;
+  P.smem = sizeof(AdjSmem);
+  const int limit = persistent_grid_limit(device, adj_kernel(kAdjCols), P.smem);
+  P.cols = kAdjCols;
+  AdjGeom g = adj_slices(N, M, limit, P.cols);
+  // 2 columns a lane where their units, of a third of the elements (each taking
+  // up to 1.6 times as long: a row's record and sums are shared by fewer
+  // columns), end sooner: backward at 100^2 1.52 -> 1.04 ms, 1007^2 1.59 -> 1.09 (16
+  // units of 304 before), 4000^2 2.53 -> 2.12; 3000^2 1.72 either way, 5000 x 4000
+  // 2.49 with 6 and 2.59 with 2
+  if (layout != CESA_LAYOUT_RANGED) {
+    const int limit2 = persistent_grid_limit(device, adj_kernel(kAdjColsSmall), P.smem);
+    const AdjGeom h = adj_slices(N, M, limit2, kAdjColsSmall);
+    const double t6 = (double)((g.units + limit - 1) / limit) * g.len * kAdjCols;
+    const double t2 = (double)((h.units + limit2 - 1) / limit2) * h.len * kAdjColsSmall * 1.6;
+    if (t2 < t6 && limit2 == limit) {
+      P.cols = kAdjColsSmall;
+      g = h;
+    }
+  }
   g.ranged = 0;
   g.nch = (M + kAdjRows - 1) / kAdjRows;
   g.kmax = 0;
@@ -726,9 +785,9 @@ AdjPlan plan_adj(int N, int M, int device, int layout) {
   const long per = (T + limit - 1) / limit;
   const int waves = (g.units + limit - 1) / limit;
   const bool ranged =
-      layout == CESA_LAYOUT_RANGED ||
+      P.cols == kAdjCols && (layout == CESA_LAYOUT_RANGED ||
       (layout == CESA_LAYOUT_AUTO && T >= 8L * limit &&
-       (two_per_sm || (double)per < (double)waves * g.len / kAdjRows));
+       (two_per_sm || (double)per < (double)waves * g.len / kAdjRows)));
   if (ranged) {
     P.geo.ranged = 1;
     P.geo.pair_num = two_per_sm ? kAdjRangedPairNum : 0;
@@ -748,7 +807,7 @@ size_t part_x_len(const AdjGeom& g, int N) {
 
 // Workspace of the adjoint: control block and counters (cleared), gradient
 // accumulators gX, gY (cleared), split partials, records and column partials.
-size_t emicp_adjoint_ws_need(int N, int M, int device, int layout) {
+size_t emicp_adjoint_ws_need(int N, int M, int nsteps, int device, int layout) {
   const AdjPlan P = plan_adj(N, M, device, layout);
   Carve c(nullptr);
   c.take<Ctl>(1);
@@ -760,6 +819,7 @@ size_t emicp_adjoint_ws_need(int N, int M, int device, int layout) {
   c.take<float4>((size_t)P.geo.nb * M);
   c.take<df>((size_t)2 * P.grid * 16);
   c.take<float4>(part_x_len(P.geo, N));
+  c.take<float>((size_t)nsteps * kAdjStep);
   return c.off;
 }
 
@@ -779,6 +839,7 @@ int enqueue_emicp_adjoint(const EmicpAdjointLaunch& L, void* ws, size_t ws_bytes
   float4* part_z = c.take<float4>((size_t)P.geo.nb * L.M);
   df* rec = c.take<df>((size_t)2 * P.grid * 16);
   float4* part_x = c.take<float4>(part_x_len(P.geo, L.N));
+  float* steps = c.take<float>((size_t)L.nsteps * kAdjStep);
   if (c.off > ws_bytes) return (int)cudaErrorInvalidValue;
   e = cudaMemsetAsync(ws, 0, zero_bytes, st);
   // ranged dL/dx slots that no block writes must read as zero
@@ -791,7 +852,7 @@ int enqueue_emicp_adjoint(const EmicpAdjointLaunch& L, void* ws, size_t ws_bytes
   A.N = L.N;
   A.geo = P.geo;
   A.nsteps = L.nsteps;
-  A.tape = L.tape;
+  A.steps = steps;
   A.row_tape = L.row_tape;
   A.g_out = L.g_out;
   A.hdr = L.hdr;
@@ -808,8 +869,11 @@ int enqueue_emicp_adjoint(const EmicpAdjointLaunch& L, void* ws, size_t ws_bytes
   A.d_status = L.d_status;
   A.timeout_ns = L.timeout_ns;
   if (L.nsteps > 0) {
+    adjoint_map_kernel<<<L.nsteps, 32, 0, st>>>(L.tape, steps);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
     void* args[] = {(void*)&A};
-    e = cudaLaunchCooperativeKernel((const void*)emicp_adjoint_kernel, dim3(P.grid), dim3(kThreads), args, P.smem,
+    e = cudaLaunchCooperativeKernel(adj_kernel(P.cols), dim3(P.grid), dim3(kThreads), args, P.smem,
                                     st);
     if (e != cudaSuccess) return (int)e;
   } else {
