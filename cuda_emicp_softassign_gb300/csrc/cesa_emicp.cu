@@ -86,10 +86,14 @@ struct EmicpArgs {
 // splits), records stored as packed duplicates (35.4), kLocalR2 = 16 (32.1).
 constexpr float kLocalR2 = 48.f;
 
-// Poses of the local form are refined in the last steps, where sigma is small
-// and their errors reach the result (the ones of earlier steps are contracted
-// away): the short form's rounding is then more than made up for. ~2 us a step.
-constexpr int kRefineSteps = 16;
+// The poses of the local form are refined (horn_refine_dd), and those of the last
+// steps on small clouds: the short form's rounding is then more than made up for,
+// and gradients, which see the poses' noise most, come out closer to FP64 than with
+// FP32 solves. At 10,007 x 9001 and 7000 x 7500, 16 pairs, gradients are 0.9e-6 -
+// 2.6e-6 off with all 66 steps refined, 0.8e-6 - 4.6e-6 with the last 30, 0.9e-6 -
+// 5.7e-6 with 16, 2.1e-6 - 1.1e-5 with none and direct differences. ~2 us a
+// step, a third of a small clouds' step: they take the second half only.
+constexpr int kSmallRefine = 32;
 
 struct EmicpElemLocal {  // q = 2 z~ of two owned points; s = (x~, -|x~|^2)
   __device__ __forceinline__ void operator()(float2 (&acc)[5], const float2 (&q)[3], float4 s) const {
@@ -299,7 +303,8 @@ __device__ __forceinline__ bool em_local_sweep(const int& bid, const int& G, Swe
 // 256th pair of columns against 4 rows at a time: direct differences, 11
 // FP32 ops per element (the scale rides on the difference's FFMA). Bound by that
 // chain (about 5.7 us a step) up to 2000 points, by the FP32 pipe from 5000 on:
-// N = M = 1007 591 -> 426 us, 8171 x 6007 1897 -> 1679 (device call).
+// N = M = 1007 591 -> 493 us, 8171 x 6007 1897 -> 1739 (device call, poses of the
+// second half refined).
 constexpr int kRowsOwn = 32;                // most rows of a block
 constexpr int kRowsMaxN = 8192;             // X in shared memory, two blocks to an SM
 constexpr int kRowsPad = 2 * kThreads;      // columns are padded to this
@@ -652,7 +657,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     // ---- grid-wide moments -> pose (every block computes the same pose)
     reduce_block_partials<kEmNV>(rb, G, s_red, s_tot);
     tl.mark(6);
-    const bool refine = (kTeam || A.blk) && step + kRefineSteps >= A.nsteps;
+    const bool refine = kRows ? step + kSmallRefine >= A.nsteps : kTeam || A.blk;
     em_moments_to_S_block(s_tot, s_emS, refine);
     if (tid == 0) {
       float Xc[3], Yc[3], S[9];
@@ -1078,15 +1083,15 @@ constexpr int kEmPairNum = 208;  // SM pairs: the favoured block's share, 13 / 1
 bool emicp_local_pays(int N, int M) { return (double)N * (double)M >= 2.4e7; }
 
 // Rows of a block in the small clouds' form, 0 where it is not taken: X has to
-// fit shared memory beside a second block's, and up to 7e7 affinities a step the
+// fit shared memory beside a second block's, and up to 6e7 affinities a step the
 // barrier that it saves is worth more than the local sweep's shorter element
-// (general or local form -> this, us: 100^2 664 -> 379, 600 x 500 581 -> 410,
-// 1007^2 591 -> 426, 2000^2 734 -> 568, 4001^2 1086 -> 996, 6000 x 5000 1475 ->
-// 1386, 8171 x 6007 1897 -> 1679; 8000 x 9000 2401 -> 2420). A whole number of
-// passes of 4 rows; 8 rather than 4 where that leaves one block to an SM (1007:
-// 448 -> 426).
+// (general or local form -> this, both without refined poses, us: 100^2 664 -> 379, 600 x
+// 500 581 -> 410, 1007^2 591 -> 426, 2000^2 734 -> 568, 4001^2 1086 -> 996, 6000 x 5000
+// 1475 -> 1386, 8171 x 6007 1897 -> 1679; 8000 x 9000 2401 -> 2420; the refinement
+// adds about 60). A whole number of passes of 4 rows; 8 rather than 4 where that
+// leaves one block to an SM (1007: 448 -> 426).
 int emicp_small_rows(int N, int M, int limit) {
-  if (N > kRowsMaxN || (double)N * (double)M >= 7e7) return 0;
+  if (N > kRowsMaxN || (double)N * (double)M >= 6e7) return 0;
   int own = (M + 4 * limit - 1) / (4 * limit) * 4;
   if (own == 4 && M > 2 * limit) own = 8;
   return own <= kRowsOwn ? own : 0;
