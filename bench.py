@@ -218,23 +218,30 @@ def algorithmic_work(kind, N, M, p):
     return e * n * (8.0 * sweeps + 12.0), e * n * (sweeps + 1), e * n * (sweeps + 1)
 
 
-def ranged_sweep(n_own, n_stream, grid):
-    """Whether a sweep owning n_own points and streaming n_stream takes the
-    ranged decomposition (at least 16 (128-point block, 512-point chunk) tasks
-    per block of the persistent grid)."""
-    return -(-n_own // 128) * -(-n_stream // 512) >= 16 * grid
+def emicp_form(N, M):
+    """The form an EM-ICP registration takes (csrc/cesa_emicp.cu): "rows" on
+    small clouds (whole rows to a block, the target in shared memory), "local"
+    (sorted rows, block-centred exponents) from 2.4e7 affinities a step, else
+    "slices". `grid`: the launch's blocks, at most two per SM."""
+    import torch
+    limit = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    own = 4 * -(-M // (4 * limit))
+    if N <= 8192 and N * M < 6e7 and own <= 32:
+        return "rows"
+    return "local" if N * M >= 2.4e7 else "slices"
 
 
 def executed_work(kind, N, M, p, grid):
     """FP32-pipe ops the kernels execute for one registration, where they
-    differ from the algorithmic count: the ranged EM-ICP sweep and the
-    matrix-free Softassign sweeps run on clouds scaled by the exponent's
-    factor (and fold 2^c0 into the streamed weights), so that the scale
-    multiply is gone: EM-ICP 11 per element, Sinkhorn 7, final 11."""
+    differ from the algorithmic count: EM-ICP 8 per element in the local form
+    (where a block's radius allows it, 98% of the default schedule at 40,097
+    points; 11 elsewhere), 11 on small clouds. The matrix-free Softassign sweeps
+    run on clouds scaled by the exponent's factor (and fold 2^c0 into the
+    streamed weights), so that the scale multiply is gone: Sinkhorn 7, final 11."""
     n = pose_updates(kind, p)
     e = float(N) * float(M)
     if kind == "emicp":
-        return (11.0 if ranged_sweep(M, N, grid) else 12.0) * e * n
+        return {"rows": 11.0, "local": 8.0, "slices": 12.0}[emicp_form(N, M)] * e * n
     return e * n * (7.0 * 2 * p.I1 + 11.0)
 
 
@@ -244,12 +251,15 @@ def materialised_bytes(N, M, p):
     return 4.0 * (1 + 2 * p.I1) * float(N) * float(M) * p.JMAX * p.I0
 
 
-def kernels_per_registration(kind, form=None):
-    # prep_center + 2 x prep_pack (+ 2 x fill for the slack vectors) + the persistent kernel;
-    # the banded Softassign kernel initialises the slack itself
-    if kind == "softassign" and form != "banded":
-        return 6
-    return 4
+def kernels_per_registration(kind, form=None, N=0, M=0, auto=True):
+    # prep_center + 2 x prep_pack (+ 2 x fill for the slack vectors) + the persistent kernel, under AUTO
+    # after the series kernel; the banded Softassign kernel initialises the slack itself
+    if kind == "softassign":
+        return (4 if form == "banded" else 6) + (1 if auto else 0)
+    if kind == "emicp":  # the local form sorts the rows and measures their blocks
+        return 6 if emicp_form(N, M) == "local" else 4
+    # ICP's grid search: setup, and 2 x (bin, 2 x scan, scatter)
+    return 13 if N >= 4096 and N * M >= 4e7 else 4
 
 
 def config_of(args, kind, X, Y, p, fixture):
@@ -755,7 +765,8 @@ def run_batch(args, rank, world, local):
             "e2e": {"value": world * npairs / e2e_s, "unit": "registrations/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": 48 * npairs},
             "clocks": clocks,
-            "gpu_launches": 3 * args.steps,
+            # centre, pack, the teams' sort, pack, blocks and kernel, the series (at least one cluster size), the rounds
+            "gpu_launches": 8 * args.steps,
             "wall_s_timed_region": t_wall}
     print(json.dumps(line), flush=True)
 
@@ -974,14 +985,19 @@ def run_ours(args, rank, world, local):
         q.JMAX = 1
         rep = cesa.softassign(X, Y, param=q, trace=True)[3]
         form_used = FORM_NAMES.get(rep.sinkhorn_form, str(rep.sinkhorn_form))
-        if form_used == "matrix_free":
+        if args.sinkhorn_form == "auto":
+            roofline["kernel"] = "softassign_series_kernel"
+            roofline["note"] += (". Under AUTO the updates that a short series represents run in the series form "
+                                 "(O(N + M) per update), so the achieved rate is not a pipe rate; the form "
+                                 "named is the one that takes the schedule up where the series stops")
+        elif form_used == "matrix_free":
             roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp, rep.grid_blocks)
     if kind == "emicp":
         q = copy.copy(p)
         q.sigma_inf = q.sigma_p2 * 0.95  # one sigma step: the plan and grid of this size
         rep = cesa.emicp(X, Y, param=q, trace=True)[3]
         roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp, rep.grid_blocks)
-    if form_used == "banded":
+    if form_used == "banded" and args.sinkhorn_form != "auto":
         roofline["note"] += (". The banded form computes each affinity once per inner iteration and "
                              "keeps the tile in shared memory for the other 2*I1 sweeps, so it executes "
                              "fewer operations than this per-sweep count: per element and pose update 1 ex2 "
@@ -1021,7 +1037,8 @@ def run_ours(args, rank, world, local):
             "e2e": {"value": whole_job_rate(args.steps, world, e2e_s), "unit": "registrations/s",
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 12 * 4},
             "clocks": clocks,
-            "gpu_launches": kernels_per_registration(kind, form_used) * args.steps,
+            "gpu_launches": kernels_per_registration(
+                kind, form_used, N, M, args.sinkhorn_form == "auto") * args.steps,
             "wall_s_timed_region": t_wall}
     if kind == "softassign":
         line["sinkhorn"] = {"form": form_used, "requested": args.sinkhorn_form, "tuner": tuned}

@@ -38,7 +38,9 @@ extern "C" {
 typedef struct CUstream_st* cesa_stream_t;
 
 /* Sinkhorn normalisation forms for Softassign (cesa_params.sinkhorn_form). */
-#define CESA_SINKHORN_AUTO 0         /* per-size choice by the built-in tuner */
+#define CESA_SINKHORN_AUTO 0         /* per-size choice by the built-in tuner, after the series form for
+                                        the updates that a short series represents (high temperatures
+                                        against the clouds' extent; their trace records carry gap -1) */
 #define CESA_SINKHORN_MATRIX_FREE 1  /* scaling vectors, affinities recomputed per sweep */
 #define CESA_SINKHORN_MATERIALISED 2 /* affinity matrix stored once per inner iteration */
 #define CESA_SINKHORN_BANDED 3       /* matrix-free, one thread-block cluster per band of 64 rows
@@ -183,10 +185,11 @@ typedef struct cesa_pair {
 
 /*
  * Batched registration: every pair of `pairs` (uneven sizes, EM-ICP and
- * Softassign mixed) in one persistent launch, replacing one emicp() or
- * softassign() call per pair. The pairs advance in lock step through their own
- * schedules; each step of every pair is split into (pair, tile) units that all
- * blocks of the GPU share. Each pair's result equals a single-pair call of the
+ * Softassign mixed) in a few launches, replacing one emicp() or softassign()
+ * call per pair. The EM-ICP pairs share one launch, each by blocks of its own;
+ * the Softassign pairs run their leading updates in the series form (where
+ * sinkhorn_form is AUTO), a cluster each, and advance in lock step through what
+ * is left of their schedules. Each pair's result equals a single-pair call of the
  * same algorithm up to FP32 rounding of the summation order (the Sinkhorn
  * passes complete in a different place). npairs <= CESA_MAX_BATCH. The device
  * variant enqueues on `stream` and writes the device status to *d_status when
