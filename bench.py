@@ -736,10 +736,21 @@ def run_batch(args, rank, world, local):
                 "ex2_achieved_tops": ex2_ops / mean_s / 1e12,
                 "ex2_peak_tops": ex2_peak / 1e12 if ex2_peak else None,
                 "ops_per_batch": fp32_ops}
-    # Lower bound of the batch's time: the work at the measured FP32 peak, and no pair can finish
-    # faster than its own latency floor (its single-pair launch, which already runs at or near the
-    # peak for large pairs). The batch cannot beat max(total work / peak, longest single pair).
-    work_s = fp32_ops / fp32_peak if fp32_peak else None
+    # What the forms in use cannot do without: 8 ops per EM-ICP affinity (block-centred exponents), and, where
+    # the Softassign pairs' form is AUTO, nothing for them (the series form does O(N + M) an update). No pair can
+    # finish faster than its own single launch on the whole GPU nearly does.
+    need = 0.0
+    for algo, X, Y, p in pairs:
+        if algo == cesa.ALGO_EMICP:
+            need += 8.0 * len(X) * len(Y) * pose_updates("emicp", p)
+    if args.sinkhorn_form != "auto":
+        need = fp32_ops
+    work_s = need / fp32_peak if fp32_peak else None
+    if args.sinkhorn_form == "auto":
+        roofline.update(kernel="emicp_teams_kernel", achieved=need / mean_s / 1e12, ops_needed_per_batch=need,
+                        frac=need / mean_s / fp32_peak if fp32_peak else None,
+                        note="achieved = the EM-ICP pairs' 8 FP32 ops per affinity / the batch's time, which "
+                             "includes the Softassign pairs' series updates (latency-bound)")
     longest = max(per_pair_ms) * 1e-3
     bound_s = max(work_s or 0.0, longest)
     cpu = None
@@ -758,8 +769,8 @@ def run_batch(args, rank, world, local):
             "batch_time_bound": {"ms": bound_s * 1e3, "work_at_fp32_peak_ms": work_s * 1e3 if work_s else None,
                                  "longest_single_pair_ms": longest * 1e3,
                                  "max_speedup_vs_one_pair_per_launch": single_ms * 1e-3 / bound_s,
-                                 "note": "the batch cannot finish before its FP32 work at the measured peak, "
-                                         "nor before its longest pair alone"},
+                                 "note": "the FP32 work that the forms in use need at the measured peak, and the "
+                                         "longest pair alone"},
             "roofline": roofline,
             "cpu_baseline": cpu,
             "e2e": {"value": world * npairs / e2e_s, "unit": "registrations/s", "h2d_bytes_per_step": h2d,
@@ -976,8 +987,7 @@ def run_ours(args, rank, world, local):
                 "ops_per_registration": fp32_ops,
                 "note": "achieved = algorithmic FP32-pipe ops of one registration / event time of its launch "
                         "sequence (prep kernels included); executed_fp32_ops_per_registration, where given, "
-                        "is what the kernels issue on the FP32 pipe (clouds pre-scaled by the exponent's "
-                        "factor, one op fewer per element)"}
+                        "is what the kernels issue on the FP32 pipe"}
     form_used = None
     if kind == "softassign":
         # the form the library resolved for this request (AUTO: tuned or by size), as it reports it
@@ -987,6 +997,7 @@ def run_ours(args, rank, world, local):
         form_used = FORM_NAMES.get(rep.sinkhorn_form, str(rep.sinkhorn_form))
         if args.sinkhorn_form == "auto":
             roofline["kernel"] = "softassign_series_kernel"
+            roofline["frac"] = None
             roofline["note"] += (". Under AUTO the updates that a short series represents run in the series form "
                                  "(O(N + M) per update), so the achieved rate is not a pipe rate; the form "
                                  "named is the one that takes the schedule up where the series stops")
@@ -997,6 +1008,15 @@ def run_ours(args, rank, world, local):
         q.sigma_inf = q.sigma_p2 * 0.95  # one sigma step: the plan and grid of this size
         rep = cesa.emicp(X, Y, param=q, trace=True)[3]
         roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp, rep.grid_blocks)
+        if emicp_form(N, M) == "rows":
+            roofline["kernel"] = "emicp_rows_kernel"
+        done = roofline["executed_fp32_ops_per_registration"] / mean_s
+        roofline["frac_algorithmic_ops"] = roofline["frac"]
+        roofline["achieved"] = done / 1e12
+        roofline["frac"] = done / fp32_peak if fp32_peak else None
+        roofline["note"] = ("achieved = FP32-pipe ops that the kernels execute for one registration (EM-ICP's "
+                            "local form: 8 of the algorithm's 12 per element) / event time of its launch sequence "
+                            "(prep kernels included); frac_algorithmic_ops counts the algorithm's 12")
     if form_used == "banded" and args.sinkhorn_form != "auto":
         roofline["note"] += (". The banded form computes each affinity once per inner iteration and "
                              "keeps the tile in shared memory for the other 2*I1 sweeps, so it executes "

@@ -31,7 +31,7 @@
 // ~32 us at D = 8), not its arithmetic (2 P FMAs per point and pass). Default
 // schedule, one box, affinity kernels -> this: N = M = 413 20.1 -> 6.6 ms, 2000
 // 12.9 -> 7.4, 20,000 461 -> 13.5; 30 updates from T = 0.1 at 7001 x 6007 4.25
-// -> 1.13.
+// -> 1.32.
 #include <vector>
 
 #include "cesa_kernels.h"
