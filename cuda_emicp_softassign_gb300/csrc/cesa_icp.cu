@@ -60,6 +60,7 @@ struct IcpGrid {
   float h, inv_h;
   int dim[3];   // cells per axis
   int ncells;
+  float margin; // what the searches add to a distance in cells, for rounding
 };
 
 // z = R y + t with one fixed rounding (both searches use it, so their squared
@@ -136,14 +137,14 @@ __device__ __forceinline__ bool ring_done(const IcpGrid& g, const RingQuery& q, 
   if (!found) return false;
   float m = 3.0e38f;
   for (int a = 0; a < 3; ++a) m = fminf(m, fminf(q.f[a] - (float)(q.c[a] - r), (float)(q.c[a] + r + 1) - q.f[a]));
-  const float bound = fmaxf(m - 1e-4f, 0.f) * g.h;
+  const float bound = fmaxf(m - g.margin, 0.f) * g.h;
   return bound * bound > best * (1.f + 1e-5f);
 }
 
 // Whether cell i can hold a point nearer than the best distance.
 __device__ __forceinline__ bool cell_may_hold(const IcpGrid& g, const RingQuery& q, int ix, int iy, int iz,
                                               float best) {
-  const float gap = fmaxf(sqrtf(cell_gap2(q.f, ix, iy, iz)) - 1e-4f, 0.f);
+  const float gap = fmaxf(sqrtf(cell_gap2(q.f, ix, iy, iz)) - g.margin, 0.f);
   return gap * gap <= best * (1.f + 1e-5f) * g.inv_h * g.inv_h;
 }
 
@@ -301,7 +302,7 @@ struct BallBox {
 };
 
 __device__ __forceinline__ float ball_radius(const IcpGrid& g, float best) {
-  return fmaf(sqrtf(best * (1.f + 1e-5f)), g.inv_h, 1e-4f);
+  return fmaf(sqrtf(best * (1.f + 1e-5f)), g.inv_h, g.margin);
 }
 
 __device__ __forceinline__ BallBox ball_box(const IcpGrid& g, float zx, float zy, float zz, float best) {
@@ -339,8 +340,11 @@ __device__ __forceinline__ void ball_nearest(const IcpGrid& g, const int* start,
   group_min<W>(best, bi);
 }
 
-// One block: the bounding box of the target and the grid (about one cell per
-// four target points over the bounding box, at most cap cells).
+// One block: the bounding box of the target and the grid over it, about cap
+// cells (at most cap, and at most kIcpAxis on an axis). The grid always covers
+// the box: the searches go by the cells' places, so that a point clamped into a
+// cell from beyond it would not be found.
+constexpr int kIcpAxis = 1024;
 __global__ void __launch_bounds__(1024) k_icp_grid_setup(const float4* X, int N, int cap, IcpGrid* g) {
   __shared__ float s_lo[3][32], s_hi[3][32];
   float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
@@ -384,17 +388,19 @@ __global__ void __launch_bounds__(1024) k_icp_grid_setup(const float4* X, int N,
   int d[3];
   for (int it = 0; it < 64; ++it) {
     long long n = 1;
+    int longest = 0;
     for (int a = 0; a < 3; ++a) {
-      d[a] = (int)fmin(fmax(ceil(E[a] / h), 1.0), 1024.0);
+      d[a] = (int)fmin(fmax(ceil(E[a] / h), 1.0), 1e6);
       n *= d[a];
+      longest = max(longest, d[a]);
     }
-    if (n <= cap) break;
-    h *= 1.1;
+    if (n <= cap && longest < kIcpAxis) break;
+    h *= 1.1;  // (64 turns: a factor of 445; the longest axis wants at most 62, at 2.5e8 cells)
   }
   // the cells cover [lo, lo + d h) with a margin of half a cell below
   for (int a = 0; a < 3; ++a) {
     g->lo[a] = (float)(L[a] - 0.5 * h);
-    d[a] = min(d[a] + 1, 1024);
+    d[a] = min(d[a] + 1, kIcpAxis);
   }
   long long n = (long long)d[0] * d[1] * d[2];
   while (n > cap) {  // the margin cell may not fit: drop it on the largest axis
@@ -406,6 +412,9 @@ __global__ void __launch_bounds__(1024) k_icp_grid_setup(const float4* X, int N,
   g->h = (float)h;
   g->inv_h = (float)(1.0 / h);
   for (int a = 0; a < 3; ++a) g->dim[a] = d[a];
+  // a place in cells is rounded twice (2^-24 each), a point's and the query's,
+  // on three axes: under 4.2e-7 of the longest axis
+  g->margin = 1e-4f + 5e-7f * (float)max(d[0], max(d[1], d[2]));
   g->ncells = (int)n;
 }
 
