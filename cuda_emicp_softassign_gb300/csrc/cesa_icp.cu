@@ -259,7 +259,7 @@ __device__ __forceinline__ bool column_run(const IcpGrid& g, const int* start, c
   const float gx = fmaxf(fmaxf((float)ix - f[0], f[0] - (float)(ix + 1)), 0.f);
   const float gy = fmaxf(fmaxf((float)iy - f[1], f[1] - (float)(iy + 1)), 0.f);
   const float rest = fmaf(-gy, gy, fmaf(-gx, gx, B * B));
-  if (!(rest >= 0.f)) return false;
+  if (rest < 0.f) return false;  // (not a number, from infinite radii: the whole column)
   const float dz = sqrtf(rest) + 1e-5f;
   const float z0 = fmaxf(floorf(f[2] - dz), 0.f), z1 = fminf(floorf(f[2] + dz), (float)(g.dim[2] - 1));
   if (!(z0 <= z1)) return false;
@@ -612,12 +612,15 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
           float best;
           int bi;
           candidate(W8{}, r, z, best, bi);
-          const bool found = best < 1e30f;  // else a coordinate is not finite: no match (phase B takes the first point)
-          const BallBox q = ball_box(g, z[0], z[1], z[2], found ? best : 0.f);
+          // without a candidate, or with an infinite distance, the ball is the
+          // whole grid; a query that is not finite has no match (phase B takes the
+          // first point)
+          const bool finite = isfinite(z[0]) && isfinite(z[1]) && isfinite(z[2]);
+          const BallBox q = ball_box(g, z[0], z[1], z[2], best);
           const bool small = (q.x1 - q.x0 + 1) * (q.y1 - q.y0 + 1) <= kIcpColumns;
-          ball_nearest<8>(g, A.cell_start, A.sorted, q, found && small && j < A.M, z[0], z[1], z[2], best, bi);
+          ball_nearest<8>(g, A.cell_start, A.sorted, q, finite && small && j < A.M, z[0], z[1], z[2], best, bi);
           if ((lane & 7) == 0 && j < A.M) {
-            if (small || !found)
+            if (small || !finite)
               __stcg(A.part + r, make_float2(best, __int_as_float(bi)));
             else
               A.heavy[atomicAdd(A.heavy_n, 1)] = r;

@@ -1,7 +1,8 @@
 """The ICP grid search on targets of uneven extents (csrc/cesa_icp.cu): tubes,
-corridors and lines along every axis. The grid has to cover its target, and
-matches and (bitwise) poses are the exhaustive search's, in the first iteration,
-which starts from a sample of the target, and in later ones, which start from the
+corridors and lines along every axis, and very large coordinates. The grid has to
+cover its target and a search to reach every cell that can hold a match: matches
+and (bitwise) poses are the exhaustive search's, in the first iteration, which
+starts from a sample of the target, and in later ones, which start from the
 previous match."""
 import numpy as np
 import pytest
@@ -45,4 +46,13 @@ def test_collinear_target(cesa, torch_cuda, n, axis):
     X, Y = _box(n, 4000, np.roll((1, 0, 0), axis), seed=n + axis)
     Y += np.float32(0.01)
     (_, na), (_, nb) = _both(cesa, torch_cuda, X, Y, iters=1)
+    assert np.array_equal(na, nb)
+
+
+@pytest.mark.parametrize("scale", [1e-12, 1e15, 1e17, 1e19])
+def test_scales(cesa, torch_cuda, scale):
+    """Squared distances of 1e30 and above count like any other; at 1e19 most
+    overflow (a query whose distances are all infinite takes the first point)."""
+    X, Y = _box(40000, 2000, (1, 1, 0.3), seed=9)
+    (_, na), (_, nb) = _both(cesa, torch_cuda, X * np.float32(scale), Y * np.float32(scale), iters=1)
     assert np.array_equal(na, nb)
