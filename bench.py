@@ -251,7 +251,7 @@ def materialised_bytes(N, M, p):
     return 4.0 * (1 + 2 * p.I1) * float(N) * float(M) * p.JMAX * p.I0
 
 
-def kernels_per_registration(kind, form=None, N=0, M=0, auto=True):
+def kernels_per_registration(kind, p, form=None, N=0, M=0, auto=True):
     # prep_center + 2 x prep_pack (+ 2 x fill for the slack vectors) + the persistent kernel, under AUTO
     # after the series kernel; the banded Softassign kernel initialises the slack itself
     if kind == "softassign":
@@ -259,7 +259,8 @@ def kernels_per_registration(kind, form=None, N=0, M=0, auto=True):
     if kind == "emicp":  # the local form sorts the rows and measures their blocks
         return 6 if emicp_form(N, M) == "local" else 4
     # ICP's grid search: setup, and 2 x (bin, 2 x scan, scatter)
-    return 13 if N >= 4096 and N * M >= 4e7 else 4
+    import cuda_emicp_softassign_gb300 as cesa
+    return 13 if cesa.icp_search_used(N, M, p) == cesa.ICP_SEARCH_GRID else 4
 
 
 def config_of(args, kind, X, Y, p, fixture):
@@ -1058,12 +1059,12 @@ def run_ours(args, rank, world, local):
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 12 * 4},
             "clocks": clocks,
             "gpu_launches": kernels_per_registration(
-                kind, form_used, N, M, args.sinkhorn_form == "auto") * args.steps,
+                kind, p, form_used, N, M, args.sinkhorn_form == "auto") * args.steps,
             "wall_s_timed_region": t_wall}
     if kind == "softassign":
         line["sinkhorn"] = {"form": form_used, "requested": args.sinkhorn_form, "tuner": tuned}
     if kind == "icp":
-        # value is the default search (a uniform grid from 4096 target points on), whose work depends
+        # value is the default search (a uniform grid on large clouds), whose work depends
         # on the data; the FP32 roofline is that of the exhaustive search, timed here on the same pair
         pe = copy.copy(p)
         pe.icp_search = cesa.ICP_SEARCH_EXHAUSTIVE
@@ -1085,7 +1086,7 @@ def run_ours(args, rank, world, local):
         roofline["note"] = ("achieved = 6 FP32-pipe ops per point pair (squared distance; the compare-select "
                             "of (distance, index) runs on the ALU pipe) x N x M x iterations / event time of "
                             "the exhaustive search on the same pair")
-        used = args.icp_search if args.icp_search != "auto" else ("grid" if N >= 4096 else "exhaustive")
+        used = "grid" if cesa.icp_search_used(N, M, p) == cesa.ICP_SEARCH_GRID else "exhaustive"
         line["icp_search"] = {"value_search": used,
                               "ms_per_step": total_ms / args.steps, "exhaustive_ms_per_step": exh_s * 1e3,
                               "note": "both searches are exact and return the same matches"}

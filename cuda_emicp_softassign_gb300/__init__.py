@@ -133,6 +133,8 @@ def lib():
             fn.restype = _i
         L.cesa_icp_device.argtypes = [_p, _i, _p, _i, _p, _p, _p, _p, _p]
         L.cesa_icp_device.restype = _i
+        L.cesa_icp_search_used.argtypes = [_i, _i, _p, _p]
+        L.cesa_icp_search_used.restype = _i
         L.cesa_load_points.argtypes = [ctypes.c_char_p, ctypes.POINTER(ctypes.POINTER(ctypes.c_float)),
                                        ctypes.POINTER(_i)]
         L.cesa_load_points.restype = _i
@@ -325,6 +327,14 @@ def icp_device(dX, dY, dRt, param=None, d_nn=None, d_status=None, stream=None):
                                _dptr(d_status) if d_status is not None else None,
                                ctypes.c_void_p(_stream_handle(stream)))
     _check(rc, "icp_device")
+
+
+def icp_search_used(N, M, param=None):
+    """The search that an ICP call of these sizes takes (ICP_SEARCH_EXHAUSTIVE or _GRID)."""
+    s = ctypes.c_int(0)
+    _check(lib().cesa_icp_search_used(int(N), int(M), ctypes.byref(param or Params.default()), ctypes.byref(s)),
+           "icp_search_used")
+    return s.value
 
 
 def load_points(path):

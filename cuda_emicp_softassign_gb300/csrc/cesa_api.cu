@@ -504,6 +504,14 @@ int cesa_icp(const float* X, int N, const float* Y, int M, float R[9], float t[3
   return run_host(3, X, N, Y, M, R, t, p, rep);
 }
 
+int cesa_icp_search_used(int N, int M, const cesa_params* p, int* search) {
+  if (N < 1 || M < 1 || !search) return CESA_ERR_INVALID_ARGUMENT;
+  const int rc = check_icp_params(p);
+  if (rc) return rc;
+  *search = icp_takes_grid(N, M, p->icp_search) ? CESA_ICP_SEARCH_GRID : CESA_ICP_SEARCH_EXHAUSTIVE;
+  return CESA_OK;
+}
+
 int cesa_icp_device(const float* dX, int N, const float* dY, int M, float* dRt, const cesa_params* p,
                     int* d_nn, int* d_status, cesa_stream_t stream) {
   int rc = check_points(dX, N, dY, M);

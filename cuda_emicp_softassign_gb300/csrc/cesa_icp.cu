@@ -856,6 +856,21 @@ struct Carve {
   }
 };
 
+}  // namespace
+
+// The exhaustive search scans the target for whole units of kIcpRows rows, so it
+// is their number that counts: below 4e7 padded pairs it is the faster one
+// (6000^2 0.58 ms against 0.79, 4096 x 9000 0.58 against 0.72), above it the grid
+// (8000 x 5000 0.86 against 0.69, 40,000 x 30 1.00 against 0.59, 10^6 x 30 8.28
+// against 1.49).
+bool icp_takes_grid(int N, int M, int search) {
+  if (search != CESA_ICP_SEARCH_AUTO) return search == CESA_ICP_SEARCH_GRID;
+  const double padded = (double)N * (double)((M + kIcpRows - 1) / kIcpRows) * (double)kIcpRows;
+  return N >= 4096 && padded >= 4e7;
+}
+
+namespace {
+
 struct IcpPlan {
   int grid, nrb, S, slice_len, units;
   bool use_grid;
@@ -867,20 +882,17 @@ struct IcpPlan {
 IcpPlan plan_icp(int N, int M, int device, int search) {
   IcpPlan P;
   const int limit = persistent_grid_limit(device, (const void*)icp_kernel, 0);
-  P.use_grid = search == CESA_ICP_SEARCH_GRID || 
-               // below ~6500^2 pairs every point is scanned sooner (5000^2: 0.71 ms against 0.82;
-               // 8000^2: 1.00 against 0.90)
-               (search == CESA_ICP_SEARCH_AUTO && N >= 4096 && (double)N * (double)M >= 4e7);
+  P.use_grid = icp_takes_grid(N, M, search);
   // Two cells per target point (scans are points of a surface: ~20 to an
   // occupied cell): N = M = 40,097 1.70 ms, with 1/2, 1, 4 and 8 cells 2.02,
   // 1.76, 2.03, 2.25; 10,007 x 9001 0.88, with 1 and 4 0.94 and 0.92.
   P.cap = std::max(64, (int)std::min(2.0 * N, std::max(4.2e6, N / 4.0)));
-  if (P.use_grid) {  // one slice: every row is searched whole by one thread
+  if (P.use_grid) {  // one slice: every row is searched whole, by 8 lanes or a warp
     P.nrb = (M + kIcpRows - 1) / kIcpRows;
     P.S = 1;
     P.slice_len = N;
     P.units = 0;
-    P.grid = limit;  // rows are dealt in warp-sized chunks over all co-resident blocks
+    P.grid = limit;  // rows are dealt to the warps of all co-resident blocks
     return P;
   }
   P.nrb = (M + kIcpRows - 1) / kIcpRows;

@@ -280,6 +280,8 @@ struct IcpLaunch {
   int* d_status;
   uint64_t timeout_ns;
 };
+// Whether a search (CESA_ICP_SEARCH_*) of these sizes goes by the grid.
+bool icp_takes_grid(int N, int M, int search);
 size_t icp_ws_need(int N, int M, int device, int search);
 int enqueue_icp(const IcpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, int* grid_used);
 

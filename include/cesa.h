@@ -94,7 +94,8 @@ typedef struct cesa_params {
 
 /* ICP nearest-neighbour search (cesa_params.icp_search). Both are exact and
  * give the same matches (the first of equal distances in X order). */
-#define CESA_ICP_SEARCH_AUTO 0       /* uniform grid from 4096 target points and N x M = 4e7 on, else exhaustive */
+#define CESA_ICP_SEARCH_AUTO 0       /* uniform grid from 4096 target points and N x M = 4e7 on (M in whole
+                                        1024s), else exhaustive */
 #define CESA_ICP_SEARCH_EXHAUSTIVE 1 /* every target point, tiled through shared memory */
 #define CESA_ICP_SEARCH_GRID 2       /* uniform grid over the target, the cells within reach of a candidate */
 
@@ -241,6 +242,10 @@ int cesa_icp(const float* X, int N, const float* Y, int M, float R[9], float t[3
              cesa_report* report);
 int cesa_icp_device(const float* dX, int N, const float* dY, int M, float* dRt, const cesa_params* p,
                     int* d_nn, int* d_status, cesa_stream_t stream);
+
+/* The search that an ICP call of these sizes takes, in *search:
+ * CESA_ICP_SEARCH_EXHAUSTIVE or CESA_ICP_SEARCH_GRID. */
+int cesa_icp_search_used(int N, int M, const cesa_params* p, int* search);
 
 /*
  * One EM-ICP sigma step (E-step + weighted moments) from pose (R, t): the
