@@ -21,6 +21,14 @@
 #define CAT(a, b) CAT_(a, b)
 #define FN(name) CAT(name, SUFFIX)
 
+/* Sums over the rows of Softassign's matrix are taken in ORACLE_PARTS equal
+ * parts, added in their order: one result per input, whatever the number of
+ * threads and in every run. */
+#undef ORACLE_PARTS
+#undef PART_BEGIN
+#define ORACLE_PARTS 16
+#define PART_BEGIN(p, n) ((int)((long)(n) * (p) / ORACLE_PARTS))
+
 /*
  * EM-ICP, one sigma step: E-step (updateA, row sums + outlier term,
  * normalizeRowsOfA) and the weighted moments (lambda, X', Xc, Yc, S).
@@ -213,6 +221,7 @@ static double FN(softassign_inner)(const float* X, int N, const float* Y, int M,
   const float* Yz = Y + 2 * M;
   const REAL T = (REAL)T_cur;
   const REAL sqT = SQRT(T);
+  REAL* part = (REAL*)malloc(sizeof(REAL) * (size_t)ORACLE_PARTS * (size_t)M);
   /* updateM, src/softassign.cu:106-135: M = exp(-(|x_r - (R y_c + t)|^2 - alpha)/T)/sqrt(T) */
 #pragma omp parallel for schedule(static)
   for (int r = 0; r < N; ++r) {
@@ -238,19 +247,18 @@ static double FN(softassign_inner)(const float* X, int N, const float* Y, int M,
       for (int c = 0; c < M; ++c) row[c] /= sum;
       s[r] /= sum;
     }
-    for (int c = 0; c < M; ++c) cs[c] = 0;
-#pragma omp parallel
-    {
-      REAL* part = (REAL*)calloc((size_t)M, sizeof(REAL));
-#pragma omp for schedule(static)
-      for (int r = 0; r < N; ++r) {
+    for (size_t i = 0; i < (size_t)ORACLE_PARTS * M; ++i) part[i] = 0;
+#pragma omp parallel for schedule(static)
+    for (int p = 0; p < ORACLE_PARTS; ++p) {
+      REAL* pp = part + (size_t)p * M;
+      for (int r = PART_BEGIN(p, N); r < PART_BEGIN(p + 1, N); ++r) {
         const REAL* row = Mtx + (size_t)r * M;
-        for (int c = 0; c < M; ++c) part[c] += row[c];
+        for (int c = 0; c < M; ++c) pp[c] += row[c];
       }
-#pragma omp critical
-      for (int c = 0; c < M; ++c) cs[c] += part[c];
-      free(part);
     }
+    for (int c = 0; c < M; ++c) cs[c] = 0;
+    for (int p = 0; p < ORACLE_PARTS; ++p)
+      for (int c = 0; c < M; ++c) cs[c] += part[(size_t)p * M + c];
     for (int c = 0; c < M; ++c) cs[c] += u[c];
 #pragma omp parallel for schedule(static)
     for (int r = 0; r < N; ++r) {
@@ -293,12 +301,12 @@ static double FN(softassign_inner)(const float* X, int N, const float* Y, int M,
     Yw[3 * c + 2] = cs[c] * Yz[c] - Yc[2];
   }
   /* D = M Yw (N x 3), S = Xw^T D -- src/softassign.cu:761-772 */
-  REAL Sacc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma omp parallel
-  {
-    REAL Sl[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma omp for schedule(static)
-    for (int r = 0; r < N; ++r) {
+  REAL Sp[ORACLE_PARTS][9];
+#pragma omp parallel for schedule(static)
+  for (int p = 0; p < ORACLE_PARTS; ++p) {
+    REAL* Sl = Sp[p];
+    for (int k = 0; k < 9; ++k) Sl[k] = 0;
+    for (int r = PART_BEGIN(p, N); r < PART_BEGIN(p + 1, N); ++r) {
       const REAL* row = Mtx + (size_t)r * M;
       REAL D[3] = {0, 0, 0};
       for (int c = 0; c < M; ++c) {
@@ -310,10 +318,11 @@ static double FN(softassign_inner)(const float* X, int N, const float* Y, int M,
       for (int j = 0; j < 3; ++j)
         for (int i = 0; i < 3; ++i) Sl[i + 3 * j] += xw[i] * D[j];
     }
-#pragma omp critical
-    for (int k = 0; k < 9; ++k) Sacc[k] += Sl[k];
   }
-  for (int k = 0; k < 9; ++k) S[k] = Sacc[k];
+  for (int k = 0; k < 9; ++k) S[k] = 0;
+  for (int p = 0; p < ORACLE_PARTS; ++p)
+    for (int k = 0; k < 9; ++k) S[k] += Sp[p][k];
+  free(part);
   free(Yw);
   return (double)sumM;
 }
