@@ -218,30 +218,29 @@ def algorithmic_work(kind, N, M, p):
     return e * n * (8.0 * sweeps + 12.0), e * n * (sweeps + 1), e * n * (sweeps + 1)
 
 
-def emicp_form(N, M):
-    """The form an EM-ICP registration takes (csrc/cesa_emicp.cu): "rows" on
-    small clouds (whole rows to a block, the target in shared memory), "local"
-    (sorted rows, block-centred exponents) from 2.4e7 affinities a step, else
-    "slices". `grid`: the launch's blocks, at most two per SM."""
-    import torch
-    limit = 2 * torch.cuda.get_device_properties(0).multi_processor_count
-    own = 4 * -(-M // (4 * limit))
-    if N <= 8192 and N * M < 6e7 and own <= 32:
-        return "rows"
-    return "local" if N * M >= 2.4e7 else "slices"
+def emicp_form(N, M, p):
+    """Name of the form an EM-ICP registration takes: "rows" on small clouds, "local"
+    (sorted rows, block-centred exponents), "ranges" or "slices" (direct differences)."""
+    import cuda_emicp_softassign_gb300 as cesa
+    return {cesa.EMICP_FORM_ROWS: "rows", cesa.EMICP_FORM_LOCAL: "local", cesa.EMICP_FORM_RANGES: "ranges",
+            cesa.EMICP_FORM_SLICES: "slices"}[cesa.emicp_form(N, M, p)]
 
 
-def executed_work(kind, N, M, p, grid):
+EMICP_KERNEL = {"rows": "emicp_rows_kernel", "local": "emicp_kernel", "ranges": "emicp_ranges_kernel",
+                "slices": "emicp_kernel"}
+
+
+def executed_work(kind, N, M, p, form=None):
     """FP32-pipe ops the kernels execute for one registration, where they
     differ from the algorithmic count: EM-ICP 8 per element in the local form
     (where a block's radius allows it, 98% of the default schedule at 40,097
-    points; 11 elsewhere), 11 on small clouds. The matrix-free Softassign sweeps
+    points; 11 elsewhere), 11 on small clouds and over task ranges. The matrix-free Softassign sweeps
     run on clouds scaled by the exponent's factor (and fold 2^c0 into the
     streamed weights), so that the scale multiply is gone: Sinkhorn 7, final 11."""
     n = pose_updates(kind, p)
     e = float(N) * float(M)
     if kind == "emicp":
-        return {"rows": 11.0, "local": 8.0, "slices": 12.0}[emicp_form(N, M)] * e * n
+        return {"rows": 11.0, "local": 8.0, "ranges": 11.0, "slices": 12.0}[form] * e * n
     return e * n * (7.0 * 2 * p.I1 + 11.0)
 
 
@@ -257,7 +256,7 @@ def kernels_per_registration(kind, p, form=None, N=0, M=0, auto=True):
     if kind == "softassign":
         return (4 if form == "banded" else 6) + (1 if auto else 0)
     if kind == "emicp":  # the local form sorts the rows and measures their blocks
-        return 6 if emicp_form(N, M) == "local" else 4
+        return 6 if emicp_form(N, M, p) == "local" else 4
     # ICP's grid search: setup, and 2 x (bin, 2 x scan, scatter)
     import cuda_emicp_softassign_gb300 as cesa
     return 13 if cesa.icp_search_used(N, M, p) == cesa.ICP_SEARCH_GRID else 4
@@ -1003,14 +1002,11 @@ def run_ours(args, rank, world, local):
                                  "(O(N + M) per update), so the achieved rate is not a pipe rate; the form "
                                  "named is the one that takes the schedule up where the series stops")
         elif form_used == "matrix_free":
-            roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp, rep.grid_blocks)
+            roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp)
     if kind == "emicp":
-        q = copy.copy(p)
-        q.sigma_inf = q.sigma_p2 * 0.95  # one sigma step: the plan and grid of this size
-        rep = cesa.emicp(X, Y, param=q, trace=True)[3]
-        roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp, rep.grid_blocks)
-        if emicp_form(N, M) == "rows":
-            roofline["kernel"] = "emicp_rows_kernel"
+        form = emicp_form(N, M, p)
+        roofline["executed_fp32_ops_per_registration"] = executed_work(kind, N, M, sp, form)
+        roofline["kernel"] = EMICP_KERNEL[form]
         done = roofline["executed_fp32_ops_per_registration"] / mean_s
         roofline["frac_algorithmic_ops"] = roofline["frac"]
         roofline["achieved"] = done / 1e12

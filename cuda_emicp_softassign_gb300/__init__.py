@@ -37,6 +37,7 @@ SINKHORN_AUTO = 0
 SINKHORN_MATRIX_FREE = 1
 SINKHORN_MATERIALISED = 2
 SINKHORN_BANDED = 3
+EMICP_FORM_ROWS, EMICP_FORM_LOCAL, EMICP_FORM_RANGES, EMICP_FORM_SLICES = 1, 2, 3, 4
 ICP_SEARCH_AUTO = 0
 ICP_SEARCH_EXHAUSTIVE = 1
 ICP_SEARCH_GRID = 2
@@ -133,6 +134,8 @@ def lib():
             fn.restype = _i
         L.cesa_icp_device.argtypes = [_p, _i, _p, _i, _p, _p, _p, _p, _p]
         L.cesa_icp_device.restype = _i
+        L.cesa_emicp_form.argtypes = [_i, _i, _p, _p]
+        L.cesa_emicp_form.restype = _i
         L.cesa_icp_search_used.argtypes = [_i, _i, _p, _p]
         L.cesa_icp_search_used.restype = _i
         L.cesa_load_points.argtypes = [ctypes.c_char_p, ctypes.POINTER(ctypes.POINTER(ctypes.c_float)),
@@ -280,6 +283,14 @@ def emicp(X, Y, R=None, t=None, param=None, trace=False, timeline=0):
 def softassign(X, Y, R=None, t=None, param=None, trace=False, timeline=0):
     """Annealed Softassign on the GPU (replaces softassign(), src/softassign.cu:256-886)."""
     return _host_call("cesa_softassign", X, Y, R, t, param or Params.default(), trace, timeline)
+
+
+def emicp_form(N, M, param=None):
+    """The form (EMICP_FORM_*) that an EM-ICP call of these sizes and this schedule takes here."""
+    f = ctypes.c_int(0)
+    _check(lib().cesa_emicp_form(int(N), int(M), ctypes.byref(param or Params.default()), ctypes.byref(f)),
+           "emicp_form")
+    return f.value
 
 
 def find_rt_from_s(Xc, Yc, S, q_prev=None):

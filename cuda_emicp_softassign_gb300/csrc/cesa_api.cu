@@ -269,7 +269,7 @@ int run_host(int kind, const float* X, int N, const float* Y, int M, float R[9],
   float* dY = reinterpret_cast<float*>(static_cast<char*>(C.io.p) + bx);
   float* dRt = reinterpret_cast<float*>(static_cast<char*>(C.io.p) + bx + by);
   const int form = kind == 2 ? resolve_form(p->sinkhorn_form, N, M, dev) : 0;
-  const size_t need = kind == 1   ? emicp_ws_need(N, M, dev)
+  const size_t need = kind == 1   ? emicp_ws_need(N, M, nsteps, dev)
                       : kind == 2 ? softassign_ws_need(N, M, form, dev)
                                   : icp_ws_need(N, M, dev, p->icp_search);
   e = C.ws.ensure(need);
@@ -542,6 +542,19 @@ int cesa_icp_device(const float* dX, int N, const float* dY, int M, float* dRt, 
   return map_cuda((cudaError_t)enqueue_icp(L, C.ws.p, C.ws.bytes, st, nullptr));
 }
 
+int cesa_emicp_form(int N, int M, const cesa_params* p, int* form) {
+  if (N < 1 || M < 1 || !form) return CESA_ERR_INVALID_ARGUMENT;
+  const int rc = check_emicp_params(p);
+  if (rc) return rc;
+  const long nsteps = emicp_steps(p->sigma_p2, p->sigma_inf, p->sigma_factor);
+  if (nsteps < 0) return CESA_ERR_INVALID_ARGUMENT;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return CESA_ERR_NO_DEVICE;
+  std::lock_guard<std::mutex> lock(g_mu);
+  *form = emicp_form(N, M, nsteps, dev);
+  return CESA_OK;
+}
+
 int cesa_emicp_device(const float* dX, int N, const float* dY, int M, float* dRt,
                       const cesa_params* p, int* d_status, cesa_stream_t stream) {
   int rc = check_points(dX, N, dY, M);
@@ -556,7 +569,7 @@ int cesa_emicp_device(const float* dX, int N, const float* dY, int M, float* dRt
   cudaStream_t st = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lock(g_mu);
   StreamCtx& C = ctx_for(dev, st);
-  cudaError_t e = C.ws.ensure(emicp_ws_need(N, M, dev));
+  cudaError_t e = C.ws.ensure(emicp_ws_need(N, M, nsteps, dev));
   if (e != cudaSuccess) return map_cuda(e);
   EmicpLaunch L{};
   L.dX = dX;
@@ -781,7 +794,7 @@ int cesa_emicp_forward_device(const float* dX, int N, const float* dY, int M, fl
   cudaStream_t st = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lock(g_mu);
   StreamCtx& C = ctx_for(dev, st);
-  cudaError_t e = C.ws.ensure(emicp_ws_need(N, M, dev));
+  cudaError_t e = C.ws.ensure(emicp_ws_need(N, M, nsteps, dev));
   if (e != cudaSuccess) return map_cuda(e);
   const TapeLayout T = tape_layout(N, M, nsteps);
   char* tb = static_cast<char*>(tape);
@@ -806,7 +819,7 @@ int cesa_emicp_forward_device(const float* dX, int N, const float* dY, int M, fl
   // the packed clouds and offsets the forward used
   CenterHdr* hdr = nullptr;
   float4 *rows = nullptr, *cols = nullptr;
-  emicp_ws_views(C.ws.p, N, M, dev, &hdr, &rows, &cols);
+  emicp_ws_views(C.ws.p, N, M, nsteps, dev, &hdr, &rows, &cols);
   e = cudaMemcpyAsync(tb + T.hdr, hdr, sizeof(CenterHdr), cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(tb + T.cols, cols, sizeof(float4) * (size_t)N, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(tb + T.rows, rows, sizeof(float4) * (size_t)M, cudaMemcpyDeviceToDevice, st);
@@ -1164,7 +1177,7 @@ int cesa_emicp_step_device(const float* dX, int N, const float* dY, int M, const
   cudaStream_t st = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lock(g_mu);
   StreamCtx& C = ctx_for(dev, st);
-  cudaError_t e = C.ws.ensure(emicp_ws_need(N, M, dev));
+  cudaError_t e = C.ws.ensure(emicp_ws_need(N, M, 1, dev));
   if (e == cudaSuccess) e = C.io.ensure(256);
   if (e == cudaSuccess) e = C.trace.ensure(sizeof(double) * 32);
   if (e != cudaSuccess) return map_cuda(e);

@@ -19,8 +19,9 @@
 //                   + 1 MUFU per element;
 //   large clouds    the local sweep: Y sorted, every unit about a centre of its
 //                   own, 8 ops + 1 MUFU;
-//   what is left    (few rows against many columns) (row block, column slice)
-//                   units, direct differences and a scale: 12 ops + 1 MUFU.
+//   what is left    (lopsided clouds, single steps) direct differences over (row
+//                   block, column slice) units with a scale, 12 ops + 1 MUFU, or
+//                   over task ranges on scaled copies of X, 11.
 //
 // Coordinates are centred on the device (FP32 offsets oX, oY) before the
 // loop. EM-ICP's S is translation invariant, so only Xc, Yc and t are shifted
@@ -31,6 +32,7 @@
 #include <cstdlib>
 #include <vector>
 
+#include "../../include/cesa.h"
 #include "cesa_kernels.h"
 #include "cesa_ops.cuh"
 #include "cesa_pose.h"
@@ -49,7 +51,9 @@ struct EmicpArgs {
   const CenterHdr* hdr;
   float* dRt;           // PoseIO in/out, caller frame
   float* part;          // row partials [5][S][Mp] (accumulator, column slice, row); ranged: [5][nblk][kmax][kBlockPts]
-  const float4* blk;    // local sweeps: centre and radius of every owned block's rows (null: the plain sweep)
+  const float4* xs;     // direct sweeps over ranges: two copies of X' scaled by a step's sc (step parity)
+  const float4* blk;    // local sweeps: centre and radius of every owned block's rows (NaN: not compact)
+  int refine;           // teams: refine every step's pose
   int Mp;
   df* rbpart;           // [2][grid][kEmNV] moments per block (step parity)
   Ctl* ctl;
@@ -431,10 +435,12 @@ struct TeamBlock {
 };
 
 // One registration by blocks 0 .. G - 1, this one block bid; false after a
-// failure (status set). kTeam: one of several in the launch (local sweeps, no
-// tape); the caller has initialised the stage barriers and the pipe. kRows:
-// small clouds, whole rows to a block (sm and pipe unused).
-constexpr int kPlain = 0, kTeams = 1, kSmall = 2;
+// failure (status set). kPlain: local sweeps (A.blk) or direct differences over
+// slices. kRanges: direct differences over task ranges, in a kernel of its own
+// (beside the local sweeps it made them 1% slower). kTeams: one of several in the
+// launch (local sweeps, no tape); the caller has initialised the stage barriers
+// and the pipe. kSmall: small clouds, whole rows to a block (sm and pipe unused).
+constexpr int kPlain = 0, kTeams = 1, kSmall = 2, kRanges = 3;
 template <int kMode>
 __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pipe& pipe, const int& bid, const int& G,
                                           RowsSmem* rs = nullptr, float* xs = nullptr) {
@@ -453,7 +459,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
   const int tid = threadIdx.x;
 
   if (tid == 0) {
-    if (kMode == kPlain) {
+    if (!kTeam && !kRows) {
       for (int s = 0; s < kStages; ++s) mbar_init(&sm.full[s], 1);
       mbar_init_fence();
     }
@@ -496,17 +502,35 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     horn.reset();
     horn_tape.reset();
   }
-  if (kMode == kPlain) pipe_init(pipe);
+  if (!kTeam && !kRows) pipe_init(pipe);
   unsigned epoch = 0;
   const StreamSrc src{A.cols, nullptr, true};
   float s2 = A.sigma0;
   Timeline tl{kTeam ? nullptr : A.tl, A.tl_cap, 0};
   bool good = true;
+  // Direct sweeps over ranges stream X' scaled by sc (and scale the owned rows alike),
+  // so that an element needs no scale of its own. Each step's copy is written by
+  // all blocks during the previous step's row completion.
+  constexpr bool copies = kMode == kRanges;
+  auto scale_x = [&](int par, float f) {
+    float4* dst = const_cast<float4*>(A.xs) + (size_t)par * A.N;
+    for (int i = bid * kThreads + tid; i < A.N; i += G * kThreads) {
+      const float4 x = ld_cg(A.cols + i);
+      __stcg(dst + i, make_float4(x.x * f, x.y * f, x.z * f, 0.f));
+    }
+  };
+  if (copies && A.nsteps > 0) {
+    scale_x(0, sqrtf(kLog2e / (2.f * s2)));
+    good = grid_sync(A.ctl, epoch, (unsigned)G, A.timeout_ns, 22);
+  }
   const int own_rows = kRows ? A.geo.slice_len : 0;  // small clouds: rows of a block
   const int own_r0 = bid * own_rows, own_n = max(0, min(own_rows, A.M - own_r0));
   if (kRows) rows_load(A, *rs, xs, own_r0, own_n);
-  for (int step = 0; step < A.nsteps; ++step) {
+  for (int step = 0; step < A.nsteps && good; ++step) {
     tl.mark(1);
+    // the scaled X' was written by other blocks' ordinary stores, ahead of a
+    // grid barrier; the bulk copies that stream it read through the async proxy
+    if (copies && tid == 0) asm volatile("fence.proxy.async.global;" ::: "memory");
     const float outlier = expf(-A.d_02 / s2);  // src/emicp.cu:489
     float R[9], tc[3];
 #pragma unroll
@@ -532,14 +556,19 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
       rows_sweep(A, *rs, xs, sc, own_n);
       tl.mark(4);
       __syncthreads();
-    } else if (kTeam || A.blk) {
+    } else if (kTeam || copies || A.blk) {
       float Rs[9], tcs[3];
 #pragma unroll
       for (int k = 0; k < 9; ++k) Rs[k] = R[k] * sc;
 #pragma unroll
       for (int k = 0; k < 3; ++k) tcs[k] = tc[k] * sc;
       if (tid == 0 && s_pair[0] >= 0) s_tsweep = global_ns();
-      const bool ok = kTeam || A.geo.ranged
+      const bool ok = copies
+                          ? sweep_units<5, EmicpElemScaled, NoPrep, NoFin, true, 1>(
+                                sm, pipe, A.geo, StreamSrc{A.xs + (size_t)(step & 1) * A.N, nullptr, false}, A.rows, true,
+                                Rs, tcs, 0u, A.part, nullptr, EmicpElemScaled{}, NoPrep{}, NoFin{}, A.ctl, A.timeout_ns,
+                                10, tl, A.Mp, &oc_rows, &rs_rows)
+                      : kTeam || A.geo.ranged
                           ? em_local_sweep<1>(bid, G, sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
                                               A.ctl, A.timeout_ns, 10, tl, oc_rows, &rs_rows)
                           : em_local_sweep<0>(bid, G, sm, s_local, pipe, A.geo, src, A.rows, A.blk, Rs, tcs, sc, A.part, A.Mp,
@@ -575,6 +604,8 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
         }
       }
     }
+    // the next step's scaled X' (its buffer was last read by the previous step's sweep)
+    if (copies && step + 1 < A.nsteps) scale_x((step + 1) & 1, sqrtf(kLog2e / (2.f * (s2 * A.sigma_factor))));
     // ---- rows completed, each block a contiguous share of them; its 16
     // moments are one record. Thread t first sums the slice partials of
     // (row, accumulator) pairs t, t + kThreads, ... (loads in flight together),
@@ -585,7 +616,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
                   rb + (size_t)bid * kEmNV);
     } else {
       const int S = A.geo.slices;
-      const float inv_sc = kTeam || A.blk ? 1.f / sc : 1.f;  // local sweeps: the e x sums are sc times too large
+      const float inv_sc = kTeam || copies || A.blk ? 1.f / sc : 1.f;  // the e x sums are sc times too large
       const int rpc = (A.M + G - 1) / G;
       const int r0 = bid * rpc;
       const int nrows = max(0, min(rpc, A.M - r0));
@@ -657,7 +688,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     // ---- grid-wide moments -> pose (every block computes the same pose)
     reduce_block_partials<kEmNV>(rb, G, s_red, s_tot);
     tl.mark(6);
-    const bool refine = kRows ? step + kSmallRefine >= A.nsteps : kTeam || A.blk;
+    const bool refine = kRows ? step + kSmallRefine >= A.nsteps : kTeam ? A.refine != 0 : (!copies && A.blk != nullptr);
     em_moments_to_S_block(s_tot, s_emS, refine);
     if (tid == 0) {
       float Xc[3], Yc[3], S[9];
@@ -739,6 +770,12 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_kernel(const EmicpArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Pipe pipe;
   emicp_run<kPlain>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) emicp_ranges_kernel(const EmicpArgs A) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  Pipe pipe;
+  emicp_run<kRanges>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x);
 }
 
 __global__ void __launch_bounds__(kThreads, 2) emicp_rows_kernel(const EmicpArgs A) {
@@ -1034,7 +1071,7 @@ struct TeamPrep {
 
 __global__ void __launch_bounds__(1024) em_sort_teams_kernel(const TeamPrep* __restrict__ tab) {
   const TeamPrep P = tab[blockIdx.x];
-  em_sort(P.Y, P.M, P.keys, P.perm, P.perm + P.M);
+  if (P.perm) em_sort(P.Y, P.M, P.keys, P.perm, P.perm + P.M);
 }
 
 __global__ void em_pack_teams_kernel(const TeamPrep* __restrict__ tab) {
@@ -1044,7 +1081,12 @@ __global__ void em_pack_teams_kernel(const TeamPrep* __restrict__ tab) {
 
 __global__ void __launch_bounds__(kBlockPts) em_block_teams_kernel(const TeamPrep* __restrict__ tab) {
   const TeamPrep P = tab[blockIdx.y];
-  if ((int)blockIdx.x * kBlockPts < P.M) em_block(P.rows, P.M, P.blk);
+  if ((int)blockIdx.x * kBlockPts >= P.M) return;
+  if (!P.perm) {  // unsorted: no block counts as compact
+    if (threadIdx.x == 0) P.blk[blockIdx.x] = make_float4(0.f, 0.f, 0.f, __int_as_float(0x7fc00000));
+    return;
+  }
+  em_block(P.rows, P.M, P.blk);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1067,7 +1109,7 @@ struct EmicpPlan {
   int grid;
   SweepGeom geo;
   size_t smem;
-  bool local;  // sorted Y, local sweeps
+  bool local;  // sorted Y, local sweeps, refined poses
   bool rows;   // small clouds: whole rows to a block, X in shared memory
 };
 
@@ -1075,12 +1117,24 @@ size_t sweep_smem() { return sizeof(SweepSmem); }
 
 constexpr int kEmPairNum = 208;  // SM pairs: the favoured block's share, 13 / 16
 
-// Of the others, the local sweep (and the sort that it wants) is taken from 2.4e7
-// affinities a step on: below, a step is mostly latency and the prepare step's barrier per chunk
-// costs as much as the shorter element gives (4001^2: 1.045 -> 1.043 ms, 3000^2
-// 0.878 -> 0.897, 1007^2 0.576 -> 0.624; 6000 x 5000 1.46 -> 1.41, 12,000^2
-// 4.47 -> 4.01, 17,000^2 8.75 -> 7.75).
-bool emicp_local_pays(int N, int M) { return (double)N * (double)M >= 2.4e7; }
+// The others take the local sweep, with the sort that it wants and refined poses,
+// where that ends sooner over the whole schedule. Its shorter element saves 4.9e-5
+// ns of an affinity (40,097^2: 5.2 ms of 36), a refined pose costs 1.7 us a step, the
+// sort, by one block, 5 to 7 ns a row. Hence 4.6e7 affinities a step, and 1.35e5 columns
+// over all steps for a row. Default schedule, direct / local (ms): 9000 x 4000 1.59 / 1.63, x 6000
+// 2.11 / 2.07, 20,000 x 2000 1.71 / 1.73, x 3000 2.26 / 2.20, 2000 x 50,000 3.83 / 3.82, 2500 x 40,000
+// 4.30 / 4.08, 1000 x 400,000 11.6 / 13.5, 30 x 10^6 8.2 / 16.0; 16 steps: 3500 x 30,000 1.07 /
+// 1.10, 20,000 x 3000 0.60 / 0.59; one step of 40,097^2 0.78 / 0.91.
+bool emicp_sort_pays(int N, long nsteps) { return (double)N * (double)nsteps >= 1.35e5; }
+bool emicp_local_pays(int N, int M, long nsteps) {
+  return (double)N * (double)M >= 4.6e7 && emicp_sort_pays(N, nsteps);
+}
+
+// A batch's pairs are sorted side by side, a block each: it is not worth it only
+// for long thin ones (one pair alone, unsorted against sorted, ms: 129 x 190,001
+// 2.72 / 3.87, 300 x 100,000 2.47 / 3.03, 700 x 40,000 1.89 / 2.14; 3000 x 100,000 8.4 sorted, 10.4 in
+// lock step with direct differences).
+bool emicp_team_sorts(int N, int M, long nsteps) { return M <= 32768 || emicp_sort_pays(N, nsteps); }
 
 // Rows of a block in the small clouds' form, 0 where it is not taken: X has to
 // fit shared memory beside a second block's, and up to 6e7 affinities a step the
@@ -1097,10 +1151,11 @@ int emicp_small_rows(int N, int M, int limit) {
   return own <= kRowsOwn ? own : 0;
 }
 
-EmicpPlan plan_emicp(int N, int M, int device) {
+EmicpPlan plan_emicp(int N, int M, long nsteps, int device) {
   EmicpPlan P;
   P.smem = sweep_smem();
-  const int limit = persistent_grid_limit(device, (const void*)emicp_kernel, P.smem);
+  const int limit = std::min(persistent_grid_limit(device, (const void*)emicp_kernel, P.smem),
+                             persistent_grid_limit(device, (const void*)emicp_ranges_kernel, P.smem));
   P.local = P.rows = false;
   const int own =
       emicp_small_rows(N, M, persistent_grid_limit(device, (const void*)emicp_rows_kernel, rows_smem(kRowsMaxN)));
@@ -1111,7 +1166,7 @@ EmicpPlan plan_emicp(int N, int M, int device) {
     P.geo = SweepGeom{M, N, 0, 0, own, 0, 0, 0, 0, 0};
     return P;
   }
-  P.local = emicp_local_pays(N, M);
+  P.local = emicp_local_pays(N, M, nsteps);
   const SweepGeomH h = plan_sweep(M, N, limit);
   P.geo = SweepGeom{h.n_own, h.n_stream, h.nblk, h.slices, h.slice_len, h.units, 0, 0, 0, 0};
   P.grid = h.units < limit ? h.units : limit;
@@ -1119,7 +1174,7 @@ EmicpPlan plan_emicp(int N, int M, int device) {
   // chunk of 512 streamed points, instead of units dealt in waves; with two
   // blocks on every SM, each SM's pair splits its range 13 : 3, the larger
   // part to the block the SM favours.
-  if (P.local && ranged_pays(h.nblk, N, limit)) {
+  if (ranged_pays(h.nblk, N, limit)) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const char* ev = getenv("CESA_SM_PAIRS");  // "0": equal shares (for comparisons)
@@ -1135,6 +1190,7 @@ struct EmicpCarved {
   CenterHdr* hdr;
   float4* rows;
   float4* cols;
+  float4* xs;
   float4* blk;
   unsigned* keys;
   int* perm;
@@ -1153,6 +1209,7 @@ EmicpCarved carve_emicp(void* base, const EmicpPlan& P, int N, int M, size_t* to
   w.hdr = c.take<CenterHdr>(1);
   w.rows = c.take<float4>((size_t)M);
   w.cols = c.take<float4>((size_t)N);
+  w.xs = c.take<float4>(P.geo.ranged && !P.local ? (size_t)2 * N : 0);
   w.blk = c.take<float4>(P.local ? (size_t)P.geo.nblk : 0);
   w.keys = c.take<unsigned>(P.local ? (size_t)M : 0);
   w.perm = c.take<int>(P.local ? (size_t)2 * M : 0);
@@ -1166,16 +1223,24 @@ EmicpCarved carve_emicp(void* base, const EmicpPlan& P, int N, int M, size_t* to
 }
 }  // namespace
 
-void emicp_ws_views(void* ws, int N, int M, int device, CenterHdr** hdr, float4** rows, float4** cols) {
-  const EmicpPlan P = plan_emicp(N, M, device);
+void emicp_ws_views(void* ws, int N, int M, long nsteps, int device, CenterHdr** hdr, float4** rows, float4** cols) {
+  const EmicpPlan P = plan_emicp(N, M, nsteps, device);
   EmicpCarved w = carve_emicp(ws, P, N, M, nullptr);
   *hdr = w.hdr;
   *rows = w.rows;
   *cols = w.cols;
 }
 
-size_t emicp_ws_need(int N, int M, int device) {
-  const EmicpPlan P = plan_emicp(N, M, device);
+int emicp_form(int N, int M, long nsteps, int device) {
+  const EmicpPlan P = plan_emicp(N, M, nsteps, device);
+  return P.rows         ? CESA_EMICP_FORM_ROWS
+         : P.local      ? CESA_EMICP_FORM_LOCAL
+         : P.geo.ranged ? CESA_EMICP_FORM_RANGES
+                        : CESA_EMICP_FORM_SLICES;
+}
+
+size_t emicp_ws_need(int N, int M, long nsteps, int device) {
+  const EmicpPlan P = plan_emicp(N, M, nsteps, device);
   size_t total = 0;
   carve_emicp(nullptr, P, N, M, &total);
   return total;
@@ -1185,7 +1250,7 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return (int)e;
-  const EmicpPlan P = plan_emicp(L.N, L.M, device);
+  const EmicpPlan P = plan_emicp(L.N, L.M, L.nsteps, device);
   size_t total = 0;
   EmicpCarved w = carve_emicp(ws, P, L.N, L.M, &total);
   if (total > ws_bytes) return (int)cudaErrorInvalidValue;
@@ -1225,7 +1290,9 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   A.hdr = w.hdr;
   A.dRt = L.dRt;
   A.part = w.part;
+  A.xs = w.xs;
   A.blk = P.local ? w.blk : nullptr;
+  A.refine = 0;
   A.Mp = w.Mp;
   A.rbpart = w.rbpart;
   A.ctl = w.ctl;
@@ -1241,8 +1308,10 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   A.tl_cap = L.timeline_cap;
   A.timeout_ns = L.timeout_ns;
   void* args[] = {(void*)&A};
-  e = cudaLaunchCooperativeKernel(P.rows ? (const void*)emicp_rows_kernel : (const void*)emicp_kernel, dim3(P.grid), dim3(kThreads), args,
-                                  P.smem, st);
+  const void* kernel = P.rows                     ? (const void*)emicp_rows_kernel
+                       : P.geo.ranged && !P.local ? (const void*)emicp_ranges_kernel
+                                                  : (const void*)emicp_kernel;
+  e = cudaLaunchCooperativeKernel(kernel, dim3(P.grid), dim3(kThreads), args, P.smem, st);
   return (int)e;
 }
 
@@ -1386,9 +1455,11 @@ TeamsCarved carve_teams(void* base, const EmTeamJob* jobs, int n, const TeamPlan
     if (!A.geo.ranged) A.part = c.take<float>((size_t)5 * A.geo.slices * A.Mp);
     A.rbpart = c.take<df>((size_t)2 * P.size[(size_t)j] * kEmNV);
     A.pair_t = c.take<float>((size_t)P.size[(size_t)j]);
+    const bool sorted = emicp_team_sorts(J.N, J.M, J.nsteps);
+    A.refine = sorted;
     float4* blk = c.take<float4>((size_t)A.geo.nblk);
-    unsigned* keys = c.take<unsigned>((size_t)J.M);
-    int* perm = c.take<int>((size_t)2 * J.M);
+    unsigned* keys = sorted ? c.take<unsigned>((size_t)J.M) : nullptr;
+    int* perm = sorted ? c.take<int>((size_t)2 * J.M) : nullptr;
     float4* rows = c.take<float4>((size_t)J.M);
     A.rows = rows;
     A.blk = blk;

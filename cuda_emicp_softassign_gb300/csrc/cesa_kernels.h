@@ -173,7 +173,8 @@ SweepGeomH plan_sweep(int n_own, int n_stream, int grid_limit);
 int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, int* grid_used);
 int enqueue_softassign(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st,
                        int* grid_used);
-size_t emicp_ws_need(int N, int M, int device);
+int emicp_form(int N, int M, long nsteps, int device);  // CESA_EMICP_FORM_*
+size_t emicp_ws_need(int N, int M, long nsteps, int device);
 size_t softassign_ws_need(int N, int M, int form, int device);
 size_t softassign_mat_ws_need(int N, int M, int device);
 int enqueue_softassign_mat(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, int* grid_used);
@@ -223,7 +224,7 @@ struct EmicpAdjointLaunch {
 size_t emicp_adjoint_ws_need(int N, int M, int nsteps, int device, int layout);
 int enqueue_emicp_adjoint(const EmicpAdjointLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st);
 // The forward workspace's packed clouds and centring header (for the tape).
-void emicp_ws_views(void* ws, int N, int M, int device, CenterHdr** hdr, float4** rows, float4** cols);
+void emicp_ws_views(void* ws, int N, int M, long nsteps, int device, CenterHdr** hdr, float4** rows, float4** cols);
 
 void softassign_ws_views(void* ws, int N, int M, int device, CenterHdr** hdr, float4** rows, float4** cols);
 

@@ -142,6 +142,14 @@ void cesa_params_default(cesa_params* p);
 int cesa_emicp(const float* X, int N, const float* Y, int M, float R[9], float t[3],
                const cesa_params* p, cesa_report* rep);
 
+/* The form that an EM-ICP call of these sizes and this schedule takes on the
+ * current device, in *form. The choice is by speed alone. */
+#define CESA_EMICP_FORM_ROWS 1   /* small clouds: whole rows to a block, the target in shared memory */
+#define CESA_EMICP_FORM_LOCAL 2  /* sorted rows, exponents about a centre per block of 128 */
+#define CESA_EMICP_FORM_RANGES 3 /* direct differences, contiguous ranges of tasks per block */
+#define CESA_EMICP_FORM_SLICES 4 /* direct differences, (row block, column slice) units */
+int cesa_emicp_form(int N, int M, const cesa_params* p, int* form);
+
 /*
  * Annealed Softassign. Replaces softassign(), src/softassign.cu:256-886
  * (declared at src/3dregistration.h:82-86). Same conventions as cesa_emicp.
