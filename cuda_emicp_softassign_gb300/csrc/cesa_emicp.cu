@@ -439,12 +439,13 @@ struct TeamBlock {
 // slices. kRanges: direct differences over task ranges, in a kernel of its own
 // (beside the local sweeps it made them 1% slower). kTeams: one of several in the
 // launch (local sweeps, no tape); the caller has initialised the stage barriers
-// and the pipe. kSmall: small clouds, whole rows to a block (sm and pipe unused).
-constexpr int kPlain = 0, kTeams = 1, kSmall = 2, kRanges = 3;
+// and the pipe. kSmall: small clouds, whole rows to a block (sm and pipe unused);
+// kSmallOut: the same for a caller that wants the rows.
+constexpr int kPlain = 0, kTeams = 1, kSmall = 2, kRanges = 3, kSmallOut = 4;
 template <int kMode>
 __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pipe& pipe, const int& bid, const int& G,
                                           RowsSmem* rs = nullptr, float* xs = nullptr) {
-  constexpr bool kTeam = kMode == kTeams, kRows = kMode == kSmall;
+  constexpr bool kTeam = kMode == kTeams, kRows = kMode == kSmall || kMode == kSmallOut;
   __shared__ float s_pose[12];
   __shared__ df s_red[kThreads];
   __shared__ OwnCache oc_rows;
@@ -540,7 +541,23 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     if (kRows) {
       __syncthreads();  // (the first step: the rows are there)
       const float scr = sqrtf(kLog2e / (2.f * s2));
-      if (tid < kRowsOwn) {
+      if (kMode == kSmallOut) {
+        // The rows are asked for: -z scaled is rounded once (warp i: coordinate i). Rounded before
+        // the scale as well, as below, the rows' sums of e^2 are 1.15 times further off FP64
+        // than with direct differences unscaled, so 0.7 times. A registration, whose
+        // refined poses make up for it, keeps the shorter chain (0.15 us a step).
+        const int i = tid >> 5, row = tid & 31;
+        static_assert(kRowsOwn == 32, "a warp per coordinate");
+        if (i < 3) {
+          const float4 y = rs->y[row];
+          df z = df_make(s_pose[9 + i]);
+          df_add_prod(z, s_pose[3 * i], y.x);
+          df_add_prod(z, s_pose[3 * i + 1], y.y);
+          df_add_prod(z, s_pose[3 * i + 2], y.z);
+          z = dd_fast(z.hi, z.lo);
+          reinterpret_cast<float*>(&rs->nz[row])[i] = -__fmaf_rn(scr, z.hi, __fmul_rn(scr, z.lo));
+        }
+      } else if (tid < kRowsOwn) {
         const float4 y = rs->y[tid];
         rs->nz[tid] = make_float4(-scr * (R[0] * y.x + R[1] * y.y + R[2] * y.z + tc[0]),
                                   -scr * (R[3] * y.x + R[4] * y.y + R[5] * y.z + tc[1]),
@@ -778,10 +795,11 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_ranges_kernel(const EmicpAr
   emicp_run<kRanges>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x);
 }
 
+template <int kMode>
 __global__ void __launch_bounds__(kThreads, 2) emicp_rows_kernel(const EmicpArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Pipe pipe;
-  emicp_run<kSmall>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x,
+  emicp_run<kMode>(A, *reinterpret_cast<SweepSmem*>(smem_raw), pipe, (int)blockIdx.x, (int)gridDim.x,
                     reinterpret_cast<RowsSmem*>(smem_raw), reinterpret_cast<float*>(smem_raw + sizeof(RowsSmem)));
 }
 
@@ -1125,7 +1143,10 @@ constexpr int kEmPairNum = 208;  // SM pairs: the favoured block's share, 13 / 1
 // 2.11 / 2.07, 20,000 x 2000 1.71 / 1.73, x 3000 2.26 / 2.20, 2000 x 50,000 3.83 / 3.82, 2500 x 40,000
 // 4.30 / 4.08, 1000 x 400,000 11.6 / 13.5, 30 x 10^6 8.2 / 16.0; 16 steps: 3500 x 30,000 1.07 /
 // 1.10, 20,000 x 3000 0.60 / 0.59; one step of 40,097^2 0.78 / 0.91.
-bool emicp_sort_pays(int N, long nsteps) { return (double)N * (double)nsteps >= 1.35e5; }
+// (Never for a single step: it returns its rows, whose sums direct differences leave nearer to
+// FP64 at small sigma: 2.2e-7 against 3.8e-7 rms at 10,007 x 9001, sigma_p2 = 1e-4; no refined
+// pose makes up for them.)
+bool emicp_sort_pays(int N, long nsteps) { return nsteps > 1 && (double)N * (double)nsteps >= 1.35e5; }
 bool emicp_local_pays(int N, int M, long nsteps) {
   return (double)N * (double)M >= 4.6e7 && emicp_sort_pays(N, nsteps);
 }
@@ -1154,11 +1175,10 @@ int emicp_small_rows(int N, int M, int limit) {
 EmicpPlan plan_emicp(int N, int M, long nsteps, int device) {
   EmicpPlan P;
   P.smem = sweep_smem();
-  const int limit = std::min(persistent_grid_limit(device, (const void*)emicp_kernel, P.smem),
-                             persistent_grid_limit(device, (const void*)emicp_ranges_kernel, P.smem));
+  const int limit = persistent_grid_limit(device, (const void*)emicp_kernel, P.smem);
   P.local = P.rows = false;
   const int own =
-      emicp_small_rows(N, M, persistent_grid_limit(device, (const void*)emicp_rows_kernel, rows_smem(kRowsMaxN)));
+      emicp_small_rows(N, M, persistent_grid_limit(device, (const void*)emicp_rows_kernel<kSmall>, rows_smem(kRowsMaxN)));
   if (own > 0) {
     P.rows = true;
     P.smem = rows_smem(N);
@@ -1174,7 +1194,10 @@ EmicpPlan plan_emicp(int N, int M, long nsteps, int device) {
   // chunk of 512 streamed points, instead of units dealt in waves; with two
   // blocks on every SM, each SM's pair splits its range 13 : 3, the larger
   // part to the block the SM favours.
-  if (ranged_pays(h.nblk, N, limit)) {
+  // (The query also sets the kernel's shared-memory limit.)
+  const bool ranges = ranged_pays(h.nblk, N, limit) &&
+                      (P.local || persistent_grid_limit(device, (const void*)emicp_ranges_kernel, P.smem) >= limit);
+  if (ranges) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const char* ev = getenv("CESA_SM_PAIRS");  // "0": equal shares (for comparisons)
@@ -1308,9 +1331,13 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   A.tl_cap = L.timeline_cap;
   A.timeout_ns = L.timeout_ns;
   void* args[] = {(void*)&A};
-  const void* kernel = P.rows                     ? (const void*)emicp_rows_kernel
+  const void* kernel = P.rows                     ? (const void*)emicp_rows_kernel<kSmall>
                        : P.geo.ranged && !P.local ? (const void*)emicp_ranges_kernel
                                                   : (const void*)emicp_kernel;
+  if (P.rows && L.row_out) {
+    kernel = (const void*)emicp_rows_kernel<kSmallOut>;
+    if (persistent_grid_limit(device, kernel, rows_smem(kRowsMaxN)) < P.grid) return (int)cudaErrorCooperativeLaunchTooLarge;
+  }
   e = cudaLaunchCooperativeKernel(kernel, dim3(P.grid), dim3(kThreads), args, P.smem, st);
   return (int)e;
 }
