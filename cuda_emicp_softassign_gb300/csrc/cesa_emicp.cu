@@ -1172,7 +1172,7 @@ int emicp_small_rows(int N, int M, int limit) {
   return own <= kRowsOwn ? own : 0;
 }
 
-EmicpPlan plan_emicp(int N, int M, long nsteps, int device) {
+EmicpPlan plan_emicp_as(int N, int M, bool local, int device) {
   EmicpPlan P;
   P.smem = sweep_smem();
   const int limit = persistent_grid_limit(device, (const void*)emicp_kernel, P.smem);
@@ -1186,7 +1186,7 @@ EmicpPlan plan_emicp(int N, int M, long nsteps, int device) {
     P.geo = SweepGeom{M, N, 0, 0, own, 0, 0, 0, 0, 0};
     return P;
   }
-  P.local = emicp_local_pays(N, M, nsteps);
+  P.local = local;
   const SweepGeomH h = plan_sweep(M, N, limit);
   P.geo = SweepGeom{h.n_own, h.n_stream, h.nblk, h.slices, h.slice_len, h.units, 0, 0, 0, 0};
   P.grid = h.units < limit ? h.units : limit;
@@ -1234,15 +1234,27 @@ EmicpCarved carve_emicp(void* base, const EmicpPlan& P, int N, int M, size_t* to
   w.cols = c.take<float4>((size_t)N);
   w.xs = c.take<float4>(P.geo.ranged && !P.local ? (size_t)2 * N : 0);
   w.blk = c.take<float4>(P.local ? (size_t)P.geo.nblk : 0);
-  w.keys = c.take<unsigned>(P.local ? (size_t)M : 0);
-  w.perm = c.take<int>(P.local ? (size_t)2 * M : 0);
   w.part = c.take<float>(P.geo.ranged ? (size_t)5 * P.geo.nblk * P.geo.kmax * kBlockPts
                                       : (size_t)5 * P.geo.slices * w.Mp);
+  // the sort's keys (M) and orders (2 M) lie where the sweeps' partials, at least 5 M
+  // words, are written later: a sorted registration takes no more than one that is not
+  w.keys = reinterpret_cast<unsigned*>(w.part);
+  w.perm = reinterpret_cast<int*>(w.part) + M;
   w.rbpart = c.take<df>((size_t)2 * P.grid * kEmNV);
   w.pair_tab = c.take<unsigned>(P.geo.pair_num ? 2 * kPairCap + 1 : 0);
   w.pair_t = c.take<float>(P.geo.pair_num ? (size_t)P.grid : 0);
   if (total) *total = c.off;
   return w;
+}
+
+// cap: the workspace at hand. Sorted rows over slices want 16 bytes a block more
+// than unsorted ones; where only those fit, they run.
+EmicpPlan plan_emicp(int N, int M, long nsteps, int device, size_t cap = SIZE_MAX) {
+  EmicpPlan P = plan_emicp_as(N, M, emicp_local_pays(N, M, nsteps), device);
+  size_t total = 0;
+  carve_emicp(nullptr, P, N, M, &total);
+  if (P.local && total > cap) P = plan_emicp_as(N, M, false, device);
+  return P;
 }
 }  // namespace
 
@@ -1262,8 +1274,8 @@ int emicp_form(int N, int M, long nsteps, int device) {
                         : CESA_EMICP_FORM_SLICES;
 }
 
-size_t emicp_ws_need(int N, int M, long nsteps, int device) {
-  const EmicpPlan P = plan_emicp(N, M, nsteps, device);
+size_t emicp_ws_need(int N, int M, long nsteps, int device, size_t cap) {
+  const EmicpPlan P = plan_emicp(N, M, nsteps, device, cap);
   size_t total = 0;
   carve_emicp(nullptr, P, N, M, &total);
   return total;
@@ -1273,16 +1285,13 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return (int)e;
-  const EmicpPlan P = plan_emicp(L.N, L.M, L.nsteps, device);
+  const EmicpPlan P = plan_emicp(L.N, L.M, L.nsteps, device, ws_bytes);
   size_t total = 0;
   EmicpCarved w = carve_emicp(ws, P, L.N, L.M, &total);
   if (total > ws_bytes) return (int)cudaErrorInvalidValue;
   if (grid_used) *grid_used = P.grid;
-  // the control block starts at zero every launch, and so do the ranged
-  // partial slots (those no block writes must read as zero)
+  // the control block starts at zero every launch
   e = cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), st);
-  if (e == cudaSuccess && P.geo.ranged)
-    e = cudaMemsetAsync(w.part, 0, sizeof(float) * 5 * (size_t)P.geo.nblk * P.geo.kmax * kBlockPts, st);
   if (e == cudaSuccess && P.geo.pair_num)
     e = cudaMemsetAsync(w.pair_tab, 0, sizeof(unsigned) * (2 * kPairCap + 1), st);
   if (e != cudaSuccess) return (int)e;
@@ -1297,6 +1306,10 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
     em_pack_rows_kernel<<<pg_y < 1024 ? pg_y : 1024, pb, 0, st>>>(L.dY, L.M, w.hdr, nullptr, w.rows);
   }
   e = cudaGetLastError();
+  // ranged partial slots that no block writes must read as zero (after the sort,
+  // which uses the same memory)
+  if (e == cudaSuccess && P.geo.ranged)
+    e = cudaMemsetAsync(w.part, 0, sizeof(float) * 5 * (size_t)P.geo.nblk * P.geo.kmax * kBlockPts, st);
   if (e != cudaSuccess) return (int)e;
   if (L.nsteps <= 0) return 0;
 

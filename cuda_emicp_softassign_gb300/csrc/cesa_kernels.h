@@ -174,7 +174,8 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
 int enqueue_softassign(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st,
                        int* grid_used);
 int emicp_form(int N, int M, long nsteps, int device);  // CESA_EMICP_FORM_*
-size_t emicp_ws_need(int N, int M, long nsteps, int device);
+// cap: the workspace at hand, where that is fixed.
+size_t emicp_ws_need(int N, int M, long nsteps, int device, size_t cap = SIZE_MAX);
 size_t softassign_ws_need(int N, int M, int form, int device);
 size_t softassign_mat_ws_need(int N, int M, int device);
 int enqueue_softassign_mat(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, int* grid_used);

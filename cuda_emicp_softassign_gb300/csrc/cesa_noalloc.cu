@@ -45,7 +45,7 @@ extern "C" int cesa_emicp_device_noalloc(const float* dX, int N, const float* dY
   // The same lock as every other entry point: the plan behind the size check
   // and the launch is made once, for this device.
   std::lock_guard<std::mutex> lock(cesa::api_mutex());
-  if (cesa::emicp_ws_need(N, M, nsteps, dev) > kNoAllocScratchBytes) return CESA_ERR_NOALLOC_LIMIT;
+  if (cesa::emicp_ws_need(N, M, nsteps, dev, kNoAllocScratchBytes) > kNoAllocScratchBytes) return CESA_ERR_NOALLOC_LIMIT;
   if (!g_scratch_addr[dev]) {
     // The name g_noalloc_scratch is a host-side stand-in here, not a device
     // address. Resolve the device address once per device, with that device
