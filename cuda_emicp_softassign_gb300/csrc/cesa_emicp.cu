@@ -325,8 +325,9 @@ __host__ __device__ constexpr size_t rows_smem(int N) {
 __device__ __forceinline__ void rows_load(const EmicpArgs& A, RowsSmem& rs, float* xs, int r0, int nrows) {
   const int Np = (A.N + kRowsPad - 1) / kRowsPad * kRowsPad;
   for (int i = threadIdx.x; i < Np; i += kThreads) {
-    // padding columns: far away, affinity 0
-    const float4 x = i < A.N ? ld_cg(A.cols + i) : make_float4(1e18f, 1e18f, 1e18f, 0.f);
+    // padding columns: so far away that their affinity is 0 at every finite sigma_p2
+    // (the scale is 4.6e-20 and more: formed without 2 sigma_p2, which overflows)
+    const float4 x = i < A.N ? ld_cg(A.cols + i) : make_float4(3e38f, 3e38f, 3e38f, 0.f);
     xs[i] = x.x;
     xs[Np + i] = x.y;
     xs[2 * Np + i] = x.z;
@@ -540,7 +541,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
     for (int k = 0; k < 3; ++k) tc[k] = s_pose[9 + k];
     if (kRows) {
       __syncthreads();  // (the first step: the rows are there)
-      const float scr = sqrtf(kLog2e / (2.f * s2));
+      const float scr = sqrtf(0.5f * kLog2e / s2);
       if (kMode == kSmallOut) {
         // The rows are asked for: -z scaled is rounded once (warp i: coordinate i). Rounded before
         // the scale as well, as below, the rows' sums of e^2 are 1.15 times further off FP64
@@ -568,7 +569,7 @@ __device__ __forceinline__ bool emicp_run(const EmicpArgs& A, SweepSmem& sm, Pip
 
     // e = exp(-d2 / (2 s2)) = 2^(nk d2). Every unit stores its rows' partial
     // sums over its column slice (deferred: no completion counter).
-    const float sc = sqrtf(kLog2e / (2.f * s2));
+    const float sc = kRows ? sqrtf(0.5f * kLog2e / s2) : sqrtf(kLog2e / (2.f * s2));
     if (kRows) {
       rows_sweep(A, *rs, xs, sc, own_n);
       tl.mark(4);
