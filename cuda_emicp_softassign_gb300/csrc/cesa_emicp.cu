@@ -817,8 +817,8 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_rows_kernel(const EmicpArgs
 // small pairs, by a step's latency; the teams' sizes are even numbers of
 // blocks, which leaves up to 8% of the chip idle (20 x 14 of 304 blocks).
 __global__ void __launch_bounds__(kThreads, 2) emicp_teams_kernel(const EmicpArgs* __restrict__ jobs,
-                                                                  const TeamBlock* __restrict__ blocks, Ctl* ctl,
-                                                                  unsigned* pair_tab, uint64_t timeout_ns) {
+                                                                  int njobs, const TeamBlock* __restrict__ blocks,
+                                                                  Ctl* ctl, unsigned* pair_tab, uint64_t timeout_ns) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SweepSmem& sm = *reinterpret_cast<SweepSmem*>(smem_raw);
   __shared__ EmicpArgs s_args;
@@ -835,7 +835,10 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_teams_kernel(const EmicpArg
     if (pair_tab) {
       const int2 pr = join_sm_pair(pair_tab, timeout_ns);
       vb = pr.x >= 0 && pr.x < (int)gridDim.x / 2 ? 2 * pr.x + pr.y : -1;
-      if (vb < 0) set_status(ctl, kStatusInternal, 25);
+      if (vb < 0) {  // every registration's blocks leave at their first barrier
+        set_status(ctl, kStatusInternal, 25);
+        for (int j = 0; j < njobs; ++j) set_status(jobs[j].ctl, kStatusInternal, 25);
+      }
     }
     s_vb = vb;
   }
@@ -1555,7 +1558,7 @@ int enqueue_emicp_teams(const EmTeamJob* jobs, int n, void* ws, size_t ws_bytes,
   const EmicpArgs* jobs_d = w.args;
   const TeamBlock* blocks_d = w.blocks;
   Ctl* main_ctl = static_cast<Ctl*>(ctl);
-  void* args[] = {(void*)&jobs_d, (void*)&blocks_d, (void*)&main_ctl, (void*)&w.pair_tab, (void*)&timeout_ns};
+  void* args[] = {(void*)&jobs_d, (void*)&n, (void*)&blocks_d, (void*)&main_ctl, (void*)&w.pair_tab, (void*)&timeout_ns};
   return (int)cudaLaunchCooperativeKernel((const void*)emicp_teams_kernel, dim3(G), dim3(kThreads), args, sweep_smem(),
                                           st);
 }
