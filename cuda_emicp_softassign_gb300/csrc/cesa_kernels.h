@@ -113,7 +113,9 @@ struct SeriesHand {
 // The leading pose updates of a schedule whose affinities a short series
 // represents (cesa_softassign_series.cu). Fits when both clouds' shares fit
 // the shared memory of one cluster.
-bool softassign_series_fits(int N, int M);
+bool softassign_series_fits(int N, int M);  // on the current device
+// CTAs of the cluster that takes a pair where max_cluster is the largest there is; 0: none does.
+int softassign_series_cluster(int N, int M, int max_cluster);
 // max_degree: the highest degree of the series that is worth it against the
 // affinity kernel that would run the update instead.
 int enqueue_softassign_series(const SoftassignLaunch& L, const float4* rows, const float4* cols, const CenterHdr* hdr,

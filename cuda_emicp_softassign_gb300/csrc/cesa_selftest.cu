@@ -7,6 +7,7 @@
 
 #include "../../include/cesa.h"
 #include "cesa_common.cuh"
+#include "cesa_kernels.h"
 #include "cesa_sweep.cuh"
 
 namespace {
@@ -105,4 +106,9 @@ extern "C" int cesa_self_test_partition(int nblk, int nch, int grid, int pair_nu
       if (cesa::ranged_block_of(g, o * nch, grid) != b) return CESA_ERR_INTERNAL;
   }
   return next == (long)nblk * nch ? CESA_OK : CESA_ERR_INTERNAL;
+}
+
+extern "C" int cesa_self_test_series_cluster(int N, int M, int max_cluster) {
+  if (max_cluster < 0 || max_cluster > 16 || (max_cluster & (max_cluster - 1))) return 0;
+  return cesa::softassign_series_cluster(N, M, max_cluster);
 }

@@ -32,6 +32,7 @@
 // schedule, one box, affinity kernels -> this: N = M = 413 20.1 -> 6.6 ms, 2000
 // 12.9 -> 7.4, 20,000 461 -> 13.5; 30 updates from T = 0.1 at 7001 x 6007 4.25
 // -> 1.32.
+#include <mutex>
 #include <vector>
 
 #include "cesa_kernels.h"
@@ -941,16 +942,18 @@ struct SeriesPlan {
   size_t smem = 0;
 };
 
-// The least power of two of CTAs that leaves each at most `pts` points of a
-// cloud (0: the choice for one pair alone).
-SeriesPlan plan_series(int N, int M, int pts = 0) {
+// The least power of two of CTAs, up to max_cluster, that leaves each at most
+// `pts` points of a cloud (0: the choice for one pair alone); CS = 0 where the
+// points do not fit.
+SeriesPlan plan_series(int N, int M, int max_cluster, int pts = 0) {
   SeriesPlan P;
+  if (max_cluster < 1) return P;
   const int n = N > M ? N : M;
   int CS = 1;
   // one pair: 128 up to 512 points (7.0 against 7.2 ms with 256 at N = M =
   // 413), else 256 (7.7 against 7.7 with 128 and 9.0 with 512 at 2000)
   if (pts == 0) pts = n <= 512 ? 128 : 256;
-  while (CS < kSerMaxCS && (n + CS - 1) / CS > pts) CS *= 2;
+  while (2 * CS <= max_cluster && (n + CS - 1) / CS > pts) CS *= 2;
   const int nr = (N + CS - 1) / CS, nc = (M + CS - 1) / CS;
   const size_t smem =
       sizeof(float) * ((size_t)kLState + (size_t)kRowArr * ((nr + 3) & ~3) + (size_t)kColArr * ((nc + 3) & ~3));
@@ -963,26 +966,81 @@ SeriesPlan plan_series(int N, int M, int pts = 0) {
 }
 }  // namespace
 
+int softassign_series_cluster(int N, int M, int max_cluster) {
+  if (N < 1 || M < 1 || N >= (1 << 24) || M >= (1 << 24)) return 0;
+  return plan_series(N, M, max_cluster).CS;
+}
+
+namespace {
+cudaError_t series_limits(const void* k) {
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerSmemMax);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+
+cudaLaunchAttribute cluster_attr(int CS) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = CS;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  return at;
+}
+
+// The largest cluster that the device (or the partition of it) holds with the
+// most shared memory that a CTA takes here, for both kernels; 0: none. Asked once
+// per device.
+int series_max_cluster(int device) {
+  static std::mutex mu;
+  static int cached[64];  // 1 + the answer
+  std::lock_guard<std::mutex> lock(mu);
+  if (device < 0 || device >= 64) return 0;
+  if (cached[device] > 0) return cached[device] - 1;
+  int best = 0;
+  for (int CS = kSerMaxCS; CS >= 1 && best == 0; CS /= 2) {
+    bool all = true;
+    for (const void* k : {(const void*)softassign_series_kernel, (const void*)softassign_series_batch_kernel}) {
+      cudaLaunchAttribute at[1] = {cluster_attr(CS)};
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(CS);
+      cfg.blockDim = dim3(kSerThreads);
+      cfg.dynamicSmemBytes = kSerSmemMax;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (series_limits(k) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      all = all && n > 0;
+    }
+    if (all) best = CS;
+  }
+  cached[device] = best + 1;
+  return best;
+}
+}  // namespace
+
 bool softassign_series_fits(int N, int M) {
-  return N > 0 && M > 0 && N < (1 << 24) && M < (1 << 24) && plan_series(N, M).CS > 0;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return softassign_series_cluster(N, M, series_max_cluster(device)) > 0;
 }
 
 namespace {
 cudaError_t launch_series(const void* k, int clusters, int CS, size_t smem, void** args, cudaStream_t st,
                           bool beside = false) {
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerSmemMax);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  const cudaError_t e = series_limits(k);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * CS);
   cfg.blockDim = dim3(kSerThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CS;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2] = {cluster_attr(CS), {}};
   cfg.attrs = at;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
@@ -994,7 +1052,10 @@ cudaError_t launch_series(const void* k, int clusters, int CS, size_t smem, void
 int enqueue_softassign_series(const SoftassignLaunch& L, const float4* rows, const float4* cols, const CenterHdr* hdr,
                               float* s_out, float* u_out, SeriesHand* hand, int max_degree, void* ctl,
                               cudaStream_t st) {
-  const SeriesPlan P = plan_series(L.N, L.M);
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  const SeriesPlan P = plan_series(L.N, L.M, series_max_cluster(device));
   if (P.CS < 1) return (int)cudaErrorInvalidConfiguration;
   SeriesArgs A{};
   A.rows = rows;
@@ -1035,10 +1096,10 @@ size_t softassign_series_table_bytes(int njobs) { return sizeof(SeriesArgs) * (s
 // / 129 / 105 CTAs) and 25 ms one cluster size after the other. Clusters of 16 leave SMs
 // of their GPCs over, so 7/8 of the SMs count (154 CTAs did not fit 152 SMs:
 // 12.5 ms; 129 did).
-int batch_points(const SeriesJob* jobs, int njobs, int sms) {
+int batch_points(const SeriesJob* jobs, int njobs, int max_cluster, int sms) {
   for (int pts = 256; pts <= 1024; pts *= 2) {
     long ctas = 0;
-    for (int i = 0; i < njobs; ++i) ctas += plan_series(jobs[i].N, jobs[i].M, pts).CS;
+    for (int i = 0; i < njobs; ++i) ctas += plan_series(jobs[i].N, jobs[i].M, max_cluster, pts).CS;
     if (ctas <= (long)sms * 7 / 8) return pts;
   }
   return kSerBatchPts;
@@ -1049,7 +1110,8 @@ int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return (int)e;
-  const int pts = batch_points(jobs, njobs, sms);
+  const int max_cluster = series_max_cluster(device);
+  const int pts = batch_points(jobs, njobs, max_cluster, sms);
   // one launch per cluster size, its pairs in the order given
   std::vector<SeriesArgs> tab;
   tab.reserve((size_t)njobs);
@@ -1062,7 +1124,7 @@ int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_
     Group g{CS, (int)tab.size(), 0, 0};
     for (int i = 0; i < njobs; ++i) {
       const SeriesJob& J = jobs[i];
-      const SeriesPlan P = plan_series(J.N, J.M, pts);
+      const SeriesPlan P = plan_series(J.N, J.M, max_cluster, pts);
       if (P.CS != CS) continue;
       SeriesArgs A{};
       A.rows = J.rows;

@@ -424,6 +424,12 @@ int cesa_self_test_waits(int which, int timeout_us, int* status_out, int* where_
  * CESA_ERR_INVALID_ARGUMENT; *kmax_out receives kmax. */
 int cesa_self_test_partition(int nblk, int nch, int grid, int pair_num, int* kmax_out);
 
+/* Host-side check of the Softassign series form's clusters (no counterpart in the
+ * reference; needs no GPU): the thread blocks of the cluster that takes an N x M pair
+ * on a device whose largest cluster is max_cluster blocks (a power of two up to 16), or 0
+ * where none does and the affinity kernels run alone. */
+int cesa_self_test_series_cluster(int N, int M, int max_cluster);
+
 /* Library version as major*10000 + minor*100 + patch. */
 int cesa_version(void);
 
