@@ -110,7 +110,8 @@ namespace {
 __device__ __forceinline__ void st_dsmem(const float* p, unsigned rank, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dsmem_addr(p, rank)), "f"(v) : "memory");
 }
-__device__ __forceinline__ void st_dsmem2(const float* p, unsigned rank, float a, float b) {
+// (float2: the store wants 8-byte alignment)
+__device__ __forceinline__ void st_dsmem2(const float2* p, unsigned rank, float a, float b) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dsmem_addr(p, rank)), "f"(a), "f"(b) : "memory");
 }
 
@@ -705,15 +706,16 @@ __device__ __noinline__ void series_update(Ser& Sg, df wsc, int I1, float lam, f
     warp_sum_df32(v, at(kLRed) + warp * kSerRedRows * kSerRedLd, reinterpret_cast<df*>(wd) + warp * 32);
   }
   __syncthreads();
-  float* slotD = at(kLSlotD);
+  float2* slotD = reinterpret_cast<float2*>(at(kLSlotD));
+  static_assert(kLSlotD % 2 == 0, "pairs");
   if (tid < 32 * 4) {
     const int k = tid & 31;
     const df s = sum16d(wd + 2 * k);
 #pragma unroll 1
-    for (int r = tid >> 5; r < S.CS; r += 4) st_dsmem2(slotD + (S.rank * 32 + k) * 2, (unsigned)r, s.hi, s.lo);
+    for (int r = tid >> 5; r < S.CS; r += 4) st_dsmem2(slotD + S.rank * 32 + k, (unsigned)r, s.hi, s.lo);
   }
   ser_sync(S);
-  if (tid < 32) reinterpret_cast<df*>(at(kLTot))[tid] = sum16d(slotD + 2 * tid);
+  if (tid < 32) reinterpret_cast<df*>(at(kLTot))[tid] = sum16d(at(kLSlotD) + 2 * tid);
   __syncthreads();
   Sg.par = S.par;
 }
@@ -745,7 +747,7 @@ constexpr float kTolEqual = 2.98e-8f, kTolUnequal = 2e-9f;
 
 // The updates of one pair, by one cluster.
 __device__ __forceinline__ void series_run(const SeriesArgs& A) {
-  __shared__ float s_rad[kSerMaxCS][2];
+  __shared__ float2 s_rad[kSerMaxCS];
   __shared__ float s_wr[2][kSerWarps];
   __shared__ SaPoseScratch ps;
   __shared__ HornState<float> horn;
@@ -828,14 +830,14 @@ __device__ __forceinline__ void series_run(const SeriesArgs& A) {
       rx = nan_max(rx, s_wr[0][w]);
       ry = nan_max(ry, s_wr[1][w]);
     }
-    for (int r = 0; r < S.CS; ++r) st_dsmem2(s_rad[S.rank], (unsigned)r, rx, ry);
+    for (int r = 0; r < S.CS; ++r) st_dsmem2(&s_rad[S.rank], (unsigned)r, rx, ry);
   }
   ser_sync(S);
-  rx = s_rad[0][0];
-  ry = s_rad[0][1];
+  rx = s_rad[0].x;
+  ry = s_rad[0].y;
   for (int r = 1; r < S.CS; ++r) {
-    rx = nan_max(rx, s_rad[r][0]);
-    ry = nan_max(ry, s_rad[r][1]);
+    rx = nan_max(rx, s_rad[r].x);
+    ry = nan_max(ry, s_rad[r].y);
   }
   rx = sqrtf(rx) * 1.0001f;
   ry = sqrtf(ry) * 1.0001f;
