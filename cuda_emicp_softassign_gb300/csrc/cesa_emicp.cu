@@ -78,14 +78,17 @@ struct EmicpArgs {
 // 2^-|z~|^2 multiplies a row's sums once: 3 FFMA for the exponent in place of
 // 3 FADD + FMUL + 2 FFMA, 8 FP32 ops per element in place of 11. It is taken
 // while the block's scaled radius is at most sqrt(kLocalR2), where 2^|z~|^2
-// cannot overflow a sum of e^2 and the rounding of |x~|^2 (of affinities that
-// count, |x~| < 6 + radius) stays at the level of the coordinates' own;
-// otherwise the block sweeps direct differences (EmicpElemScaled). Y is sorted
+// cannot overflow a sum of e^2; otherwise the block sweeps direct differences
+// (EmicpElemScaled). The exponent is rounded at the size of |x~|^2 (of affinities that
+// count, |x~| < 6 + radius), not of d^2: at small sigma a row's sum of e^2 is further
+// off FP64 than by direct differences (10,007 x 9001, rms: 2.5e-7 -> 3.4e-7 at sigma_p2 =
+// 3e-4, 2.2e-7 -> 3.8e-7 at 1e-4, 9.7e-7 -> 1.25e-6 at 1.06e-5). Refined poses more than make
+// up for that in poses and gradients. Y is sorted
 // along a Hilbert curve so that blocks are compact: at N = M = 40,097 98% of the
 // default schedule's affinities take the short form, at 8171 points 91%.
 // Bound by the FP32 pipe as before (72% of it busy where every block is short,
-// 23.0 instructions per 128 elements against 29.5): N = M = 40,097 36.3 -> 30.9
-// ms, 17,000 8.75 -> 7.57, 8171 x 6007 1.97 -> 1.86. Not kept: 8 owned points a
+// 23.0 instructions per 128 elements against 29.5): N = M = 40,097 36.3 -> 31.5
+// ms (poses refined), 17,000 8.75 -> 7.57. Not kept: 8 owned points a
 // lane (256 per unit 33.0 ms, or 128 over half-warps 33.4, at their best pair
 // splits), records stored as packed duplicates (35.4), kLocalR2 = 16 (32.1).
 constexpr float kLocalR2 = 48.f;
@@ -906,8 +909,8 @@ __device__ __forceinline__ unsigned hilbert_index(unsigned (&x)[3]) {
 // Order of Y along a Hilbert curve of 32^3 cells over its bounding cube: a
 // stable radix sort of 15-bit keys (two 8-bit digits) by one block, warp w on
 // the w-th contiguous segment, so that the order does not depend on timing.
-// perm receives it (tmp: scratch of M). One block: 40,097 points take about
-// 0.1% of the registration that they are sorted for.
+// perm receives it (tmp: scratch of M). One block, 5 to 7 ns a point: 0.8% of a
+// registration of 40,097 points; emicp_sort_pays and emicp_team_sorts say where not.
 __device__ __forceinline__ void em_sort(const float* __restrict__ Y, int M, unsigned* keys, int* perm, int* tmp) {
   constexpr int kW = 32, kDig = 256;
   __shared__ float s_lo[3][kW], s_hi[3][kW];

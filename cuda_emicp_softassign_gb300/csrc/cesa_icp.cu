@@ -571,8 +571,8 @@ __global__ void __launch_bounds__(kThreads, 2) icp_kernel(const IcpArgs A) {
     for (int k = 0; k < 9; ++k) R[k] = s_pose[k];
 #pragma unroll
     for (int k = 0; k < 3; ++k) tc[k] = s_pose[9 + k];
-    // ---- phase A (grid): each row's nearest point by rings of cells; rows over
-    // the per-thread budget are searched again by a whole warp after a barrier
+    // ---- phase A (grid): each row's nearest point, by 8 lanes from a candidate
+    // (rows with wide balls by a warp after a barrier)
     if (A.grid) {
       const IcpGrid g = *A.grid;
       const int warp = tid >> 5, lane = tid & 31;

@@ -9,8 +9,10 @@
 //   F_r = e^(-|x_r - delta|^2 / T),  G_c = e^(-(|z_c|^2 + 2 z_c.delta) / T),
 // and e^(u.v) = sum_|k|<=D u^k v^k / k! over the monomials of three variables.
 // The truncation is at most q^(D+1)/(D+1)! e^q of a term, q = 2 max|x| max|z| / T
-// (independent of the pose): D is the smallest degree (2..8) for which that is
-// below 2^-25, half an FP32 unit in the last place. A row pass is then: the
+// (independent of the pose): D is the smallest degree (2..8, or up to what the
+// caller gives: 6 beside the banded kernel, 4 there on unequal counts) for which
+// that is below 2^-25, half an FP32 unit in the last place, or 2e-9 for clouds of
+// unequal counts (kTolEqual, kTolUnequal). A row pass is then: the
 // P = C(D+3, 3) moments sum_c b_c G_c v_c^k of the columns, and per row the
 // polynomial sum_k (moment_k / k!) u_r^k; a column pass likewise. The default
 // schedule on scans of 0.2 extent (alignScaleOnce's scale) has q from 4e-4 at
@@ -27,11 +29,13 @@
 // final sweep and the pose are those of the affinity kernels
 // (src/softassign.cu:494-798), the scalings and the slack as (hi, lo) pairs.
 // What bounds it is latency: an update is a chain of ~8 exchanges and the
-// fixed-order sums before and after each (~14 us up to 4000 points, D <= 4;
-// ~32 us at D = 8), not its arithmetic (2 P FMAs per point and pass). Default
-// schedule, one box, affinity kernels -> this: N = M = 413 20.1 -> 6.6 ms, 2000
-// 12.9 -> 7.4, 20,000 461 -> 13.5; 30 updates from T = 0.1 at 7001 x 6007 4.25
-// -> 1.32.
+// fixed-order sums before and after each, up to some 2000 points, and from there on the
+// points' polynomials too (2 P FMAs per point and pass). us an update at D = 2, 4 and 6:
+// N = M = 100 10.4, 12.6, 16.6; 413 12.4, 14.6, 18.0; 2000 13.9, 17.3, 23.1; 7001 17.2, 22.9, 33.0; 20,000
+// 25.0, 34.2, 51.4. Default schedule, affinity kernels -> this: N = M = 413 20.1 -> 6.6
+// ms, 2000 12.9 -> 7.4, 20,000 461 -> 13.6; 30 updates from T = 0.1 at 7001 x 6007
+// 4.25 -> 1.2 to 1.6, and 2.5 where a pair's extent leaves the last ones to the affinity
+// kernels (8 pairs).
 #include <mutex>
 #include <vector>
 
