@@ -30,7 +30,7 @@ NVFLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-co
 SOURCES = ["cesa_api.cu", "cesa_emicp.cu", "cesa_softassign.cu", "cesa_noalloc.cu", "cesa_selftest.cu",
            "cesa_batch.cu", "cesa_softassign_mat.cu", "cesa_emicp_adjoint.cu",
            "cesa_softassign_adjoint.cu", "cesa_icp.cu", "cesa_io.cpp", "cesa_softassign_band.cu",
-           "cesa_softassign_series.cu"]
+           "cesa_softassign_series.cu", "cesa_teams.cpp"]
 HEADERS = ["cesa_common.cuh", "cesa_sweep.cuh", "cesa_pose.h", "cesa_kernels.h", "cesa_prep.cuh", "cesa_ops.cuh",
            "cesa_sa_pose.cuh", "cesa_pose_dd.cuh"]
 

@@ -634,11 +634,12 @@ int cesa_register_batch_device(const cesa_pair* pairs, int npairs, int* d_status
   cudaStream_t st = (cudaStream_t)stream;
   std::lock_guard<std::mutex> lock(g_mu);
   StreamCtx& C = ctx_for(dev, st);
-  cudaError_t e = C.ws.ensure(batch_ws_need(rec.data(), npairs, dev));
+  TeamPlan plan;
+  cudaError_t e = C.ws.ensure(batch_ws_need(rec.data(), npairs, dev, &plan));
   if (e != cudaSuccess) return map_cuda(e);
   C.last_kind = 3;
   C.last_trace_steps = 0;
-  return map_cuda((cudaError_t)enqueue_batch(rec.data(), npairs, d_status, batch_timeout_ns(pairs, npairs),
+  return map_cuda((cudaError_t)enqueue_batch(rec.data(), npairs, plan, d_status, batch_timeout_ns(pairs, npairs),
                                              C.ws.p, C.ws.bytes, st, nullptr, nullptr));
 }
 
@@ -683,14 +684,15 @@ int cesa_register_batch(const cesa_pair* pairs, int npairs, cesa_report* rep) {
   }
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(dpose, hpose.data(), sizeof(float) * hpose.size(), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = C.ws.ensure(batch_ws_need(rec.data(), npairs, dev));
+  TeamPlan plan;
+  if (e == cudaSuccess) e = C.ws.ensure(batch_ws_need(rec.data(), npairs, dev, &plan));
   if (e != cudaSuccess) return map_cuda(e);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEventCreate(&ev0);
   cudaEventCreate(&ev1);
   int grid = 0, rounds = 0;
   cudaEventRecord(ev0, st);
-  int kerr = enqueue_batch(rec.data(), npairs, nullptr, batch_timeout_ns(pairs, npairs), C.ws.p, C.ws.bytes, st,
+  int kerr = enqueue_batch(rec.data(), npairs, plan, nullptr, batch_timeout_ns(pairs, npairs), C.ws.p, C.ws.bytes, st,
                            &grid, &rounds);
   cudaEventRecord(ev1, st);
   if (kerr != 0) e = (cudaError_t)kerr;

@@ -880,7 +880,7 @@ size_t batch_smem(int npairs) {
 
 }  // namespace
 
-size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device) {
+size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device, TeamPlan* plan) {
   Ctl* ctl = nullptr;
   size_t zb = 0;
   BPair* dp = nullptr;
@@ -890,10 +890,10 @@ size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device) {
   const int G = persistent_grid_limit(device, (const void*)batch_kernel, batch_smem(npairs));
   std::vector<EmTeamJob> teams;
   const size_t own = carve_batch(nullptr, pairs, npairs, G, nullptr, &teams, &ctl, &zb, &dp, &rounds, &rctr, &stab);
-  return own + emicp_teams_ws_need(teams.data(), (int)teams.size(), device);
+  return own + emicp_teams_ws_need(teams.data(), (int)teams.size(), device, plan);
 }
 
-int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint64_t timeout_ns, void* ws,
+int enqueue_batch(const BatchLaunchPair* pairs, int npairs, const TeamPlan& plan, int* d_status, uint64_t timeout_ns, void* ws,
                   size_t ws_bytes, cudaStream_t st, int* grid_used, int* rounds_out) {
   if (npairs < 1 || npairs > kMaxBatchPairs) return (int)cudaErrorInvalidValue;
   int device = 0;
@@ -923,8 +923,8 @@ int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint6
   if (e != cudaSuccess) return (int)e;
   if (grid_used) *grid_used = limit;
   if (rounds == 0) return 0;
-  const int te = enqueue_emicp_teams(teams.data(), (int)teams.size(), static_cast<char*>(ws) + own, ws_bytes - own, ctl,
-                                     timeout_ns, st);
+  const int te = enqueue_emicp_teams(teams.data(), (int)teams.size(), plan, static_cast<char*>(ws) + own, ws_bytes - own,
+                                     ctl, timeout_ns, st);
   if (te) return te;
   // The leading updates of the Softassign pairs, as far as a short series
   // represents their affinities: a cluster per pair, before the lock-step

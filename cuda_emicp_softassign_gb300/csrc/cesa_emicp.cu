@@ -432,12 +432,6 @@ __device__ __forceinline__ void rows_finish(const EmicpArgs& A, RowsSmem& rs, in
   if (lane < 16) __stcg(reinterpret_cast<float2*>(rec + k), make_float2(s.hi, s.lo));
 }
 
-// A block's part in emicp_teams_kernel: jobs [first, first + njobs), block
-// `rank` of the `size` blocks that run them.
-struct TeamBlock {
-  int first, njobs, rank, size;
-};
-
 // One registration by blocks 0 .. G - 1, this one block bid; false after a
 // failure (status set). kPlain: local sweeps (A.blk) or direct differences over
 // slices. kRanges: direct differences over task ranges, in a kernel of its own
@@ -810,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, 2) emicp_rows_kernel(const EmicpArgs
 // Many registrations in one cooperative launch, each by a team of blocks of
 // its own: a team goes through its registrations one after the other and waits
 // for nobody else, so that pairs of any sizes fill the chip without a step of
-// one being a step of all (plan_teams). All sweeps are local and ranged: one
+// one being a step of all (cesa_teams.cpp). All sweeps are local and ranged: one
 // sweep loop (with the slice layout beside it ptxas made it 8% slower), its
 // arguments in shared memory. In lock step over all pairs, with direct
 // differences, a step paid two grid barriers and a last wave of units; lock step
@@ -1363,90 +1357,6 @@ int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t 
 }
 
 namespace {
-// A batch's registrations over the launch's blocks. A registration takes about
-// nsteps (kTeamStepNs + M (N kTeamElemNs + kTeamRowNs) / g) on g blocks (an
-// element of a block that shares its SM: 0.096-0.098 measured for M <= 5120; a
-// row's sums and completion; the barriers and the pose of a step). For the least
-// t that the blocks can keep, every one that needs more than a block gets the
-// fewest that hold it to t, and the others go to single blocks, as many on one
-// as stay below t. Teams of whole SMs come first (their pairs of blocks split
-// the sweep by pair_num); an odd number of blocks, or one, takes kTeamOdd times
-// as long for the lack of that. The blocks of a pair depend on t and its own
-// size, not on where it stands in the batch.
-constexpr double kTeamElemNs = 0.095, kTeamRowNs = 30.0, kTeamStepNs = 8000.0, kTeamOdd = 1.2;
-
-struct TeamPlan {
-  std::vector<TeamBlock> blocks;
-  std::vector<int> order;  // job -> index in the caller's list
-  std::vector<int> size;   // blocks of every job
-};
-
-TeamPlan plan_teams(const EmTeamJob* jobs, int n, int G) {
-  TeamPlan P;
-  std::vector<double> cost((size_t)n), need((size_t)n);  // need: time on one block
-  P.order.resize((size_t)n);
-  P.size.resize((size_t)n);
-  double sum = 0.0;
-  for (int i = 0; i < n; ++i) {
-    const double steps = (double)jobs[i].nsteps;
-    P.order[(size_t)i] = i;
-    cost[(size_t)i] = steps * (double)jobs[i].M * ((double)jobs[i].N * kTeamElemNs + kTeamRowNs);
-    need[(size_t)i] = kTeamOdd * cost[(size_t)i] + steps * kTeamStepNs;
-    sum += need[(size_t)i];
-  }
-  std::stable_sort(P.order.begin(), P.order.end(), [&](int a, int b) { return need[(size_t)a] > need[(size_t)b]; });
-  // sizes for a time t, and the blocks they take (more than G: not kept)
-  auto fill = [&](double t) -> long {
-    long used = 0;
-    double left = 0.0;
-    for (int j = 0; j < n && used <= G; ++j) {
-      const size_t i = (size_t)P.order[(size_t)j];
-      const double run = t - jobs[i].nsteps * kTeamStepNs;
-      int g = 1;
-      if (need[i] > t) {
-        const double e = run > 0.0 ? std::ceil(0.5 * cost[i] / run) * 2.0 : 2.0 * G;
-        const double o = run > 0.0 ? std::ceil(kTeamOdd * cost[i] / run) : 2.0 * G;
-        g = (int)std::min(std::min(e, o), 2.0 * G);
-        used += g;
-      } else if (left >= need[i]) {
-        left -= need[i];
-      } else {
-        left = t - need[i];
-        used += 1;
-      }
-      P.size[(size_t)j] = g;
-    }
-    return used;
-  };
-  double lo = 0.0, hi = sum;  // all on one block
-  for (int k = 0; k < 24; ++k) {
-    const double t = 0.5 * (lo + hi);
-    if (fill(t) <= G) hi = t;
-    else lo = t;
-  }
-  fill(hi);
-  for (int odd = 0; odd < 2; ++odd)
-    for (int j = 0; j < n; ++j) {
-      const int g = P.size[(size_t)j];
-      if (g > 1 && (g & 1) == odd)
-        for (int r = 0; r < g; ++r) P.blocks.push_back(TeamBlock{j, 1, r, g});
-    }
-  double left = -1.0;
-  for (int j = 0; j < n; ++j) {  // single blocks: consecutive in the order
-    if (P.size[(size_t)j] > 1) continue;
-    const double w = need[(size_t)P.order[(size_t)j]];
-    if (left >= w) {
-      left -= w;
-      P.blocks.back().njobs += 1;
-    } else {
-      left = hi - w;
-      P.blocks.push_back(TeamBlock{j, 1, 0, 1});
-    }
-  }
-  if ((int)P.blocks.size() < G) P.blocks.resize((size_t)G, TeamBlock{0, 0, 0, 0});  // the rest idle
-  return P;
-}
-
 struct TeamsCarved {
   Ctl* ctl;  // one per job; cleared, as are the ranged partials behind them
   unsigned* pair_tab;
@@ -1525,22 +1435,22 @@ int teams_grid(int device, bool* pairs) {
 }
 }  // namespace
 
-size_t emicp_teams_ws_need(const EmTeamJob* jobs, int n, int device) {
+size_t emicp_teams_ws_need(const EmTeamJob* jobs, int n, int device, TeamPlan* plan) {
   if (n < 1) return 0;
   bool pairs = false;
-  const TeamPlan P = plan_teams(jobs, n, teams_grid(device, &pairs));
-  return carve_teams(nullptr, jobs, n, P, pairs, 0).total;
+  *plan = plan_teams(jobs, n, teams_grid(device, &pairs));
+  return carve_teams(nullptr, jobs, n, *plan, pairs, 0).total;
 }
 
-int enqueue_emicp_teams(const EmTeamJob* jobs, int n, void* ws, size_t ws_bytes, void* ctl, uint64_t timeout_ns,
-                        cudaStream_t st) {
+int enqueue_emicp_teams(const EmTeamJob* jobs, int n, const TeamPlan& P, void* ws, size_t ws_bytes, void* ctl,
+                        uint64_t timeout_ns, cudaStream_t st) {
   if (n < 1) return 0;
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return (int)e;
   bool pairs = false;
   const int G = teams_grid(device, &pairs);
-  const TeamPlan P = plan_teams(jobs, n, G);
+  if ((int)P.order.size() != n) return (int)cudaErrorInvalidValue;
   TeamsCarved w = carve_teams(ws, jobs, n, P, pairs, timeout_ns);
   if (w.total > ws_bytes || (int)P.blocks.size() != G) return (int)cudaErrorInvalidValue;
   int max_blk = 1;

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <vector>
 
 struct cesa_params;
 
@@ -199,13 +200,27 @@ struct EmTeamJob {
   const CenterHdr* hdr;
   float* dRt;            // PoseIO in/out (device)
 };
-size_t emicp_teams_ws_need(const EmTeamJob* jobs, int n, int device);
-int enqueue_emicp_teams(const EmTeamJob* jobs, int n, void* ws, size_t ws_bytes, void* ctl, uint64_t timeout_ns,
-                        cudaStream_t st);
+// A block's part in emicp_teams_kernel: jobs [first, first + njobs), block
+// `rank` of the `size` blocks that run them.
+struct TeamBlock {
+  int first, njobs, rank, size;
+};
+struct TeamPlan {
+  std::vector<TeamBlock> blocks;
+  std::vector<int> order;  // job -> index in the caller's list
+  std::vector<int> size;   // blocks of every job
+  double time_ns = 0.0;    // modelled time of the longest team
+};
+TeamPlan plan_teams(const EmTeamJob* jobs, int n, int G);  // G blocks (host arithmetic)
+// The workspace that the plan, made here, wants.
+size_t emicp_teams_ws_need(const EmTeamJob* jobs, int n, int device, TeamPlan* plan);
+int enqueue_emicp_teams(const EmTeamJob* jobs, int n, const TeamPlan& plan, void* ws, size_t ws_bytes, void* ctl,
+                        uint64_t timeout_ns, cudaStream_t st);
 
 // Batched registration.
-size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device);
-int enqueue_batch(const BatchLaunchPair* pairs, int npairs, int* d_status, uint64_t timeout_ns, void* ws,
+// plan: the EM-ICP pairs' teams, for the enqueue_batch that follows.
+size_t batch_ws_need(const BatchLaunchPair* pairs, int npairs, int device, TeamPlan* plan);
+int enqueue_batch(const BatchLaunchPair* pairs, int npairs, const TeamPlan& plan, int* d_status, uint64_t timeout_ns, void* ws,
                   size_t ws_bytes, cudaStream_t st, int* grid_used, int* rounds_out);
 
 // EM-ICP adjoint over a recorded forward (tape).

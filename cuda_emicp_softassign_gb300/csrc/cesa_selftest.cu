@@ -5,6 +5,8 @@
 // control block and leaves the context usable.
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "../../include/cesa.h"
 #include "cesa_common.cuh"
 #include "cesa_kernels.h"
@@ -111,4 +113,48 @@ extern "C" int cesa_self_test_partition(int nblk, int nch, int grid, int pair_nu
 extern "C" int cesa_self_test_series_cluster(int N, int M, int max_cluster) {
   if (max_cluster < 0 || max_cluster > 16 || (max_cluster & (max_cluster - 1))) return 0;
   return cesa::softassign_series_cluster(N, M, max_cluster);
+}
+
+extern "C" int cesa_self_test_teams(int n, const int* N, const int* M, const int* nsteps, int grid, int* blocks_out,
+                                    double* time_ms) {
+  if (n < 1 || n > 4096 || !N || !M || !nsteps || grid < 2 || grid > 4096 || !blocks_out || !time_ms)
+    return CESA_ERR_INVALID_ARGUMENT;
+  std::vector<cesa::EmTeamJob> jobs((size_t)n);
+  for (int i = 0; i < n; ++i) {
+    if (N[i] < 1 || M[i] < 1 || nsteps[i] < 1) return CESA_ERR_INVALID_ARGUMENT;
+    jobs[(size_t)i].N = N[i];
+    jobs[(size_t)i].M = M[i];
+    jobs[(size_t)i].nsteps = nsteps[i];
+  }
+  const cesa::TeamPlan P = cesa::plan_teams(jobs.data(), n, grid);
+  // every registration once
+  if ((int)P.order.size() != n || (int)P.size.size() != n || (int)P.blocks.size() != grid) return CESA_ERR_INTERNAL;
+  std::vector<int> seen((size_t)n, 0), runs((size_t)n, 0);
+  for (int j = 0; j < n; ++j) {
+    const int i = P.order[(size_t)j];
+    if (i < 0 || i >= n || seen[(size_t)i]++) return CESA_ERR_INTERNAL;
+    blocks_out[i] = P.size[(size_t)j];
+  }
+  // teams: consecutive blocks of ranks 0 .. size - 1 with the same registrations, each
+  // of which wants that size; even ones from an even block on (whole SMs)
+  for (int b = 0; b < grid;) {
+    const cesa::TeamBlock t = P.blocks[(size_t)b];
+    if (t.njobs == 0) {
+      ++b;
+      continue;
+    }
+    if (t.rank != 0 || t.size < 1 || b + t.size > grid || t.first < 0 || t.first + t.njobs > n) return CESA_ERR_INTERNAL;
+    if (t.size % 2 == 0 && b % 2) return CESA_ERR_INTERNAL;
+    for (int r = 0; r < t.size; ++r) {
+      const cesa::TeamBlock& u = P.blocks[(size_t)(b + r)];
+      if (u.first != t.first || u.njobs != t.njobs || u.rank != r || u.size != t.size) return CESA_ERR_INTERNAL;
+    }
+    for (int k = 0; k < t.njobs; ++k)
+      if (runs[(size_t)(t.first + k)]++ || P.size[(size_t)(t.first + k)] != t.size) return CESA_ERR_INTERNAL;
+    b += t.size;
+  }
+  for (int j = 0; j < n; ++j)
+    if (runs[(size_t)j] != 1) return CESA_ERR_INTERNAL;
+  *time_ms = P.time_ns * 1e-6;
+  return CESA_OK;
 }

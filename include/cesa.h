@@ -424,6 +424,14 @@ int cesa_self_test_waits(int which, int timeout_us, int* status_out, int* where_
  * CESA_ERR_INVALID_ARGUMENT; *kmax_out receives kmax. */
 int cesa_self_test_partition(int nblk, int nch, int grid, int pair_num, int* kmax_out);
 
+/* Host-side check of a batch's EM-ICP teams (no counterpart in the reference;
+ * needs no GPU): plans n registrations of N[i] x M[i] points and nsteps[i] sigma
+ * steps over `grid` blocks, and checks that every one runs once, by consecutive
+ * blocks that agree on it. blocks_out[i]: its blocks; *time_ms: the modelled time.
+ * CESA_OK, CESA_ERR_INTERNAL where a property fails, or CESA_ERR_INVALID_ARGUMENT. */
+int cesa_self_test_teams(int n, const int* N, const int* M, const int* nsteps, int grid, int* blocks_out,
+                         double* time_ms);
+
 /* Host-side check of the Softassign series form's clusters (no counterpart in the
  * reference; needs no GPU): the thread blocks of the cluster that takes an N x M pair
  * on a device whose largest cluster is max_cluster blocks (a power of two up to 16), or 0
