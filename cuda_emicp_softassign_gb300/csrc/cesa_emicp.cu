@@ -1153,10 +1153,12 @@ bool emicp_local_pays(int N, int M, long nsteps) {
 }
 
 // A batch's pairs are sorted side by side, a block each: it is not worth it only
-// for long thin ones (one pair alone, unsorted against sorted, ms: 129 x 190,001
-// 2.72 / 3.87, 300 x 100,000 2.47 / 3.03, 700 x 40,000 1.89 / 2.14; 3000 x 100,000 8.4 sorted, 10.4 in
-// lock step with direct differences).
-bool emicp_team_sorts(int N, int M, long nsteps) { return M <= 32768 || emicp_sort_pays(N, nsteps); }
+// for long thin ones (one pair alone, unsorted against sorted and lock step, ms: 10 x
+// 32,000 1.05 / 1.40 / 1.30, 400 x 32,000 1.38 / 1.67 / 1.59, 129 x 190,001 2.72 / 3.87 / 3.17, 300 x 100,000
+// 2.47 / 3.03 / 2.65; 20 pairs of 400 x 32,000 11.4 / 10.9 / 11.2, of 800 x 32,000 18.2 / 16.9 / 17.0).
+bool emicp_team_sorts(int N, int M, long nsteps) {
+  return M <= 8192 || (M <= 32768 && N >= 500) || emicp_sort_pays(N, nsteps);
+}
 
 // Rows of a block in the small clouds' form, 0 where it is not taken: X has to
 // fit shared memory beside a second block's, and up to 6e7 affinities a step the
