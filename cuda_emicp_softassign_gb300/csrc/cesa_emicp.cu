@@ -1172,7 +1172,13 @@ int emicp_small_rows(int N, int M, int limit) {
   if (N > kRowsMaxN || (double)N * (double)M >= 6e7) return 0;
   int own = (M + 4 * limit - 1) / (4 * limit) * 4;
   if (own == 4 && M > 2 * limit) own = 8;
-  return own <= kRowsOwn ? own : 0;
+  // many rows against few columns: a block's passes take longer than the slices' second
+  // barrier (ms, slices against this: 16 x 7000 0.735 / 0.751, 100 x 9000 0.773 / 0.801, 200 x 9728 0.799
+  // / 0.814, 600 x 9000 0.862 / 0.926, 1600 x 9728 1.104 / 1.159; but 16 x 5000 0.735 / 0.691, 300 x 9728
+  // 0.857 / 0.815, 1000 x 8000 0.942 / 0.871, 2000 x 9700 1.206 / 1.169)
+  const bool thin = (own > 20 && N < 64) || (own > 24 && N < 128) ||
+                    (own > 28 && (N < 224 || (N > 512 && N < 2000)));
+  return own <= kRowsOwn && !thin ? own : 0;
 }
 
 EmicpPlan plan_emicp_as(int N, int M, bool local, int device) {

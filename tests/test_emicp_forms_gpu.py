@@ -15,6 +15,9 @@ pytestmark = pytest.mark.gpu
     (100, 100, 1e-5, "ROWS"), (1007, 1007, 1e-5, "ROWS"), (8171, 6007, 1e-5, "ROWS"),
     (9001, 9001, 1e-5, "LOCAL"), (8193, 6390, 1e-5, "LOCAL"), (40097, 40097, 1e-5, "LOCAL"),
     (3000, 100000, 1e-5, "LOCAL"), (100000, 9000, 1e-5, "LOCAL"),
+    # many rows to a block against few columns: the second barrier costs less
+    (16, 7000, 1e-5, "SLICES"), (100, 9000, 1e-5, "SLICES"), (600, 9000, 1e-5, "SLICES"), (16, 5000, 1e-5, "ROWS"),
+    (300, 9700, 1e-5, "ROWS"), (1000, 8000, 1e-5, "ROWS"), (2000, 9700, 1e-5, "ROWS"),
     # few affinities a step: the refined poses and the sort cost more than the shorter element saves
     (9000, 2700, 1e-5, "SLICES"), (190001, 129, 1e-5, "SLICES"),
     # few columns to a row, or few steps: the sort costs more
