@@ -79,27 +79,31 @@ struct TeamPacker {
   std::vector<std::vector<std::pair<double, int>>> left;  // by size: (time left, team)
   std::vector<double> sum;                                // by size
   std::vector<int> kinds;                                 // by size: shapes that want it
+  std::vector<int> sizes;                                 // sizes that some shape wants
   std::vector<std::pair<int, std::vector<int>>> teams;    // (size, registrations)
   TeamPacker(const TeamModel& m, std::vector<TeamShape>& s, int g)
       : model(m), shapes(s), G(g), left((size_t)g + 1), sum((size_t)g + 1), kinds((size_t)g + 1) {}
   // the teams' times evenly divided, which any packing wants at least
   bool may(double t, double K) {
-    std::fill(sum.begin(), sum.end(), 0.0);
-    std::fill(kinds.begin(), kinds.end(), 0);
+    for (int g : sizes) {
+      sum[(size_t)g] = 0.0;
+      kinds[(size_t)g] = 0;
+      left[(size_t)g].clear();
+    }
+    sizes.clear();
     for (TeamShape& s : shapes) {
       if (!s.fit(model, t / K, G)) return false;
-      sum[(size_t)s.blocks] += s.count * s.own;
-      kinds[(size_t)s.blocks] += 1;
+      const size_t g = (size_t)s.blocks;
+      if (kinds[g]++ == 0) sizes.push_back(s.blocks);
+      sum[g] += s.count * s.own;
     }
     double used = 0.0;
-    for (int g = 1; g <= G; ++g)
-      if (sum[(size_t)g] > 0.0) used += g * std::ceil(sum[(size_t)g] / t - 1e-9);
+    for (int g : sizes) used += g * std::ceil(sum[(size_t)g] / t - 1e-9);
     return used <= G;
   }
   // build: with the teams' registrations, not only whether they fit
   bool pack(double t, double K, bool build) {
     if (!may(t, K)) return false;
-    for (auto& h : left) h.clear();
     teams.clear();
     int used = 0, at = 0;
     for (const TeamShape& s : shapes) {
