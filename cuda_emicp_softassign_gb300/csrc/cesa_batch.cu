@@ -915,7 +915,7 @@ int enqueue_batch(const BatchLaunchPair* pairs, int npairs, const TeamPlan& plan
   if (rounds_out) *rounds_out = rounds;
   e = cudaMemsetAsync(ws, 0, zero_bytes, st);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dpairs, host.data(), sizeof(BPair) * (size_t)npairs, cudaMemcpyHostToDevice, st);
+    e = put_table(dpairs, host.data(), sizeof(BPair) * (size_t)npairs, st);
   if (e != cudaSuccess) return (int)e;
   batch_center_kernel<<<npairs, 1024, 0, st>>>(dpairs);
   batch_pack_kernel<<<dim3(16, npairs), 256, 0, st>>>(dpairs);

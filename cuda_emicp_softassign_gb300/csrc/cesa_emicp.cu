@@ -30,6 +30,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "../../include/cesa.h"
@@ -1465,11 +1466,11 @@ int enqueue_emicp_teams(const EmTeamJob* jobs, int n, const TeamPlan& P, void* w
   for (const EmicpArgs& A : w.hargs) max_blk = A.geo.nblk > max_blk ? A.geo.nblk : max_blk;
   e = cudaMemsetAsync(ws, 0, w.zero_bytes, st);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(w.args, w.hargs.data(), sizeof(EmicpArgs) * (size_t)n, cudaMemcpyHostToDevice, st);
+    e = put_table(w.args, w.hargs.data(), sizeof(EmicpArgs) * (size_t)n, st);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(w.prep, w.hprep.data(), sizeof(TeamPrep) * (size_t)n, cudaMemcpyHostToDevice, st);
+    e = put_table(w.prep, w.hprep.data(), sizeof(TeamPrep) * (size_t)n, st);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(w.blocks, P.blocks.data(), sizeof(TeamBlock) * P.blocks.size(), cudaMemcpyHostToDevice, st);
+    e = put_table(w.blocks, P.blocks.data(), sizeof(TeamBlock) * P.blocks.size(), st);
   if (e != cudaSuccess) return (int)e;
   em_sort_teams_kernel<<<n, 1024, 0, st>>>(w.prep);
   em_pack_teams_kernel<<<dim3(16, n), 256, 0, st>>>(w.prep);
@@ -1493,6 +1494,30 @@ int read_ws_status(void* ws, cudaStream_t st, int* status, int* steps, int* tl_w
   if (steps) *steps = h.steps_done;
   if (tl_written) *tl_written = (int)h.pad[0];
   return 0;
+}
+
+namespace {
+struct TableChunk {
+  unsigned w[896];
+};
+__global__ void table_chunk_kernel(unsigned* dst, int n, const __grid_constant__ TableChunk c) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = c.w[i];
+}
+}  // namespace
+
+cudaError_t put_table(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap != cudaStreamCaptureStatusActive) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  if (bytes % sizeof(unsigned)) return cudaErrorInvalidValue;
+  for (size_t at = 0; at < bytes; at += sizeof(TableChunk)) {
+    TableChunk c;
+    const size_t len = bytes - at < sizeof(c) ? bytes - at : sizeof(c);
+    memcpy(c.w, static_cast<const char*>(src) + at, len);
+    table_chunk_kernel<<<1, 256, 0, st>>>(reinterpret_cast<unsigned*>(static_cast<char*>(dst) + at),
+                                          (int)(len / sizeof(unsigned)), c);
+  }
+  return cudaGetLastError();
 }
 
 // Smem opt-in and occupancy for a persistent kernel: blocks per SM x SMs.

@@ -176,6 +176,10 @@ SweepGeomH plan_sweep(int n_own, int n_stream, int grid_limit);
 int enqueue_emicp(const EmicpLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st, int* grid_used);
 int enqueue_softassign(const SoftassignLaunch& L, void* ws, size_t ws_bytes, cudaStream_t st,
                        int* grid_used);
+// Copies a table that the caller frees after the call to the device (whole words). On
+// a stream that is being captured it goes by value, in kernel arguments: a captured copy
+// would read the host memory again at every replay.
+cudaError_t put_table(void* dst, const void* src, size_t bytes, cudaStream_t st);
 int emicp_form(int N, int M, long nsteps, int device);  // CESA_EMICP_FORM_*
 // cap: the workspace at hand, where that is fixed.
 size_t emicp_ws_need(int N, int M, long nsteps, int device, size_t cap = SIZE_MAX);

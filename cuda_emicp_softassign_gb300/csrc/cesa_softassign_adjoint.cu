@@ -1262,8 +1262,8 @@ int softassign_bwd_prepare(const SoftassignBackward& B, const SaUpdate* host_tab
   const int last = (int)B.nsteps - 1;
   cudaError_t e = cudaSuccess;
   if (B.nsteps > 0)
-    e = cudaMemcpyAsync(c.L.tab, host_tab, sizeof(SaUpdate) * (size_t)B.nsteps, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(c.A.cur, &last, sizeof(int), cudaMemcpyHostToDevice, st);
+    e = put_table(c.L.tab, host_tab, sizeof(SaUpdate) * (size_t)B.nsteps, st);
+  if (e == cudaSuccess) e = put_table(c.A.cur, &last, sizeof(int), st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(c.L.X, B.X, sizeof(float4) * (size_t)N, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(c.L.Y, B.Y, sizeof(float4) * (size_t)M, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(c.L.hdr, B.hdr, sizeof(CenterHdr), cudaMemcpyDeviceToDevice, st);
@@ -1391,7 +1391,7 @@ int softassign_bwd_persistent(const SoftassignBackward& B, const SaUpdate* host_
   const Layout& L = c.L;
   e = cudaMemsetAsync(L.ctl, 0, sizeof(Ctl), st);
   if (e == cudaSuccess && B.nsteps > 0)
-    e = cudaMemcpyAsync(L.tab, host_tab, sizeof(SaUpdate) * (size_t)B.nsteps, cudaMemcpyHostToDevice, st);
+    e = put_table(L.tab, host_tab, sizeof(SaUpdate) * (size_t)B.nsteps, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(L.X, B.X, sizeof(float4) * (size_t)N, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(L.Y, B.Y, sizeof(float4) * (size_t)M, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(L.hdr, B.hdr, sizeof(CenterHdr), cudaMemcpyDeviceToDevice, st);

@@ -1162,7 +1162,7 @@ int enqueue_softassign_series_batch(const SeriesJob* jobs, int njobs, void* dev_
     if (g.n > 0) groups.push_back(g);
   }
   if (tab.empty()) return 0;
-  e = cudaMemcpyAsync(dev_table, tab.data(), sizeof(SeriesArgs) * tab.size(), cudaMemcpyHostToDevice, st);
+  e = put_table(dev_table, tab.data(), sizeof(SeriesArgs) * tab.size(), st);
   for (size_t i = 0; i < groups.size() && e == cudaSuccess; ++i) {
     const SeriesArgs* t = static_cast<const SeriesArgs*>(dev_table) + groups[i].first;
     void* args[] = {(void*)&t};
