@@ -94,3 +94,21 @@ def test_local_on_degenerate_clouds(cesa, torch_cuda, case):
         return cesa.emicp(X, Y, param=p)
     (R1, t1), (R2, t2) = run(9000, cesa.EMICP_FORM_LOCAL), run(4800, cesa.EMICP_FORM_ROWS)
     assert np.array_equal(np.isfinite(R1), np.isfinite(R2)) and np.array_equal(np.isfinite(t1), np.isfinite(t2))
+
+
+def test_ranges_registration(cesa, oracle, torch_cuda):
+    """A registration by ranges of tasks (X scaled anew for every step): the pose after
+    each step against the FP64 oracle's, 1e-3 degrees and 1e-5 of the extent."""
+    from conftest import rot_err_deg
+    from cuda_emicp_softassign_gb300 import workloads as W
+    X, Y, _, _ = W.surface_pair(n=1025, m=330001, seed=4, max_deg=10.0, outlier_frac=0.05)
+    sched = dict(sigma_p2=0.01, sigma_inf=0.0045)  # 8 steps
+    p = cesa.Params.default(**sched)
+    assert cesa.emicp_form(1025, 330001, p) == cesa.EMICP_FORM_RANGES
+    _, _, trace, _ = cesa.emicp(X, Y, param=p, trace=True)
+    _, _, ref = oracle.emicp(X, Y, **sched)
+    assert len(trace) == len(ref) == 8
+    extent = float(np.ptp(X, 0).max())
+    for got, want in zip(trace, ref):
+        assert rot_err_deg(got[18:27].reshape(3, 3), want[18:27].reshape(3, 3)) < 1e-3
+        assert np.abs(got[27:30] - want[27:30]).max() < 1e-5 * extent
